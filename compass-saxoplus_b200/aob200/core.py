@@ -82,7 +82,8 @@ class OwnedDeviceArray(DeviceArray):
         nbytes = max(int(n), 1) * np.dtype(dtype).itemsize
         call("aob_malloc", ctypes.addressof(p), nbytes, int(device))
         super().__init__(p.value, n, dtype, shape)
-        call("aob_memcpy_h2d", self.ptr, np.zeros(nbytes, np.uint8).ctypes.data, nbytes, None)
+        zeros = np.zeros(nbytes, np.uint8)  # (a name of its own: it must outlive the copy)
+        call("aob_memcpy_h2d", self.ptr, zeros.ctypes.data, nbytes, None)
 
     def __del__(self):
         try:
