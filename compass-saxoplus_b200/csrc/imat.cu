@@ -4,14 +4,23 @@
 // The reference's SutraRtc::do_imat (libsutra/src.cpp/sutra_rtc.cpp:150-292)
 // loops over the actuators: comp_oneactu (push), raytrace to the sensor,
 // comp_image, do_centroids, then the same with the pull, and the column
-// (s_push - s_pull) / (2 push).  Here the 2 nact pokes of a chunk go through
-// four launches in total: the single-actuator DM shapes (the pixel-major CSR
-// gather with one non-zero command), the bilinear raytrace of each onto the
-// sensor's phase grid, ONE sensor launch over all pokes' sub-apertures with the
-// attached centroider fused (grid.y = poke; no cube or image is written), and
-// the push-pull difference into the matrix.  Every step has the arithmetic of
-// the corresponding separate call, so the matrix equals the poke-by-poke one
-// bit for bit.
+// (s_push - s_pull) / (2 push).
+//
+// A poke moves only the sub-apertures whose phase window meets the actuator's
+// influence patch: at 40 x 40 sub-apertures and 41 x 41 actuators about 32 of
+// 1248.  The others see a flat phase on the push and on the pull, so their
+// entries are the difference of a slope from itself.  One CTA takes one
+// actuator: it lists the sub-apertures that the patch reaches, writes the
+// entries of all the others, and forms the push and pull images of the listed
+// ones (the stages of sh_core.cuh) with the phase evaluated from the patch
+// where it is needed, so neither DM shapes, phases nor slopes go through
+// memory.  Every value has the arithmetic of the corresponding separate call,
+// so the matrix equals the poke-by-poke one bit for bit.
+//
+// Bound: issue of the sensor stages (about 86,000 images at that size).  One call
+// takes 0.26 ms (B200, warm); forming all 3.4 M images from DM shapes and phases
+// in memory took 22 ms (14.7 ms images, 2.8 ms shapes, 0.65 ms tracing, the rest
+// 1.5 GB of scratch).
 
 #include <algorithm>
 
@@ -21,93 +30,153 @@
 
 namespace aob {
 
-// poke j of the chunk: actuator a0 + j / 2, command +push (j even) or -push (odd)
-__global__ void imat_dm_kernel(float *shapes, int64_t npix, const int32_t *rowptr, const int32_t *act,
-                               const float *w, int a0, float push) {
-  const int j = blockIdx.y;
-  const int a = a0 + j / 2;
-  const float c = (j & 1) ? -push : push;
-  float *out = shapes + (int64_t)j * npix;
-  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < npix; p += (int64_t)gridDim.x * blockDim.x) {
-    float v = 0.f;  // (the other actuators' zero commands add nothing)
-    for (int k = rowptr[p]; k < rowptr[p + 1]; ++k)
-      if (act[k] == a) v += c * w[k];
-    out[p] = v;
-  }
-}
+constexpr int IMAT_THREADS = 256;
+constexpr int IMAT_LIST = 512;  // sub-apertures of one actuator listed at a time
+constexpr int IMAT_ITEMS = 16;  // images per batch, at most: 51 KB of shared memory at 40 x 40, four CTAs per SM
 
-// the raytrace of one DM shape per poke (raytrace_kernel with one source, reset)
-__global__ void imat_trace_kernel(float *phases, int nx, const float *shapes, int N, float xoff, float yoff) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  const int y = blockIdx.y * blockDim.y + threadIdx.y;
-  const int j = blockIdx.z;
-  if (x >= nx || y >= nx) return;
-  const float *d = shapes + (int64_t)j * N * N;
-  float acc = 0.f;
-  const float xref = (float)x - nx / 2.0f + nx / 2.0f + xoff;
-  const float yref = (float)y - nx / 2.0f + nx / 2.0f + yoff;
-  const int iref = (int)xref, jref = (int)yref;
-  const float xs = xref - iref, ys = yref - jref;
-  const float wx1 = 1.0f - xs, wx2 = xs, wy1 = 1.0f - ys, wy2 = ys;
-  if (iref + 1 < N && jref + 1 < N) {
-    acc += (wx1 * wy1 * d[iref + jref * N] + wx2 * wy1 * d[iref + 1 + jref * N] +
-            wx1 * wy2 * d[iref + (jref + 1) * N] + wx2 * wy2 * d[iref + 1 + (jref + 1) * N]);
-  } else {
-    acc += 0.0f;
-  }
-  phases[(int64_t)j * nx * nx + x + y * nx] = acc;
-}
+struct ImatArgs {
+  const float *influ;
+  const int32_t *i1, *j1;
+  int isz, dim;
+  float xoff, yoff, push;
+  const float *flat;  // slopes of the flat phase (2 nvalid, the sensor's order)
+  float *imat;        // nslope x nact, column-major
+};
 
-// The sensor over all pokes: CTA (x, y) takes sub-aperture batch x of poke y,
-// with the poke's phase, slopes and intensities.
-constexpr int IMAT_SH_THREADS = 256;
+// Items 2 j (push) and 2 j + 1 (pull) of listed sub-aperture j; a < 0: every item
+// is a sub-aperture of its own under a flat phase.
+struct ImatSource {
+  static constexpr bool LISTED = true;
+  const ImatArgs &A;
+  const int *list;
+  float2 *slopes;
+  int a, npup, first;  // first: item of the batch's s = 0
+  int i1, j1;
+  __device__ int sub(int s) const { return list[a < 0 ? first + s : (first + s) >> 1]; }
+  // the DM screen with actuator a's command only: dm_shape_kernel's 0 + com * influ
+  __device__ float screen(int x, int y, float com) const {
+    const int u = x - i1, v = y - j1;
+    const bool in = u >= 0 && u < A.isz && v >= 0 && v < A.isz && x < A.dim && y < A.dim;
+    return in ? com * __ldg(A.influ + u + v * A.isz + (size_t)a * A.isz * A.isz) : 0.f;
+  }
+  __device__ float phase(int s, int X, int Y) const {
+    if (a < 0) return 0.f;
+    const float xref = ray_position(X, npup, A.xoff), yref = ray_position(Y, npup, A.yoff);
+    const int i = (int)xref, j = (int)yref;
+    float acc = 0.f;
+    if (i >= 0 && j >= 0 && i + 1 < A.dim && j + 1 < A.dim) {
+      const float com = ((first + s) & 1) ? -A.push : A.push;
+      acc += ray_bilinear(xref - i, yref - j, screen(i, j, com), screen(i + 1, j, com), screen(i, j + 1, com),
+                          screen(i + 1, j + 1, com));
+    }
+    return acc;
+  }
+  __device__ void store(int s, float x, float y) const { slopes[first + s] = make_float2(x, y); }
+  // whether the phase window [x0, x0 + pd) x [y0, y0 + pd) reads the patch
+  __device__ bool reaches(int x0, int y0, int pd) const {
+    auto at = [](int i, int n, float off) { return (int)ray_position(i, n, off); };
+    return at(x0 + pd - 1, npup, A.xoff) >= i1 - 1 && at(x0, npup, A.xoff) <= i1 + A.isz - 1 &&
+           at(y0 + pd - 1, npup, A.yoff) >= j1 - 1 && at(y0, npup, A.yoff) <= j1 + A.isz - 1;
+  }
+};
+
+// shared memory behind the sensor's tables and work area: the list, then two slopes per entry
+constexpr size_t IMAT_LIST_BYTES = IMAT_LIST * (sizeof(int) + 2 * sizeof(float2));
+
 template <int NFFT, int PD>
-__global__ void __launch_bounds__(IMAT_SH_THREADS)
-    imat_sh_kernel(ShKernelArgs P, int S, int64_t phase_stride, int nslope) {
+__device__ __forceinline__ void imat_images(const ShKernelArgs &P, ImatSource &src, int nitems, int S,
+                                            unsigned char *smem, const ShSmem &L) {
+  const Team T{(int)threadIdx.x, (int)blockDim.x, 0};
+  for (int f = 0; f < nitems; f += S) {
+    src.first = f;
+    sh_batch<NFFT, PD, TEAM_CTA, NoHook, false, false, ImatSource>(P, 0, 1, min(S, nitems - f), smem, smem + L.hdr, L,
+                                                                   T, NoHook{}, src);
+  }
+}
+
+// The slopes of the flat phase, sub-apertures blockIdx.x * IMAT_ITEMS and on.
+template <int NFFT, int PD>
+__global__ void __launch_bounds__(IMAT_THREADS) imat_flat_kernel(ShKernelArgs P, ImatArgs A, int S, float *flat) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ ShKernelArgs Q;
-  if (threadIdx.x == 0) {
-    Q = P;
-    const int j = blockIdx.y;
-    Q.phase = P.phase + (int64_t)j * phase_stride;
-    Q.c_slopes = P.c_slopes + (int64_t)j * nslope;
-    Q.intensities = P.intensities + (int64_t)j * P.nvalid;
-    Q.c_intens = Q.intensities;
-  }
+  const int pd = PD > 0 ? PD : P.pdiam;
+  const ShSmem L(NFFT, P.nu, P.nv, pd, P.nrebin2 * P.npix * P.npix, P.npix * P.npix, S);
+  float2 *slopes = reinterpret_cast<float2 *>(smem + ShSmem::align16(L.bytes()));
+  int *list = reinterpret_cast<int *>(slopes + 2 * IMAT_LIST);
+  sh_load_tables<NFFT>(P, smem, threadIdx.x, blockDim.x);
+  const int k0 = blockIdx.x * IMAT_ITEMS, n = min(IMAT_ITEMS, P.nvalid - k0);
+  for (int i = threadIdx.x; i < n; i += blockDim.x) list[i] = k0 + i;
   __syncthreads();
-  const int pd = PD > 0 ? PD : Q.pdiam;
-  const ShSmem L(NFFT, Q.nu, Q.nv, pd, Q.nrebin2 * Q.npix * Q.npix, Q.npix * Q.npix, S);
-  sh_load_tables<NFFT>(Q, smem, threadIdx.x, blockDim.x);
-  for (int base = blockIdx.x; base < Q.nvalid; base += S * gridDim.x) {
-    const int Sb = min(S, (Q.nvalid - base + (int)gridDim.x - 1) / (int)gridDim.x);
-    sh_batch<NFFT, PD>(Q, base, gridDim.x, Sb, smem, smem + L.hdr, L, Team{(int)threadIdx.x, (int)blockDim.x, 0});
-  }
-}
-
-__global__ void imat_diff_kernel(float *imat, const float *slopes, int nslope, int a0, int count, float push) {
-  const int64_t n = (int64_t)nslope * count;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
-    const int i = (int)(t / nslope), s = (int)(t - (int64_t)i * nslope);
-    const float sp = slopes[(int64_t)(2 * i) * nslope + s], sm = slopes[(int64_t)(2 * i + 1) * nslope + s];
-    imat[s + (int64_t)(a0 + i) * nslope] = (sp - sm) / (2.f * push);
+  ImatSource src{A, list, slopes, -1, P.npup, 0, 0, 0};
+  imat_images<NFFT, PD>(P, src, n, S, smem, L);
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const int k = k0 + i;
+    flat[P.c_order ? 2 * k : k] = slopes[i].x;
+    flat[P.c_order ? 2 * k + 1 : k + P.nvalid] = slopes[i].y;
   }
 }
 
 template <int NFFT, int PD>
-static void launch_imat_sh(const ShKernelArgs &P, int nvalid, int S, size_t sm, int npoke, int64_t stride,
-                           int nslope, cudaStream_t s) {
-  const int gx = std::max(1, (nvalid + S - 1) / S);
-  smem_opt_in(reinterpret_cast<const void *>(imat_sh_kernel<NFFT, PD>), (int)std::max<size_t>(sm, 48 * 1024));
-  imat_sh_kernel<NFFT, PD><<<dim3(gx, npoke), IMAT_SH_THREADS, sm, s>>>(P, S, stride, nslope);
+__global__ void __launch_bounds__(IMAT_THREADS) imat_kernel(ShKernelArgs P, ImatArgs A, int S) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ int s_n;
+  const int pd = PD > 0 ? PD : P.pdiam;
+  const ShSmem L(NFFT, P.nu, P.nv, pd, P.nrebin2 * P.npix * P.npix, P.npix * P.npix, S);
+  float2 *slopes = reinterpret_cast<float2 *>(smem + ShSmem::align16(L.bytes()));
+  int *list = reinterpret_cast<int *>(slopes + 2 * IMAT_LIST);
+  sh_load_tables<NFFT>(P, smem, threadIdx.x, blockDim.x);
+  const int a = blockIdx.x;
+  ImatSource src{A, list, slopes, a, P.npup, 0, __ldg(A.i1 + a), __ldg(A.j1 + a)};
+  const int nvalid = P.nvalid;
+  float *col = A.imat + (int64_t)a * 2 * nvalid;
+  if (threadIdx.x == 0) s_n = 0;
+  __syncthreads();
+  for (int base = 0; base < nvalid; base += IMAT_THREADS) {
+    const int k = base + (int)threadIdx.x;
+    if (k < nvalid) {
+      if (src.reaches(__ldg(P.puppixx + k), __ldg(P.puppixy + k), pd)) {
+        list[atomicAdd(&s_n, 1)] = k;  // (the order within the list does not matter to any value)
+      } else {
+        const int ix = P.c_order ? 2 * k : k, iy = P.c_order ? 2 * k + 1 : k + nvalid;
+        const float fx = __ldg(A.flat + ix), fy = __ldg(A.flat + iy);
+        col[ix] = (fx - fx) / (2.f * A.push);
+        col[iy] = (fy - fy) / (2.f * A.push);
+      }
+    }
+    __syncthreads();
+    const int n = s_n;
+    if (n + IMAT_THREADS > IMAT_LIST || base + IMAT_THREADS >= nvalid) {
+      imat_images<NFFT, PD>(P, src, 2 * n, S, smem, L);
+      for (int j = threadIdx.x; j < n; j += IMAT_THREADS) {
+        const int m = list[j];
+        const float2 sp = slopes[2 * j], sm = slopes[2 * j + 1];
+        col[P.c_order ? 2 * m : m] = (sp.x - sm.x) / (2.f * A.push);
+        col[P.c_order ? 2 * m + 1 : m + nvalid] = (sp.y - sm.y) / (2.f * A.push);
+      }
+      if (threadIdx.x == 0) s_n = 0;
+      __syncthreads();
+    }
+  }
+}
+
+template <int NFFT, int PD>
+static void launch_imat(const ShKernelArgs &P, const ImatArgs &A, int nact, int S, size_t sm, float *flat,
+                        cudaStream_t s) {
+  const int lim = (int)std::max<size_t>(sm, 48 * 1024);
+  smem_opt_in(reinterpret_cast<const void *>(imat_flat_kernel<NFFT, PD>), lim);
+  smem_opt_in(reinterpret_cast<const void *>(imat_kernel<NFFT, PD>), lim);
+  imat_flat_kernel<NFFT, PD><<<(P.nvalid + IMAT_ITEMS - 1) / IMAT_ITEMS, IMAT_THREADS, sm, s>>>(P, A, S, flat);
+  AOB_LAUNCH_CHECK("imat_flat_kernel");
+  imat_kernel<NFFT, PD><<<nact, IMAT_THREADS, sm, s>>>(P, A, S);
+  AOB_LAUNCH_CHECK("imat_kernel");
 }
 template <int NFFT>
-static void launch_imat_sh_pd(const ShKernelArgs &P, int nvalid, int S, size_t sm, int npoke, int64_t stride,
-                              int nslope, cudaStream_t s) {
+static void launch_imat_pd(const ShKernelArgs &P, const ImatArgs &A, int nact, int S, size_t sm, float *flat,
+                           cudaStream_t s) {
   switch (P.pdiam) {
-    case 4: launch_imat_sh<NFFT, 4>(P, nvalid, S, sm, npoke, stride, nslope, s); break;
-    case 6: launch_imat_sh<NFFT, 6>(P, nvalid, S, sm, npoke, stride, nslope, s); break;
-    case 8: launch_imat_sh<NFFT, 8>(P, nvalid, S, sm, npoke, stride, nslope, s); break;
-    default: launch_imat_sh<NFFT, 0>(P, nvalid, S, sm, npoke, stride, nslope, s); break;
+    case 4: launch_imat<NFFT, 4>(P, A, nact, S, sm, flat, s); break;
+    case 6: launch_imat<NFFT, 6>(P, A, nact, S, sm, flat, s); break;
+    case 8: launch_imat<NFFT, 8>(P, A, nact, S, sm, flat, s); break;
+    default: launch_imat<NFFT, 0>(P, A, nact, S, sm, flat, s); break;
   }
 }
 
@@ -130,40 +199,31 @@ extern "C" int aob_imat_build(aob_sh *w, aob_centro *c, aob_dm *dm, float xoff, 
     // the reference forms the calibration images with nphot4imat photons
     // (SutraRtc::comp_images_imat, sutra_rtc.cpp:380-395); 0 keeps nphot
     if (w->nphot4imat > 0.f) P.nphot = w->nphot4imat;
-    const int nact = dm->nact, nslope = 2 * w->nvalid;
+    const int nact = dm->nact;
     const int per = chunk > 0 ? std::min(chunk, nact) : nact;
     AOB_REQUIRE(2 * (int64_t)per <= 65535, "aob_imat_build: at most 32767 actuators per chunk");
-    const int64_t npix = (int64_t)dm->dim * dm->dim, nphase = (int64_t)w->npup * w->npup;
-    DevBuf<float> shapes(2 * per * npix), phases(2 * per * nphase), slopes(2 * (int64_t)per * nslope),
-        inten(2 * (int64_t)per * w->nvalid);
-    const int S = w->pick_batch();
-    const size_t sm = w->smem_bytes(S);
-    P.bincube = nullptr;  // slopes only
-    P.binimg = nullptr;
-    P.phase = phases.p;
-    P.c_slopes = slopes.p;
-    P.intensities = inten.p;
-    for (int a0 = 0; a0 < nact; a0 += per) {
-      const int cnt = std::min(per, nact - a0), npoke = 2 * cnt;
-      const int gx = (int)std::min<int64_t>((npix + 255) / 256, 1024);
-      imat_dm_kernel<<<dim3(gx, npoke), 256, 0, s>>>(shapes.p, npix, dm->rowptr.p, dm->actidx.p, dm->weight.p, a0,
-                                                      push);
-      AOB_LAUNCH_CHECK("imat_dm_kernel");
-      const dim3 tb(16, 16), tg((w->npup + 15) / 16, (w->npup + 15) / 16, npoke);
-      imat_trace_kernel<<<tg, tb, 0, s>>>(phases.p, w->npup, shapes.p, dm->dim, xoff, yoff);
-      AOB_LAUNCH_CHECK("imat_trace_kernel");
-      if (w->nfft == 16)
-        launch_imat_sh_pd<16>(P, w->nvalid, S, sm, npoke, nphase, nslope, s);
-      else if (w->nfft == 32)
-        launch_imat_sh_pd<32>(P, w->nvalid, S, sm, npoke, nphase, nslope, s);
-      else
-        launch_imat_sh_pd<64>(P, w->nvalid, S, sm, npoke, nphase, nslope, s);
-      AOB_LAUNCH_CHECK("imat_sh_kernel");
-      const int64_t nd = (int64_t)nslope * cnt;
-      imat_diff_kernel<<<(int)std::min<int64_t>((nd + 255) / 256, 4096), 256, 0, s>>>(dev_imat, slopes.p, nslope, a0,
-                                                                                      cnt, push);
-      AOB_LAUNCH_CHECK("imat_diff_kernel");
-    }
+    DevBuf<float> flat(2 * (int64_t)w->nvalid);
+    ImatArgs A{};
+    A.influ = dm->influ.p;
+    A.i1 = dm->i1.p;
+    A.j1 = dm->j1.p;
+    A.isz = dm->influsize;
+    A.dim = dm->dim;
+    A.xoff = xoff;
+    A.yoff = yoff;
+    A.push = push;
+    A.flat = flat.p;
+    A.imat = dev_imat;
+    // images per batch: as many as leave room for several CTAs on an SM
+    int S = IMAT_ITEMS;
+    while (S > 1 && w->smem_bytes(S) + IMAT_LIST_BYTES > 56 * 1024) --S;
+    const size_t sm = ShSmem::align16(w->smem_bytes(S)) + IMAT_LIST_BYTES;
+    if (w->nfft == 16)
+      launch_imat_pd<16>(P, A, nact, S, sm, flat.p, s);
+    else if (w->nfft == 32)
+      launch_imat_pd<32>(P, A, nact, S, sm, flat.p, s);
+    else
+      launch_imat_pd<64>(P, A, nact, S, sm, flat.p, s);
     // the scratch is released below: wait for the launches that read it
     AOB_CUDA(cudaStreamSynchronize(s));
     return AOB_OK;

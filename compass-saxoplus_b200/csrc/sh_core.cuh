@@ -171,6 +171,16 @@ struct NoHook {
   __device__ void operator()() const {}
 };
 
+// Where a batch's sub-apertures come from.  The default: sub-aperture s of the
+// batch is base + s * stride of the sensor and reads the sensor's phase.  A
+// source with LISTED = true (the interaction matrix, imat.cu) names each
+// item's sub-aperture itself, forms its phase (phase(s, X, Y), X and Y on the
+// sensor's phase grid) and takes its slopes (store(s, x, y)); nothing else of
+// such an item is written.
+struct ShStrided {
+  static constexpr bool LISTED = false;
+};
+
 // Where sh_batch keeps the batch's metadata in its work area.
 struct ShMeta {
   int32_t *vx, *vy;
@@ -191,7 +201,6 @@ struct ShMeta {
 // cube (contiguous) and its npix x npix window of the binned image.
 __device__ __forceinline__ void sh_store_subap(const ShKernelArgs &P, int k, const float *bs, int vx, int vy,
                                                int lane) {
-  if (!P.bincube) return;  // (slopes only: the batched interaction-matrix images keep no cube or image)
   const int npix = P.npix, npix2 = npix * npix;
   for (int p = lane; p < npix2; p += 32) {
     const float v = bs[p];
@@ -222,10 +231,17 @@ __device__ __forceinline__ void sh_store_images(const ShKernelArgs &P, int base,
 // thread of the team once the field stage is complete (its global loads have
 // returned), before the DFTs.  With DEFER_IMG the cube and image writes are
 // left to sh_store_images (the noisy pixels stay in the work area).
-template <int NFFT, int PD, int TK = TEAM_CTA, class Hook = NoHook, bool DEFER_IMG = false, bool FS = false>
+template <int NFFT, int PD, int TK = TEAM_CTA, class Hook = NoHook, bool DEFER_IMG = false, bool FS = false,
+          class Src = ShStrided>
 __device__ __forceinline__ void sh_batch(const ShKernelArgs &P, int base, int stride, int S,
                                          const unsigned char *tables, unsigned char *work, const ShSmem &L,
-                                         const Team &T, const Hook &after_field = Hook{}) {
+                                         const Team &T, const Hook &after_field = Hook{}, const Src &src = Src{}) {
+  auto sub = [&](int s) {
+    if constexpr (Src::LISTED)
+      return src.sub(s);
+    else
+      return base + s * stride;
+  };
   const int tid = TK == TEAM_CTA ? (int)threadIdx.x : T.tid;
   const int nt = TK == TEAM_CTA ? (int)blockDim.x : (TK == TEAM_WARP ? 32 : T.nt);
   const int lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
@@ -261,7 +277,7 @@ __device__ __forceinline__ void sh_batch(const ShKernelArgs &P, int base, int st
   const int t0 = max(0, min(nE, nt - S));
   for (int mt = tid - t0; mt < S; mt += nt) {
     if (mt < 0) break;
-    const int k = base + mt * stride;
+    const int k = sub(mt);
     const int vx = __ldg(P.validsubsx + k), vy = __ldg(P.validsubsy + k);
     const float fl = __ldg(P.flux + k);
     float rx = 0.f, ry = 0.f;
@@ -294,7 +310,7 @@ __device__ __forceinline__ void sh_batch(const ShKernelArgs &P, int base, int st
           const int l = i - s * pd2;
           const int y = PD > 0 ? l / PD : udiv(l, P.mg_pd);
           const int x = l - y * pd;
-          const int k = base + s * stride;
+          const int k = sub(s);
           fv[j] = P.fs_field[(x + __ldg(P.puppixx + k)) + (y + __ldg(P.puppixy + k)) * P.fs_n];
           of[j] = __ldg(P.offsets + l);
         }
@@ -320,9 +336,13 @@ __device__ __forceinline__ void sh_batch(const ShKernelArgs &P, int base, int st
         const int l = i - s * pd2;
         const int y = PD > 0 ? l / PD : udiv(l, P.mg_pd);
         const int x = l - y * pd;
-        const int k = base + s * stride;
-        const int id = (x + __ldg(P.puppixx + k)) + (y + __ldg(P.puppixy + k)) * P.npup;
-        ph[j] = __ldcg(P.phase + id);  // (L2: a resident kernel reads a new phase every step)
+        const int k = sub(s);
+        const int X = x + __ldg(P.puppixx + k), Y = y + __ldg(P.puppixy + k);
+        const int id = X + Y * P.npup;
+        if constexpr (Src::LISTED)
+          ph[j] = src.phase(s, X, Y);
+        else
+          ph[j] = __ldcg(P.phase + id);  // (L2: a resident kernel reads a new phase every step)
         am[j] = __ldg(P.pupil + id);
         of[j] = __ldg(P.offsets + l);
       }
@@ -463,7 +483,7 @@ __device__ __forceinline__ void sh_batch(const ShKernelArgs &P, int base, int st
     part = warp_sum(part);
     if (lane == 0) {
       m_tot[s] = part;
-      P.intensities[base + s * stride] = part;
+      if constexpr (!Src::LISTED) P.intensities[base + s * stride] = part;
     }
     // normalise in place; with photon noise list the pixels by sampler
     // (inversion from the front of `order`, PTRS from the back) so that the
@@ -498,7 +518,7 @@ __device__ __forceinline__ void sh_batch(const ShKernelArgs &P, int base, int st
   for (int t = tid; t < nP; t += nt) {
     const int i = P.noise_mode >= 1 ? order[t] : t;
     const int s = udiv(i, P.mg_np2), p = i - s * npix2;
-    const int k = base + s * stride;
+    const int k = sub(s);
     float wgt = 1.f;
     if (P.ckind == 2) wgt = P.c_wper ? P.c_weights[p + k * npix2] : wt[p];
     float v = bins[i];
@@ -530,15 +550,21 @@ __device__ __forceinline__ void sh_batch(const ShKernelArgs &P, int base, int st
       cx = warp_sum(cx);
       cy = warp_sum(cy);
       if (lane == 0) {
-        const int k = base + s * stride;
+        const int k = sub(s);
         const int ix = P.c_order ? 2 * k : k;
         const int iy = P.c_order ? 2 * k + 1 : k + P.nvalid;
-        P.c_slopes[ix] = (cx / (cs + 1.e-6f) - P.c_offset) * P.c_scale - m_rx[s];
-        P.c_slopes[iy] = (cy / (cs + 1.e-6f) - P.c_offset) * P.c_scale - m_ry[s];
-        P.c_intens[k] = cs;
+        const float sx = (cx / (cs + 1.e-6f) - P.c_offset) * P.c_scale - m_rx[s];
+        const float sy = (cy / (cs + 1.e-6f) - P.c_offset) * P.c_scale - m_ry[s];
+        if constexpr (Src::LISTED) {
+          src.store(s, sx, sy);
+        } else {
+          P.c_slopes[ix] = sx;
+          P.c_slopes[iy] = sy;
+          P.c_intens[k] = cs;
+        }
       }
     }
-    if constexpr (!DEFER_IMG) sh_store_subap(P, base + s * stride, bins + s * npix2, m_vx[s], m_vy[s], lane);
+    if constexpr (!DEFER_IMG && !Src::LISTED) sh_store_subap(P, base + s * stride, bins + s * npix2, m_vx[s], m_vy[s], lane);
   }
   team_sync<TK>(T);
 }

@@ -231,15 +231,11 @@ __global__ void raytrace_kernel(float *out, int nx, int ny, RaySources S, int re
   float acc = reset ? 0.f : out[x + y * nx];
   for (int l = 0; l < S.n; ++l) {
     const int N = S.dim[l];
-    const float xref = (float)x - nx / 2.0f + nx / 2.0f + S.xoff[l];
-    const float yref = (float)y - ny / 2.0f + ny / 2.0f + S.yoff[l];
+    const float xref = ray_position(x, nx, S.xoff[l]), yref = ray_position(y, ny, S.yoff[l]);
     const int iref = (int)xref, jref = (int)yref;
-    const float xs = xref - iref, ys = yref - jref;
-    const float wx1 = 1.0f - xs, wx2 = xs, wy1 = 1.0f - ys, wy2 = ys;
     if (iref + 1 < N && jref + 1 < N) {
-      const float *d = S.data[l];
-      acc += (wx1 * wy1 * d[iref + jref * N] + wx2 * wy1 * d[iref + 1 + jref * N] +
-              wx1 * wy2 * d[iref + (jref + 1) * N] + wx2 * wy2 * d[iref + 1 + (jref + 1) * N]);
+      const float *d = S.data[l] + iref + jref * N;
+      acc += ray_bilinear(xref - iref, yref - jref, d[0], d[1], d[N], d[N + 1]);
     } else {
       acc += 0.0f;
     }
@@ -546,18 +542,25 @@ void aob::kolmo_factor_ab(int device, int n, int nst, const double *zz, const do
 }
 
 // =================================================================== DM
-aob_dm::aob_dm(int device_, int dim_, int nact_, int isz, const float *influ, const int32_t *i1, const int32_t *j1)
+aob_dm::aob_dm(int device_, int dim_, int nact_, int isz, const float *h_influ, const int32_t *h_i1,
+               const int32_t *h_j1)
     : device(device_), dim(dim_), nact(nact_), influsize(isz) {
   AOB_REQUIRE(dim > 0 && nact > 0 && isz > 0, "dm: sizes must be > 0");
-  AOB_REQUIRE(influ && i1 && j1, "dm: null arrays");
+  AOB_REQUIRE(h_influ && h_i1 && h_j1, "dm: null arrays");
   AOB_CUDA(cudaSetDevice(device));
+  influ.alloc((int64_t)isz * isz * nact);
+  influ.upload(h_influ, influ.n);
+  i1.alloc(nact);
+  i1.upload(h_i1, nact);
+  j1.alloc(nact);
+  j1.upload(h_j1, nact);
   // pixel-major CSR: pixel (i1[a]+x, j1[a]+y) receives influ[x, y, a] * com[a]
   const int64_t npix = (int64_t)dim * dim;
   std::vector<int32_t> cnt(npix + 1, 0);
   for (int a = 0; a < nact; ++a)
     for (int y = 0; y < isz; ++y)
       for (int x = 0; x < isz; ++x) {
-        const int px = i1[a] + x, py = j1[a] + y;
+        const int px = h_i1[a] + x, py = h_j1[a] + y;
         if (px >= 0 && px < dim && py >= 0 && py < dim) ++cnt[px + (int64_t)py * dim + 1];
       }
   for (int64_t p = 0; p < npix; ++p) cnt[p + 1] += cnt[p];
@@ -567,12 +570,12 @@ aob_dm::aob_dm(int device_, int dim_, int nact_, int isz, const float *influ, co
   for (int a = 0; a < nact; ++a)
     for (int y = 0; y < isz; ++y)
       for (int x = 0; x < isz; ++x) {
-        const int px = i1[a] + x, py = j1[a] + y;
+        const int px = h_i1[a] + x, py = h_j1[a] + y;
         if (px >= 0 && px < dim && py >= 0 && py < dim) {
           const int64_t p = px + (int64_t)py * dim;
           const int32_t k = fill[p]++;
           act[k] = a;
-          w[k] = influ[x + (size_t)y * isz + (size_t)a * isz * isz];
+          w[k] = h_influ[x + (size_t)y * isz + (size_t)a * isz * isz];
         }
       }
   rowptr.alloc(npix + 1);

@@ -16,6 +16,17 @@ struct RaySources {
   float xoff[RAY_MAX], yoff[RAY_MAX];
 };
 
+// Where a sample of the phase grid falls on a screen (generic_raytrace): the
+// screen's lower sample and the fraction past it, along one axis.
+__device__ __forceinline__ float ray_position(int i, int n, float off) {
+  return (float)i - n / 2.0f + n / 2.0f + off;
+}
+// Bilinear sum of four screen samples at the fractions xs, ys past the lower one.
+__device__ __forceinline__ float ray_bilinear(float xs, float ys, float d00, float d10, float d01, float d11) {
+  const float wx1 = 1.0f - xs, wx2 = xs, wy1 = 1.0f - ys, wy2 = ys;
+  return wx1 * wy1 * d00 + wx2 * wy1 * d10 + wx1 * wy2 * d01 + wx2 * wy2 * d11;
+}
+
 void raytrace(float *out, int nx, int ny, const RaySources &S, bool reset, cudaStream_t s);
 
 // One extrusion step (sim.cu): the new column/row y = A z + amp B xi + ref from the
@@ -78,6 +89,11 @@ struct aob_dm {
   int64_t nnz = 0;
   aob::DevBuf<int32_t> rowptr, actidx;
   aob::DevBuf<float> weight, shape, com;
+  // the influence functions as they were given: influsize^2 per actuator, x
+  // fastest, lower-left pixel (i1, j1) on the screen (the interaction matrix
+  // pokes one actuator at a time and needs its patch only)
+  aob::DevBuf<float> influ;
+  aob::DevBuf<int32_t> i1, j1;
   aob_dm(int device, int dim, int nact, int influsize, const float *influ, const int32_t *i1, const int32_t *j1);
   void comp_shape(const float *dev_com, cudaStream_t s);
 };
