@@ -1,15 +1,15 @@
-// Batched complex 2-D FFT for power-of-two sizes (16 .. 2048), single
-// precision, in place.  Used for the target PSF and the pyramid sensor.
+// Batched complex 2-D FFT for power-of-two sizes (8 .. 2048), single
+// precision, in place.  Used for the target PSF and the SH field stop.
 //
-// Row pass: one CTA per row, the row staged in shared memory, Stockham
-// radix-8 passes with the butterflies in registers (fft.cuh), written back.
-// Column pass: one CTA per group of 8 adjacent columns (64-byte row segments,
-// coalesced), the same transform per column in shared memory.  Twiddles come from a table computed
-// in double on the host.  Sign convention of cuFFT: forward = exp(-2 pi i k m / n),
-// inverse = exp(+2 pi i k m / n), both unnormalised.
+// Row pass: T = N / 8 threads per row, 256 threads per CTA; column pass: up to 8
+// adjacent columns per CTA (64-byte row segments).  Both hold the transform
+// in registers (fft.cuh) and read and write global memory once.  Twiddles come
+// from a table computed in double on the host.  Sign convention of cuFFT: forward
+// = exp(-2 pi i k m / n), inverse = exp(+2 pi i k m / n), both unnormalised.
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <map>
 #include <mutex>
@@ -44,47 +44,78 @@ const float2 *fft_twiddles(int device, int n) {
   return b->p;
 }
 
-__global__ void fft_rows_kernel(float2 *data, int n, int logn, const float2 *tw, int inverse) {
-  extern __shared__ float2 srow[];
-  float2 *row = data + (size_t)blockIdx.x * n;  // blockIdx.x = row index over the whole batch
-  for (int i = threadIdx.x; i < n; i += blockDim.x) srow[i] = row[i];
-  __syncthreads();
-  smem_fft_stockham<1>(srow, n, 1, tw, inverse != 0);
-  for (int i = threadIdx.x; i < n; i += blockDim.x) row[i] = srow[i];
+constexpr int FFT_ROW_THREADS = 256;
+
+template <int N, bool INV>
+__global__ void __launch_bounds__(FFT_ROW_THREADS) fft_rows_kernel(float2 *data, int64_t nrows, const float2 *tw) {
+  constexpr int T = N / 8, SEQ = FFT_ROW_THREADS / T, BS = fft_smem_elems(N);
+  __shared__ float2 s[BS > 0 ? SEQ * 2 * BS : 1];
+  const int g = threadIdx.x / T, j = threadIdx.x % T;
+  const int64_t r = (int64_t)blockIdx.x * SEQ + g;
+  float2 *row = data + r * N;
+  float2 v[8];
+#pragma unroll
+  for (int m = 0; m < 8; ++m) v[m] = r < nrows ? row[j + T * m] : make_float2(0.f, 0.f);
+  FftTw<N> W;
+  W.load(tw, j);
+  fft_regs<N, 1, BS, INV>(v, W, j, s + g * 2 * BS, GroupSync<T>{g});
+  if (r < nrows) {
+#pragma unroll
+    for (int m = 0; m < 8; ++m) row[j + T * m] = v[m];
+  }
 }
 
-constexpr int FFT_COLS = 8;
+// columns per CTA: 8, fewer where 8 would pass 512 threads
+constexpr int fft_cols(int n) { return n <= 512 ? 8 : 4096 / n; }
 
-__global__ void fft_cols_kernel(float2 *data, int n, int logn, const float2 *tw, int inverse) {
+template <int N, bool INV>
+__global__ void __launch_bounds__(N / 8 * fft_cols(N)) fft_cols_kernel(float2 *data, const float2 *tw) {
   extern __shared__ float2 scol[];
-  const int groups = n / FFT_COLS;
+  constexpr int T = N / 8, CB = fft_cols(N), BS = fft_smem_elems(N) * CB;
+  constexpr int groups = N / CB;
   const int img = blockIdx.x / groups;
-  const int c0 = (blockIdx.x - img * groups) * FFT_COLS;
-  float2 *base = data + (size_t)img * n * n + c0;
-  for (int t = threadIdx.x; t < n * FFT_COLS; t += blockDim.x) {
-    const int m = t / FFT_COLS, c = t - m * FFT_COLS;
-    scol[m * FFT_COLS + c] = base[(size_t)m * n + c];
-  }
-  __syncthreads();
-  smem_fft_stockham<4>(scol, n, FFT_COLS, tw, inverse != 0);
-  for (int t = threadIdx.x; t < n * FFT_COLS; t += blockDim.x) {
-    const int m = t / FFT_COLS, c = t - m * FFT_COLS;
-    base[(size_t)m * n + c] = scol[m * FFT_COLS + c];
-  }
+  const int c = threadIdx.x % CB, j = threadIdx.x / CB;
+  float2 *base = data + (size_t)img * N * N + (blockIdx.x - img * groups) * CB + c;
+  float2 v[8];
+#pragma unroll
+  for (int m = 0; m < 8; ++m) v[m] = base[(size_t)(j + T * m) * N];
+  FftTw<N> W;
+  W.load(tw, j);
+  fft_regs<N, CB, BS, INV>(v, W, j, scol + c, CtaSync{});
+#pragma unroll
+  for (int m = 0; m < 8; ++m) base[(size_t)(j + T * m) * N] = v[m];
+}
+
+template <int N, bool INV>
+static void fft2d_n(float2 *data, int batch, const float2 *tw, cudaStream_t s) {
+  constexpr int SEQ = FFT_ROW_THREADS / (N / 8);
+  const int64_t nrows = (int64_t)N * batch;
+  fft_rows_kernel<N, INV><<<(unsigned)((nrows + SEQ - 1) / SEQ), FFT_ROW_THREADS, 0, s>>>(data, nrows, tw);
+  AOB_LAUNCH_CHECK("fft_rows_kernel");
+  constexpr int sm = (int)sizeof(float2) * 2 * fft_smem_elems(N) * fft_cols(N);
+  smem_opt_in(reinterpret_cast<const void *>(fft_cols_kernel<N, INV>), std::max(sm, 48 * 1024));
+  fft_cols_kernel<N, INV><<<(unsigned)(N / fft_cols(N) * batch), N / 8 * fft_cols(N), sm, s>>>(data, tw);
+  AOB_LAUNCH_CHECK("fft_cols_kernel");
 }
 
 void fft2d(float2 *data, int n, int batch, bool inverse, int device, cudaStream_t s) {
-  AOB_REQUIRE(n >= FFT_COLS && n <= 2048 && (n & (n - 1)) == 0, "fft2d: n must be a power of two in [8, 2048]");
-  int logn = 0;
-  while ((1 << logn) < n) ++logn;
+  AOB_REQUIRE(n >= 8 && n <= 2048 && (n & (n - 1)) == 0, "fft2d: n must be a power of two in [8, 2048]");
   const float2 *tw = fft_twiddles(device, n);
-  smem_opt_in(reinterpret_cast<const void *>(fft_cols_kernel), 2048 * FFT_COLS * 8);
-  const int thr = std::min(512, std::max(32, n / 2));
-  fft_rows_kernel<<<n * batch, thr, n * sizeof(float2), s>>>(data, n, logn, tw, inverse ? 1 : 0);
-  AOB_LAUNCH_CHECK("fft_rows_kernel");
-  fft_cols_kernel<<<(n / FFT_COLS) * batch, 512, n * FFT_COLS * sizeof(float2), s>>>(data, n, logn, tw,
-                                                                                      inverse ? 1 : 0);
-  AOB_LAUNCH_CHECK("fft_cols_kernel");
+  auto go = [&](auto size) {
+    constexpr int N = decltype(size)::value;
+    inverse ? fft2d_n<N, true>(data, batch, tw, s) : fft2d_n<N, false>(data, batch, tw, s);
+  };
+  switch (n) {
+    case 8: go(std::integral_constant<int, 8>{}); break;
+    case 16: go(std::integral_constant<int, 16>{}); break;
+    case 32: go(std::integral_constant<int, 32>{}); break;
+    case 64: go(std::integral_constant<int, 64>{}); break;
+    case 128: go(std::integral_constant<int, 128>{}); break;
+    case 256: go(std::integral_constant<int, 256>{}); break;
+    case 512: go(std::integral_constant<int, 512>{}); break;
+    case 1024: go(std::integral_constant<int, 1024>{}); break;
+    default: go(std::integral_constant<int, 2048>{}); break;
+  }
 }
 
 }  // namespace aob

@@ -1,218 +1,175 @@
-// Batched in-place complex 2-D FFT (fft.cu).
+// Complex FFTs held in registers (device code) and the batched in-place 2-D
+// transform (fft.cu).
 #pragma once
 
 #include <cuda_runtime.h>
 
 namespace aob {
 
-__device__ __forceinline__ uint32_t bitrev(uint32_t x, int logn) { return __brev(x) >> (32 - logn); }
-
 // ---------------------------------------------------------------------------
-// Stockham auto-sort FFT in shared memory (natural order in and out), radix-8
-// passes with the butterflies in registers and a last radix-2 or radix-4 pass
-// when n is not a power of 8 (Govindaraju et al., "High performance discrete
-// Fourier transforms on graphics processors", SC'08).  ``cols`` interleaved
-// sequences: element m of sequence c is s[m * cols + c] (consecutive threads
-// take consecutive c, so accesses are contiguous).  Pass with current
-// sub-transform length ns: butterfly j of sequence c reads s[j + r n/R],
-// multiplies by W_(ns R)^(r (j mod ns)), transforms in registers and writes
-// to ((j / ns) ns R + j mod ns) + r ns.  cuFFT sign convention (forward
-// exp(-2 pi i k m / n)), unnormalised.  tw: exp(-2 pi i m / n), m < n/2.
+// A length-N transform (N a power of two, 8 .. 2048) by a group of T = N / 8
+// threads, thread j holding elements j + T m in v[m] (m < 8), natural order in
+// and out: Stockham radix-8 passes, a last radix-2 or radix-4 pass when N is not
+// a power of 8 (Govindaraju et al., "High performance discrete Fourier transforms
+// on graphics processors", SC'08).  The first pass's inputs and the last pass's
+// outputs are the thread's own elements, so a transform touches shared memory
+// only between passes (twice for N = 512) and global memory is read and
+// written straight from registers, T consecutive elements at a time.
+//   pass with sub-transform length NS: butterfly j takes elements j + r N / R,
+//   multiplies by W_(NS R)^(r (j mod NS)) and gives (j / NS) NS R + j mod NS + r NS.
+// cuFFT sign convention (forward exp(-2 pi i k m / N)), unnormalised.
 
 __device__ __forceinline__ float2 c_add(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ float2 c_sub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
-__device__ __forceinline__ float2 c_mul(float2 a, float2 b) {
-  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+// a * w, or a * conj(w) for the inverse transform
+template <bool INV>
+__device__ __forceinline__ float2 c_mulw(float2 a, float2 w) {
+  return INV ? make_float2(a.x * w.x + a.y * w.y, a.y * w.x - a.x * w.y)
+             : make_float2(a.x * w.x - a.y * w.y, a.x * w.y + a.y * w.x);
 }
 // multiply by -i (forward) or +i (inverse)
-__device__ __forceinline__ float2 c_rot(float2 a, bool inverse) {
-  return inverse ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);
+template <bool INV>
+__device__ __forceinline__ float2 c_rot(float2 a) {
+  return INV ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);
 }
 
-template <int R>
-__device__ __forceinline__ void dft_small(float2 *v, bool inverse);
-template <>
-__device__ __forceinline__ void dft_small<2>(float2 *v, bool) {
-  const float2 a = v[0], b = v[1];
-  v[0] = c_add(a, b);
-  v[1] = c_sub(a, b);
+template <bool INV>
+__device__ __forceinline__ void dft2(float2 &a, float2 &b) {
+  const float2 t = a;
+  a = c_add(t, b);
+  b = c_sub(t, b);
 }
-template <>
-__device__ __forceinline__ void dft_small<4>(float2 *v, bool inverse) {
-  const float2 t0 = c_add(v[0], v[2]), t1 = c_sub(v[0], v[2]);
-  const float2 t2 = c_add(v[1], v[3]), t3 = c_rot(c_sub(v[1], v[3]), inverse);
-  v[0] = c_add(t0, t2);
-  v[2] = c_sub(t0, t2);
-  v[1] = c_add(t1, t3);
-  v[3] = c_sub(t1, t3);
+template <bool INV>
+__device__ __forceinline__ void dft4(float2 &a, float2 &b, float2 &c, float2 &d) {
+  const float2 t0 = c_add(a, c), t1 = c_sub(a, c);
+  const float2 t2 = c_add(b, d), t3 = c_rot<INV>(c_sub(b, d));
+  a = c_add(t0, t2);
+  c = c_sub(t0, t2);
+  b = c_add(t1, t3);
+  d = c_sub(t1, t3);
 }
-template <>
-__device__ __forceinline__ void dft_small<8>(float2 *v, bool inverse) {
-  float2 e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
-  dft_small<4>(e, inverse);
-  dft_small<4>(o, inverse);
+template <bool INV>
+__device__ __forceinline__ void dft8(float2 (&v)[8]) {
+  dft4<INV>(v[0], v[2], v[4], v[6]);
+  dft4<INV>(v[1], v[3], v[5], v[7]);
   const float h = 0.70710678118654752f;  // cos(pi / 4)
-  const float sg = inverse ? 1.f : -1.f;
-  // W8^k o[k]: W8 = exp(-/+ i pi / 4)
-  const float2 o1 = make_float2(h * (o[1].x - sg * o[1].y), h * (o[1].y + sg * o[1].x));
-  const float2 o2 = c_rot(o[2], inverse);
-  const float2 o3 = make_float2(h * (-o[3].x - sg * o[3].y), h * (-o[3].y + sg * o[3].x));
-  v[0] = c_add(e[0], o[0]);
-  v[4] = c_sub(e[0], o[0]);
-  v[1] = c_add(e[1], o1);
-  v[5] = c_sub(e[1], o1);
-  v[2] = c_add(e[2], o2);
-  v[6] = c_sub(e[2], o2);
-  v[3] = c_add(e[3], o3);
-  v[7] = c_sub(e[3], o3);
+  const float sg = INV ? 1.f : -1.f;
+  // odd outputs times W8^k: W8 = exp(-/+ i pi / 4)
+  const float2 o1 = make_float2(h * (v[3].x - sg * v[3].y), h * (v[3].y + sg * v[3].x));
+  const float2 o2 = c_rot<INV>(v[5]);
+  const float2 o3 = make_float2(h * (-v[7].x - sg * v[7].y), h * (-v[7].y + sg * v[7].x));
+  const float2 e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6], o0 = v[1];
+  v[0] = c_add(e0, o0);
+  v[4] = c_sub(e0, o0);
+  v[1] = c_add(e1, o1);
+  v[5] = c_sub(e1, o1);
+  v[2] = c_add(e2, o2);
+  v[6] = c_sub(e2, o2);
+  v[3] = c_add(e3, o3);
+  v[7] = c_sub(e3, o3);
 }
 
-// W_n^m for 0 <= m < n from the half table
-__device__ __forceinline__ float2 fft_twiddle(const float2 *tw, int n, int m, bool inverse) {
-  float2 w = m < (n >> 1) ? __ldg(tw + m) : __ldg(tw + (m - (n >> 1)));
-  if (m >= (n >> 1)) w = make_float2(-w.x, -w.y);
-  if (inverse) w.y = -w.y;
-  return w;
-}
+constexpr int fft_passes(int n) { return n <= 8 ? 1 : (n <= 64 ? 2 : (n <= 512 ? 3 : 4)); }
+// Padded position of element i in shared memory: one slot skipped every eight, so
+// that the strided writes after a radix-8 pass fall on different banks.
+__device__ __forceinline__ int fft_pad(int i) { return i + (i >> 3); }
+constexpr int fft_smem_elems(int n) { return n > 8 ? n + n / 8 : 0; }  // per sequence and buffer
 
-// One Stockham pass of radix R; every thread handles at most MAXT butterflies.
-template <int R, int MAXT>
-__device__ __forceinline__ void stockham_pass(float2 *s, int n, int cols, int ns, const float2 *tw, bool inverse) {
-  const int nb = n / R;
-  const int tasks = nb * cols;
-  float2 v[MAXT][R];
-#pragma unroll
-  for (int it = 0; it < MAXT; ++it) {
-    const int t = threadIdx.x + it * blockDim.x;
-    if (t < tasks) {
-      const int j = t / cols, c = t - j * cols;
-#pragma unroll
-      for (int r = 0; r < R; ++r) v[it][r] = s[(j + r * nb) * cols + c];
-      const int k = j & (ns - 1);
-      if (ns > 1) {
-        const int step = k * (n / (ns * R));
-#pragma unroll
-        for (int r = 1; r < R; ++r) v[it][r] = c_mul(v[it][r], fft_twiddle(tw, n, r * step, inverse));
-      }
-      dft_small<R>(v[it], inverse);
-    }
+// The twiddles of thread j's butterflies in the passes after the first, read once
+// from the table tw (exp(-2 pi i m / N), m < N / 2) and kept in registers.
+template <int N>
+struct FftTw {
+  static constexpr int P = fft_passes(N) - 1;
+  float2 w[P > 0 ? 7 * P : 1];
+  static __device__ __forceinline__ float2 at(const float2 *tw, int m) {
+    float2 r = __ldg(tw + (m & (N / 2 - 1)));
+    if (m >= N / 2) r = make_float2(-r.x, -r.y);
+    return r;
   }
-  __syncthreads();
-#pragma unroll
-  for (int it = 0; it < MAXT; ++it) {
-    const int t = threadIdx.x + it * blockDim.x;
-    if (t < tasks) {
-      const int j = t / cols, c = t - j * cols;
-      const int k = j & (ns - 1);
-      const int d = (j - k) * R + k;
-#pragma unroll
-      for (int r = 0; r < R; ++r) s[(d + r * ns) * cols + c] = v[it][r];
-    }
-  }
-  __syncthreads();
-}
-
-// Transform of ``cols`` interleaved sequences of length n (a power of two,
-// 8 <= n <= 2048) in natural order, in place.  MAXT8 bounds the radix-8
-// butterflies per thread and pass: (n / 8) * cols <= MAXT8 * blockDim.x.
-// Call with all threads of the CTA; ends with a barrier.
-template <int MAXT8>
-__device__ __forceinline__ void smem_fft_stockham(float2 *s, int n, int cols, const float2 *tw, bool inverse) {
-  int ns = 1;
-  for (; ns * 8 <= n; ns *= 8) stockham_pass<8, MAXT8>(s, n, cols, ns, tw, inverse);
-  if (ns * 4 == n)
-    stockham_pass<4, 2 * MAXT8>(s, n, cols, ns, tw, inverse);
-  else if (ns * 2 == n)
-    stockham_pass<2, 4 * MAXT8>(s, n, cols, ns, tw, inverse);
-}
-
-// ---- compile-time variant: length N, COLS interleaved sequences, NT threads,
-// all pass parameters constant (divisions by constants, exactly sized
-// register blocks).  tws: the N/2 forward twiddles, in shared memory.
-template <int R, int N, int COLS, int NT, int NS>
-__device__ __forceinline__ void stockham_pass_ct(float2 *s, const float2 *tws, bool inverse) {
-  constexpr int NB = N / R;
-  constexpr int TASKS = NB * COLS;
-  constexpr int MAXT = (TASKS + NT - 1) / NT;
-  constexpr int STEP = N / (NS * R);
-  float2 v[MAXT][R];
-#pragma unroll
-  for (int it = 0; it < MAXT; ++it) {
-    const int t = threadIdx.x + it * NT;
-    if (TASKS % NT == 0 || t < TASKS) {
-      const int j = t / COLS, c = t - j * COLS;
-#pragma unroll
-      for (int r = 0; r < R; ++r) v[it][r] = s[(j + r * NB) * COLS + c];
-      if (NS > 1) {
+  template <int NS, int I>
+  __device__ __forceinline__ void fill(const float2 *tw, int j) {
+    if constexpr (NS < N) {
+      constexpr int R = NS * 8 <= N ? 8 : N / NS;
+      if constexpr (R == 8) {
         const int k = j & (NS - 1);
 #pragma unroll
-        for (int r = 1; r < R; ++r) {
-          const int m = r * k * STEP;  // < N
-          float2 w = tws[m & (N / 2 - 1)];
-          if (m >= N / 2) w = make_float2(-w.x, -w.y);
-          if (inverse) w.y = -w.y;
-          v[it][r] = c_mul(v[it][r], w);
-        }
+        for (int r = 1; r < 8; ++r) w[7 * I + r - 1] = at(tw, r * k * (N / (NS * 8)));
+      } else {  // NS R = N: butterflies j + q T, exponent r (j + q T)
+#pragma unroll
+        for (int q = 0; q < 8 / R; ++q)
+#pragma unroll
+          for (int r = 1; r < R; ++r) w[7 * I + q * (R - 1) + r - 1] = at(tw, r * (j + q * (N / 8)));
       }
-      dft_small<R>(v[it], inverse);
+      fill<NS * 8, I + 1>(tw, j);
     }
   }
-  __syncthreads();
-#pragma unroll
-  for (int it = 0; it < MAXT; ++it) {
-    const int t = threadIdx.x + it * NT;
-    if (TASKS % NT == 0 || t < TASKS) {
-      const int j = t / COLS, c = t - j * COLS;
-      const int k = j & (NS - 1);
-      const int d = (j - k) * R + k;
-#pragma unroll
-      for (int r = 0; r < R; ++r) s[(d + r * NS) * COLS + c] = v[it][r];
-    }
-  }
-  __syncthreads();
-}
-
-template <int N, int COLS, int NT, int NS>
-struct StockhamCT {
-  static __device__ __forceinline__ void run(float2 *s, const float2 *tws, bool inverse) {
-    constexpr int R = (NS * 8 <= N) ? 8 : N / NS;
-    stockham_pass_ct<R, N, COLS, NT, NS>(s, tws, inverse);
-    if constexpr (NS * R < N) StockhamCT<N, COLS, NT, NS * R>::run(s, tws, inverse);
-  }
+  __device__ __forceinline__ void load(const float2 *tw, int j) { fill<8, 0>(tw, j); }
 };
 
-// Transform of COLS interleaved length-N sequences (natural order, in place)
-// by a CTA of NT threads; ends with a barrier.
-template <int N, int COLS, int NT>
-__device__ __forceinline__ void fft_ct(float2 *s, const float2 *tws, bool inverse) {
-  StockhamCT<N, COLS, NT, 1>::run(s, tws, inverse);
-}
-
-// Radix-2 decimation-in-time transform on bit-reversed input (element m of
-// sequence c at s[bitrev(m) * cols + c]); natural-order output.  Kept for
-// callers that load in bit-reversed order.
-__device__ __forceinline__ void smem_fft(float2 *s, int n, int logn, int cols, const float2 *tw, int inverse) {
-  const int nb = (n / 2) * cols;  // butterflies per stage
-  for (int st = 0; st < logn; ++st) {
-    const int half = 1 << st;
-    const int tstep = n >> (st + 1);
-    for (int t = threadIdx.x; t < nb; t += blockDim.x) {
-      const int c = t % cols;
-      const int b = t / cols;
-      const int grp = b >> st;
-      const int pos = b & (half - 1);
-      const int i = (grp * 2 * half + pos) * cols + c;
-      const int j = i + half * cols;
-      float2 w = __ldg(tw + pos * tstep);
-      if (inverse) w.y = -w.y;
-      const float2 u = s[i], v0 = s[j];
-      const float2 v = make_float2(v0.x * w.x - v0.y * w.y, v0.x * w.y + v0.y * w.x);
-      s[i] = make_float2(u.x + v.x, u.y + v.y);
-      s[j] = make_float2(u.x - v.x, u.y - v.y);
+// The passes after the first.  s: this sequence's exchange buffers (two, fft_smem_elems
+// long, element i at s[fft_pad(i) * CS], the second BS floats2 behind the first); sync():
+// barrier over the threads that share them.
+template <int N, int CS, int BS, bool INV, int NS, int I, class Sync>
+__device__ __forceinline__ void fft_tail(float2 (&v)[8], const FftTw<N> &W, int j, float2 *s, const Sync &sync) {
+  if constexpr (NS < N) {
+    constexpr int T = N / 8, PS = NS / 8;  // PS: sub-transform length of the pass before
+    constexpr int R = NS * 8 <= N ? 8 : N / NS;
+    float2 *b = s + (I & 1) * BS;
+    const int k = j & (PS - 1);
+    const int d = (j - k) * 8 + k;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) b[fft_pad(d + r * PS) * CS] = v[r];
+    sync();
+#pragma unroll
+    for (int m = 0; m < 8; ++m) v[m] = b[fft_pad(j + T * m) * CS];
+    if constexpr (R == 8) {
+#pragma unroll
+      for (int r = 1; r < 8; ++r) v[r] = c_mulw<INV>(v[r], W.w[7 * I + r - 1]);
+      dft8<INV>(v);
+    } else if constexpr (R == 4) {
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+#pragma unroll
+        for (int r = 1; r < 4; ++r) v[q + 2 * r] = c_mulw<INV>(v[q + 2 * r], W.w[7 * I + q * 3 + r - 1]);
+        dft4<INV>(v[q], v[q + 2], v[q + 4], v[q + 6]);
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        v[q + 4] = c_mulw<INV>(v[q + 4], W.w[7 * I + q]);
+        dft2<INV>(v[q], v[q + 4]);
+      }
     }
-    __syncthreads();
+    fft_tail<N, CS, BS, INV, NS * 8, I + 1>(v, W, j, s, sync);
   }
 }
+
+// One transform.  Exchanges alternate between the two buffers, one barrier each: a
+// buffer is written again only after a barrier that followed its last reads.  That
+// also holds from one transform to the next when their number is even; after an odd
+// number (fft_odd_exchanges) the caller synchronises before the next transform.
+template <int N, int CS, int BS, bool INV, class Sync>
+__device__ __forceinline__ void fft_regs(float2 (&v)[8], const FftTw<N> &W, int j, float2 *s, const Sync &sync) {
+  dft8<INV>(v);
+  fft_tail<N, CS, BS, INV, 8, 0>(v, W, j, s, sync);
+}
+constexpr bool fft_odd_exchanges(int n) { return ((fft_passes(n) - 1) & 1) != 0; }
+
+// Barrier over one group of T consecutive threads of the CTA (a warp or less: the
+// warp; more: named barrier 1 + group; a CTA has at most 15 such groups).
+template <int T>
+struct GroupSync {
+  int group;
+  __device__ __forceinline__ void operator()() const {
+    if constexpr (T <= 32)
+      __syncwarp();
+    else
+      asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(T) : "memory");
+  }
+};
+struct CtaSync {
+  __device__ __forceinline__ void operator()() const { __syncthreads(); }
+};
 
 // n x n transforms of ``batch`` contiguous images (x fastest), in place.
 void fft2d(float2 *data, int n, int batch, bool inverse, int device, cudaStream_t s);

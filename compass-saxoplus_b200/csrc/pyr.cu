@@ -12,22 +12,22 @@
 // x sinc, FFT), binned by nrebin and normalised to nphot.
 //
 // Here the npts modulation planes (npts x nfft^2 complex, 50 MB at 512^2 x 24:
-// resident in the 126 MB L2) go through three fused passes:
+// resident in the 126 MB L2) go through three fused passes, each with the
+// transforms in registers (fft.cuh), so a plane crosses memory once per pass
+// and shared memory only between the radix-8 passes:
 //   rows   inverse transform along x of the ntot pupil rows only (the other
-//          rows of the padded field are zero), 8 rows per CTA, field and
-//          modulation tilt formed on the fly;
-//   cols   per 8 columns: inverse transform along y (zero rows skipped on
-//          load), field stop x pyramid mask, forward transform along y, all
-//          in shared memory;
-//   accum  per row: forward transform along x of 8 modulation planes at a
-//          time (interleaved in shared memory) and the weighted |.|^2 summed
-//          over the points in registers, in point order.
-// The transforms are Stockham radix-8 passes with the butterflies in
-// registers (fft.cuh, fft_ct), compiled per nfft so that every index is a
-// constant expression, in natural order, so no permutation pass is needed.
-// The pixel-transfer convolution reuses the row / column pattern, the last
-// pass bins nrebin rows per CTA, and one kernel normalises and adds the
-// Philox photon / readout noise of the SH sensor (same sampler, same streams).
+//          rows of the padded field are zero), field and modulation tilt
+//          formed on the fly, straight into the registers;
+//   cols   per group of columns: inverse transform along y, field stop x
+//          pyramid mask, forward transform along y; a CTA keeps the columns'
+//          mask and the twiddles in registers over its modulation points;
+//   accum  per row y: forward transform along x of every modulation plane, the
+//          weighted |.|^2 summed in registers by groups of threads (points g,
+//          g + G, ...), then over the groups; the complete row goes on to the
+//          pixel transfer function's first transform in the same kernel.
+// The pixel transfer function's column and second row transforms follow, the
+// last one bins its rows, and one kernel normalises and adds the Philox photon /
+// readout noise of the SH sensor (same sampler, same streams).
 
 #include <cuda_runtime.h>
 
@@ -40,8 +40,9 @@
 
 namespace aob {
 
-constexpr int PYR_SEQ = 8;        // sequences (rows or columns) per CTA
-constexpr int PYR_THREADS = 512;
+constexpr int PYR_MAX_REBIN = 8;
+constexpr int PYR_THREADS = 512;      // accum: threads per CTA, at most
+constexpr int PYR_ROW_THREADS = 256;
 
 struct PyrArgs {
   int ntot, off, npts;
@@ -58,7 +59,7 @@ struct PyrArgs {
   float *binimg;     // nb x nb
   float *partial;    // nb row sums
   float *focal_work; // npts x N x N, w_p |field stop x focal field|^2 (null: not computed)
-  int nrebin, nb, rows_per_bin_cta;
+  int nrebin, nb;
 };
 
 // complex multiply
@@ -66,218 +67,246 @@ __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
   return make_float2(a.x * b.x - a.y * b.y, a.y * b.x + a.x * b.y);
 }
 
-// shared memory of every pyramid kernel: PYR_SEQ interleaved sequences of N
-// complex values, then the N/2 twiddles
+// 1. rows of the padded pupil field, inverse transform along x; a group of
+//    N / 8 threads takes one pupil row of one modulation point: work[p][yb][:].
 template <int N>
-__device__ __forceinline__ float2 *pyr_load_twiddles(float2 *sm, const float2 *tw) {
-  float2 *tws = sm + N * PYR_SEQ;
-  for (int i = threadIdx.x; i < N / 2; i += blockDim.x) tws[i] = tw[i];
-  return tws;
-}
-
-// 1. rows of the padded pupil field, inverse transform along x; a CTA takes
-//    PYR_SEQ pupil rows of one modulation point: work[p][yb][:].
-template <int N>
-__global__ void __launch_bounds__(PYR_THREADS) pyr_rows_kernel(PyrArgs A) {
-  extern __shared__ float2 sm[];
-  float2 *tws = pyr_load_twiddles<N>(sm, A.tw);
-  const int groups = (A.ntot + PYR_SEQ - 1) / PYR_SEQ;
-  const int p = blockIdx.x / groups;
-  const int y0 = (blockIdx.x - p * groups) * PYR_SEQ;
+__global__ void __launch_bounds__(PYR_ROW_THREADS) pyr_rows_kernel(PyrArgs A) {
+  constexpr int T = N / 8, SEQ = PYR_ROW_THREADS / T, BS = fft_smem_elems(N);
+  __shared__ float2 s[SEQ * 2 * BS];
+  const int g = threadIdx.x / T, j = threadIdx.x % T;
+  const int q = blockIdx.x * SEQ + g;
+  const bool active = q < A.npts * A.ntot;
+  const int p = active ? q / A.ntot : 0, yb = active ? q - p * A.ntot : 0;
+  FftTw<N> W;
+  W.load(A.tw, j);
   const float cxp = A.cx[p], cyp = A.cy[p];
-  for (int t = threadIdx.x; t < N * PYR_SEQ; t += PYR_THREADS) {
-    const int c = t / N, i = t - c * N;
-    const int yb = y0 + c, x = i - A.off;
-    float2 v = make_float2(0.f, 0.f);
-    if (yb < A.ntot && x >= 0 && x < A.ntot) {
+  const float yy = (float)yb - A.ntot / 2.0f;
+  float2 v[8];
+#pragma unroll
+  for (int m = 0; m < 8; ++m) {
+    const int x = j + T * m - A.off;
+    v[m] = make_float2(0.f, 0.f);
+    if (active && x >= 0 && x < A.ntot) {
       const int id = x + yb * A.ntot;
-      const float xx = (float)x - A.ntot / 2.0f, yy = (float)yb - A.ntot / 2.0f;
+      const float xx = (float)x - A.ntot / 2.0f;
       float sn, cs;
       sincosf(A.phase[id] * A.mic2rad + (cxp * xx + cyp * yy), &sn, &cs);
       const float a = A.pupil[id];
-      v = make_float2(cs * a, sn * a);
+      v[m] = make_float2(cs * a, sn * a);
     }
-    sm[i * PYR_SEQ + c] = v;
   }
-  __syncthreads();
-  fft_ct<N, PYR_SEQ, PYR_THREADS>(sm, tws, true);
-  for (int t = threadIdx.x; t < N * PYR_SEQ; t += PYR_THREADS) {
-    const int c = t / N, i = t - c * N;
-    if (y0 + c < A.ntot) A.work[((size_t)p * N + y0 + c) * N + i] = sm[i * PYR_SEQ + c];
+  fft_regs<N, 1, BS, true>(v, W, j, s + g * 2 * BS, GroupSync<T>{g});
+  if (active) {
+    float2 *row = A.work + ((size_t)p * N + yb) * N;
+#pragma unroll
+    for (int m = 0; m < 8; ++m) row[j + T * m] = v[m];
   }
 }
 
-// 2. per group of PYR_SEQ columns of one modulation plane: inverse transform
-//    along y (rows outside the pupil are zero), x field stop, x pyramid
-//    phase mask (submask_krnl, submaskpyr_krnl), forward transform along y.
-//    In place in work[p].
-template <int N>
-__global__ void __launch_bounds__(PYR_THREADS) pyr_cols_kernel(PyrArgs A) {
+// columns per CTA: 8 (64-byte segments), fewer where 8 would pass 512 threads
+constexpr int pyr_cols(int n) { return n <= 512 ? 8 : 4096 / n; }
+
+// 2. per group of columns of the modulation planes blockIdx.y, blockIdx.y +
+//    gridDim.y, ...: inverse transform along y (rows outside the pupil are
+//    zero), x field stop, x pyramid phase mask (submask_krnl,
+//    submaskpyr_krnl), forward transform along y.  In place in work[p].
+//    Bound: instruction issue (about 300 per thread and transform) with one
+//    512-thread CTA per SM at these registers; the next plane's loads go out
+//    before the current one's transforms.  The whole image and its slopes at nfft
+//    512, 24 points, with a 1600-actuator command matrix: 112 us per pass, 181 us
+//    when every radix-8 pass went through shared memory and every point was
+//    read and written with bank conflicts.
+template <int N, bool FOCAL>
+__global__ void __launch_bounds__(N / 8 * pyr_cols(N)) pyr_cols_kernel(PyrArgs A) {
   extern __shared__ float2 sm[];
-  float2 *tws = pyr_load_twiddles<N>(sm, A.tw);
-  constexpr int groups = N / PYR_SEQ;
-  const int p = blockIdx.x / groups;
-  const int c0 = (blockIdx.x - p * groups) * PYR_SEQ;
-  float2 *base = A.work + (size_t)p * N * N + c0;
-  for (int t = threadIdx.x; t < N * PYR_SEQ; t += PYR_THREADS) {
-    const int m = t / PYR_SEQ, c = t - m * PYR_SEQ;
-    const int yb = m - A.off;
-    sm[t] = (yb >= 0 && yb < A.ntot) ? base[(size_t)yb * N + c] : make_float2(0.f, 0.f);
-  }
-  __syncthreads();
-  fft_ct<N, PYR_SEQ, PYR_THREADS>(sm, tws, true);
-  for (int t = threadIdx.x; t < N * PYR_SEQ; t += PYR_THREADS) {
-    const int m = t / PYR_SEQ, c = t - m * PYR_SEQ;
-    const size_t g = (size_t)(c0 + c) + (size_t)m * N;
-    const float2 a = sm[t];
+  constexpr int T = N / 8, CB = pyr_cols(N), BS = fft_smem_elems(N) * CB;
+  const int c = threadIdx.x % CB, j = threadIdx.x / CB;
+  const int x = blockIdx.x * CB + c;
+  float2 *s = sm + c;
+  FftTw<N> W;
+  W.load(A.tw, j);
+  float2 mask[8];
+#pragma unroll
+  for (int m = 0; m < 8; ++m) {
+    const size_t g = x + (size_t)(j + T * m) * N;
     const float msk = A.submask[g];
-    const float2 f = make_float2(a.x * msk, a.y * msk);
-    // the focal plane image (compute_pyrfocalplane): abs2_krnl with the point's weight
-    if (A.focal_work) A.focal_work[(size_t)p * N * N + g] = A.w[p] * (f.x * f.x + f.y * f.y);
-    sm[t] = cmul(f, A.phalfxy[g]);
+    mask[m] = A.phalfxy[g];
+    if (!FOCAL) mask[m] = make_float2(mask[m].x * msk, mask[m].y * msk);
   }
-  __syncthreads();
-  fft_ct<N, PYR_SEQ, PYR_THREADS>(sm, tws, false);
-  for (int t = threadIdx.x; t < N * PYR_SEQ; t += PYR_THREADS) {
-    const int m = t / PYR_SEQ, c = t - m * PYR_SEQ;
-    base[(size_t)m * N + c] = sm[t];
+  auto load = [&](float2(&v)[8], int p) {
+    const float2 *base = A.work + (size_t)p * N * N + x;
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+      const int yb = j + T * m - A.off;
+      v[m] = (yb >= 0 && yb < A.ntot) ? __ldcg(base + (size_t)yb * N) : make_float2(0.f, 0.f);
+    }
+  };
+  // rows [0, ntot) hold the input and are overwritten by the output: every
+  // thread of the column has its input in registers by the first barrier
+  float2 nxt[8];
+  load(nxt, blockIdx.y);
+  for (int p = blockIdx.y; p < A.npts; p += gridDim.y) {
+    float2 v[8];
+#pragma unroll
+    for (int m = 0; m < 8; ++m) v[m] = nxt[m];
+    if (p + (int)gridDim.y < A.npts) load(nxt, p + gridDim.y);
+    fft_regs<N, CB, BS, true>(v, W, j, s, CtaSync{});
+    if (fft_odd_exchanges(N)) __syncthreads();
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+      if (FOCAL) {
+        // the focal plane image (compute_pyrfocalplane): abs2_krnl with the point's weight
+        const size_t g = x + (size_t)(j + T * m) * N;
+        const float msk = A.submask[g];
+        v[m] = make_float2(v[m].x * msk, v[m].y * msk);
+        A.focal_work[(size_t)p * N * N + g] = A.w[p] * (v[m].x * v[m].x + v[m].y * v[m].y);
+      }
+      v[m] = cmul(v[m], mask[m]);
+    }
+    fft_regs<N, CB, BS, false>(v, W, j, s, CtaSync{});
+    float2 *base = A.work + (size_t)p * N * N + x;
+#pragma unroll
+    for (int m = 0; m < 8; ++m) __stcg(base + (size_t)(j + T * m) * N, v[m]);
+    if (fft_odd_exchanges(N)) __syncthreads();
   }
 }
 
-// 3. per row y: forward transform along x of PYR_SEQ modulation planes at a
-//    time, hrimg[y][x] = sum_p w_p |.|^2 in point order (abs2_krnl with the
-//    modulation weight).
+// 3. per row y: forward transform along x of every modulation plane, hrimg[y][x]
+//    = sum_p w_p |.|^2 (abs2_krnl with the modulation weight) -- group g of the
+//    CTA sums points g, g + G, ..., the groups are added in order -- then the
+//    pixel transfer function's inverse transform along x of that row.
 template <int N>
 __global__ void __launch_bounds__(PYR_THREADS) pyr_accum_kernel(PyrArgs A) {
   extern __shared__ float2 sm[];
-  float2 *tws = pyr_load_twiddles<N>(sm, A.tw);
-  constexpr int ACC = (N + PYR_THREADS - 1) / PYR_THREADS;
+  constexpr int T = N / 8, BS = fft_smem_elems(N);
+  const int g = threadIdx.x / T, j = threadIdx.x % T, G = blockDim.x / T;
   const int y = blockIdx.x;
-  float acc[ACC];
+  const GroupSync<T> sync{g};
+  float2 *s = sm + g * 2 * BS;
+  FftTw<N> W;
+  W.load(A.tw, j);
+  float acc[8];
 #pragma unroll
-  for (int j = 0; j < ACC; ++j) acc[j] = 0.f;
-  for (int p0 = 0; p0 < A.npts; p0 += PYR_SEQ) {
-    const int pb = min(PYR_SEQ, A.npts - p0);
-    for (int t = threadIdx.x; t < N * PYR_SEQ; t += PYR_THREADS) {
-      const int q = t / N, m = t - q * N;
-      sm[m * PYR_SEQ + q] = q < pb ? A.work[((size_t)(p0 + q) * N + y) * N + m] : make_float2(0.f, 0.f);
+  for (int m = 0; m < 8; ++m) acc[m] = 0.f;
+  float2 nxt[8];
+  auto load = [&](int p) {
+#pragma unroll
+    for (int m = 0; m < 8; ++m)
+      nxt[m] = p < A.npts ? __ldcg(A.work + ((size_t)p * N + y) * N + j + T * m) : make_float2(0.f, 0.f);
+  };
+  load(g);
+  // (every group makes the same number of passes: groups of one warp share its barrier)
+  for (int p = g, r = (A.npts + G - 1) / G; r > 0; --r, p += G) {
+    float2 v[8];
+#pragma unroll
+    for (int m = 0; m < 8; ++m) v[m] = nxt[m];
+    const float w = p < A.npts ? A.w[p] : 0.f;
+    if (r > 1) load(p + G);
+    fft_regs<N, 1, BS, false>(v, W, j, s, sync);
+    if (fft_odd_exchanges(N)) sync();
+    if (p < A.npts) {
+#pragma unroll
+      for (int m = 0; m < 8; ++m) acc[m] += w * (v[m].x * v[m].x + v[m].y * v[m].y);
     }
-    __syncthreads();
-    fft_ct<N, PYR_SEQ, PYR_THREADS>(sm, tws, false);
+  }
+  __syncthreads();  // the exchange buffers are free: the groups' sums, then the row
+  float *red = reinterpret_cast<float *>(sm);
 #pragma unroll
-    for (int j = 0; j < ACC; ++j) {
-      const int m = threadIdx.x + j * PYR_THREADS;
-      if (m < N)
-        for (int q = 0; q < pb; ++q) {
-          const float2 v = sm[m * PYR_SEQ + q];
-          acc[j] += A.w[p0 + q] * (v.x * v.x + v.y * v.y);
-        }
+  for (int m = 0; m < 8; ++m) red[g * N + j + T * m] = acc[m];
+  __syncthreads();
+  for (int x = threadIdx.x; x < N; x += blockDim.x) {
+    float t = red[x];
+    for (int q = 1; q < G; ++q) t += red[q * N + x];
+    A.hrimg[(size_t)y * N + x] = t;
+    red[x] = t;
+  }
+  __syncthreads();
+  float2 v[8];
+#pragma unroll
+  for (int m = 0; m < 8; ++m) v[m] = make_float2(red[j + T * m], 0.f);
+  __syncthreads();
+  // the first group takes the row on (with groups of less than a warp, that warp's)
+  if (threadIdx.x < (T < 32 ? 32 : T)) {
+    fft_regs<N, 1, BS, true>(v, W, j, s, sync);
+    if (g == 0) {
+#pragma unroll
+      for (int m = 0; m < 8; ++m) A.conv[(size_t)y * N + j + T * m] = v[m];
     }
-    __syncthreads();
   }
+}
+
+// 4. pixel transfer function, columns: inverse transform along y, x sinc, forward
+//    transform along y.  Fewer columns per CTA than in the modulation planes: one
+//    image has to spread over the whole GPU.
+constexpr int pyr_conv_cols(int n) { return n <= 1024 ? 4 : 2; }
+template <int N>
+__global__ void __launch_bounds__(N / 8 * pyr_conv_cols(N)) pyr_conv_cols_kernel(PyrArgs A) {
+  extern __shared__ float2 sm[];
+  constexpr int T = N / 8, CB = pyr_conv_cols(N), BS = fft_smem_elems(N) * CB;
+  const int c = threadIdx.x % CB, j = threadIdx.x / CB;
+  const int x = blockIdx.x * CB + c;
+  float2 *s = sm + c;
+  float2 v[8];
+  float msk[8];
 #pragma unroll
-  for (int j = 0; j < ACC; ++j) {
-    const int m = threadIdx.x + j * PYR_THREADS;
-    if (m < N) A.hrimg[(size_t)y * N + m] = acc[j];
+  for (int m = 0; m < 8; ++m) {
+    v[m] = A.conv[x + (size_t)(j + T * m) * N];
+    msk[m] = A.sincar[x + (size_t)(j + T * m) * N];
   }
+  FftTw<N> W;
+  W.load(A.tw, j);
+  fft_regs<N, CB, BS, true>(v, W, j, s, CtaSync{});
+  if (fft_odd_exchanges(N)) __syncthreads();
+#pragma unroll
+  for (int m = 0; m < 8; ++m) v[m] = make_float2(v[m].x * msk[m], v[m].y * msk[m]);
+  fft_regs<N, CB, BS, false>(v, W, j, s, CtaSync{});
+#pragma unroll
+  for (int m = 0; m < 8; ++m) A.conv[x + (size_t)(j + T * m) * N] = v[m];
 }
 
-// The single-image tails below (pixel-transfer convolution and binning) take
-// TSEQ sequences per CTA on TSEQ * 64 threads, so one image spreads over
-// N / TSEQ CTAs (256 at N = 512, TSEQ = 2) instead of N / PYR_SEQ; each
-// sequence's transform is the same whatever the CTA shape.
-// 4. pixel transfer function: TSEQ rows of hrimg (real), inverse transform along x.
-template <int N, int TSEQ>
-__global__ void __launch_bounds__(TSEQ * 64) pyr_conv_rows_kernel(PyrArgs A) {
-  constexpr int NT = TSEQ * 64;
+// 5. a few rows per CTA (a multiple of nrebin): forward transform along x, real part,
+//    binning (pyr_bimg_krnl order: x offset outer, y offset inner, then / nrebin^2)
+//    and the row sums of the binned image for the normalisation.
+template <int N>
+__global__ void __launch_bounds__(PYR_THREADS) pyr_bin_kernel(PyrArgs A, int rows) {
   extern __shared__ float2 sm[];
-  float2 *tws = sm + N * TSEQ;
-  for (int i = threadIdx.x; i < N / 2; i += NT) tws[i] = A.tw[i];
-  const int y0 = blockIdx.x * TSEQ;
-  for (int t = threadIdx.x; t < N * TSEQ; t += NT) {
-    const int c = t / N, i = t - c * N;
-    sm[i * TSEQ + c] = make_float2(A.hrimg[(size_t)(y0 + c) * N + i], 0.f);
-  }
-  __syncthreads();
-  fft_ct<N, TSEQ, NT>(sm, tws, true);
-  for (int t = threadIdx.x; t < N * TSEQ; t += NT) {
-    const int c = t / N, i = t - c * N;
-    A.conv[(size_t)(y0 + c) * N + i] = sm[i * TSEQ + c];
-  }
-}
-
-// 5. columns: inverse transform along y, x sinc, forward transform along y.
-template <int N, int TSEQ>
-__global__ void __launch_bounds__(TSEQ * 64) pyr_conv_cols_kernel(PyrArgs A) {
-  constexpr int NT = TSEQ * 64;
-  extern __shared__ float2 sm[];
-  float2 *tws = sm + N * TSEQ;
-  for (int i = threadIdx.x; i < N / 2; i += NT) tws[i] = A.tw[i];
-  const int c0 = blockIdx.x * TSEQ;
-  float2 *base = A.conv + c0;
-  for (int t = threadIdx.x; t < N * TSEQ; t += NT) {
-    const int m = t / TSEQ, c = t - m * TSEQ;
-    sm[t] = base[(size_t)m * N + c];
-  }
-  __syncthreads();
-  fft_ct<N, TSEQ, NT>(sm, tws, true);
-  for (int t = threadIdx.x; t < N * TSEQ; t += NT) {
-    const int m = t / TSEQ, c = t - m * TSEQ;
-    const float msk = A.sincar[(size_t)(c0 + c) + (size_t)m * N];
-    const float2 a = sm[t];
-    sm[t] = make_float2(a.x * msk, a.y * msk);
-  }
-  __syncthreads();
-  fft_ct<N, TSEQ, NT>(sm, tws, false);
-  for (int t = threadIdx.x; t < N * TSEQ; t += NT) {
-    const int m = t / TSEQ, c = t - m * TSEQ;
-    base[(size_t)m * N + c] = sm[t];
-  }
-}
-
-// 6. rows_per_bin_cta (a multiple of nrebin, <= TSEQ) rows per CTA: forward
-//    transform along x, real part, binning (pyr_bimg_krnl order: x offset
-//    outer, y offset inner, then / nrebin^2) and the row sums of the binned
-//    image for the normalisation.
-template <int N, int TSEQ>
-__global__ void __launch_bounds__(TSEQ * 64) pyr_bin_kernel(PyrArgs A) {
-  constexpr int NT = TSEQ * 64;
-  extern __shared__ float2 sm[];
-  float2 *tws = sm + N * TSEQ;
-  for (int i = threadIdx.x; i < N / 2; i += NT) tws[i] = A.tw[i];
-  float *real = reinterpret_cast<float *>(tws + N / 2);  // TSEQ x N
-  const int rows = A.rows_per_bin_cta;
+  constexpr int T = N / 8, BS = fft_smem_elems(N);
+  const int g = threadIdx.x / T, j = threadIdx.x % T, G = blockDim.x / T;
+  const GroupSync<T> sync{g};
+  float2 *s = sm + g * 2 * BS;
+  float *real = reinterpret_cast<float *>(sm + G * 2 * BS);  // rows x N
   const int y0 = blockIdx.x * rows;
-  for (int t = threadIdx.x; t < N * TSEQ; t += NT) {
-    const int c = t / N, i = t - c * N;
-    sm[i * TSEQ + c] = c < rows ? A.conv[(size_t)(y0 + c) * N + i] : make_float2(0.f, 0.f);
-  }
-  __syncthreads();
-  fft_ct<N, TSEQ, NT>(sm, tws, false);
-  for (int t = threadIdx.x; t < N * TSEQ; t += NT) {
-    const int c = t / N, i = t - c * N;
-    real[c * N + i] = sm[i * TSEQ + c].x;
+  FftTw<N> W;
+  W.load(A.tw, j);
+  for (int r = g; r < rows; r += G) {  // rows is a multiple of G
+    float2 v[8];
+#pragma unroll
+    for (int m = 0; m < 8; ++m) v[m] = A.conv[(size_t)(y0 + r) * N + j + T * m];
+    fft_regs<N, 1, BS, false>(v, W, j, s, sync);
+    if (fft_odd_exchanges(N)) sync();
+#pragma unroll
+    for (int m = 0; m < 8; ++m) real[r * N + j + T * m] = v[m].x;
   }
   __syncthreads();
   const int nbr = rows / A.nrebin;
   const float div = (float)(A.nrebin * A.nrebin);
-  for (int t = threadIdx.x; t < nbr * A.nb; t += NT) {
-    const int br = t / A.nb, bx = t - br * A.nb;
-    float o = 0.f;
-    for (int ii = 0; ii < A.nrebin; ++ii)
-      for (int jj = 0; jj < A.nrebin; ++jj) o = o + real[(br * A.nrebin + jj) * N + bx * A.nrebin + ii];
-    A.binimg[(size_t)(blockIdx.x * nbr + br) * A.nb + bx] = o / div;
-  }
-  __syncthreads();
-  if (threadIdx.x < nbr) {
-    const int by = blockIdx.x * nbr + threadIdx.x;
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  for (int br = threadIdx.x >> 5; br < nbr; br += nw) {  // a warp per binned row
     float sum = 0.f;
-    for (int bx = 0; bx < A.nb; ++bx) sum += A.binimg[(size_t)by * A.nb + bx];
-    A.partial[by] = sum;
+    for (int bx = lane; bx < A.nb; bx += 32) {
+      float o = 0.f;
+      for (int ii = 0; ii < A.nrebin; ++ii)
+        for (int jj = 0; jj < A.nrebin; ++jj) o = o + real[(br * A.nrebin + jj) * N + bx * A.nrebin + ii];
+      o = o / div;
+      A.binimg[(size_t)(blockIdx.x * nbr + br) * A.nb + bx] = o;
+      sum += o;
+    }
+    sum = warp_sum(sum);
+    if (lane == 0) A.partial[blockIdx.x * nbr + br] = sum;
   }
 }
 
-// 7. normalisation to nphot (sum of the row sums in row order) and noise.
+// 6. normalisation to nphot (sum of the row sums in row order) and noise.
 __global__ void pyr_norm_noise_kernel(float *binimg, const float *partial, int nb, float nphot, int noise_mode,
                                       float noise, uint32_t frame, uint32_t k0, uint32_t k1) {
   __shared__ float s_fact;
@@ -315,45 +344,66 @@ __global__ void pyr_focal_sum_kernel(float *focal, const float *work, int npts, 
   }
 }
 
-template <int N, int TSEQ>
-static void pyr_launch_tails(const PyrArgs &A, int nbin_ctas, cudaStream_t s) {
-  const size_t sm = sizeof(float2) * (N * TSEQ + N / 2);
-  const size_t bin_sm = sm + sizeof(float) * N * TSEQ;
-  const int lim = (int)std::max<size_t>(bin_sm, 48 * 1024);
-  smem_opt_in(reinterpret_cast<const void *>(pyr_conv_rows_kernel<N, TSEQ>), lim);
-  smem_opt_in(reinterpret_cast<const void *>(pyr_conv_cols_kernel<N, TSEQ>), lim);
-  smem_opt_in(reinterpret_cast<const void *>(pyr_bin_kernel<N, TSEQ>), lim);
-  pyr_conv_rows_kernel<N, TSEQ><<<N / TSEQ, TSEQ * 64, sm, s>>>(A);
-  AOB_LAUNCH_CHECK("pyr_conv_rows_kernel");
-  pyr_conv_cols_kernel<N, TSEQ><<<N / TSEQ, TSEQ * 64, sm, s>>>(A);
-  AOB_LAUNCH_CHECK("pyr_conv_cols_kernel");
-  pyr_bin_kernel<N, TSEQ><<<nbin_ctas, TSEQ * 64, bin_sm, s>>>(A);
-  AOB_LAUNCH_CHECK("pyr_bin_kernel");
+template <class K>
+static void pyr_smem(K kern, size_t bytes) {
+  smem_opt_in(reinterpret_cast<const void *>(kern), (int)std::max<size_t>(bytes, 48 * 1024));
 }
 
 template <int N>
-static void pyr_launch(const PyrArgs &A, int npts, int ntot, int nrebin, cudaStream_t s) {
-  const size_t sm = sizeof(float2) * (N * PYR_SEQ + N / 2);
+static void pyr_launch(const PyrArgs &A, int device, cudaStream_t s) {
+  constexpr int T = N / 8, BS = fft_smem_elems(N);
+  const int nsm = num_sms(device);
   {
-    const int lim = (int)std::max<size_t>(sm, 48 * 1024);
-    smem_opt_in(reinterpret_cast<const void *>(pyr_rows_kernel<N>), lim);
-    smem_opt_in(reinterpret_cast<const void *>(pyr_cols_kernel<N>), lim);
-    smem_opt_in(reinterpret_cast<const void *>(pyr_accum_kernel<N>), lim);
+    constexpr int SEQ = PYR_ROW_THREADS / T;
+    pyr_rows_kernel<N><<<(A.npts * A.ntot + SEQ - 1) / SEQ, PYR_ROW_THREADS, 0, s>>>(A);
+    AOB_LAUNCH_CHECK("pyr_rows_kernel");
   }
-  pyr_rows_kernel<N><<<npts * ((ntot + PYR_SEQ - 1) / PYR_SEQ), PYR_THREADS, sm, s>>>(A);
-  AOB_LAUNCH_CHECK("pyr_rows_kernel");
-  pyr_cols_kernel<N><<<npts * (N / PYR_SEQ), PYR_THREADS, sm, s>>>(A);
-  AOB_LAUNCH_CHECK("pyr_cols_kernel");
-  pyr_accum_kernel<N><<<N, PYR_THREADS, sm, s>>>(A);
-  AOB_LAUNCH_CHECK("pyr_accum_kernel");
-  // tails: as few rows per CTA as the binning allows (rows_per_bin_cta == TSEQ)
-  const int nbin_ctas = N / A.rows_per_bin_cta;
-  if (A.rows_per_bin_cta <= 2)
-    pyr_launch_tails<N, 2>(A, nbin_ctas, s);
-  else if (A.rows_per_bin_cta <= 4)
-    pyr_launch_tails<N, 4>(A, nbin_ctas, s);
-  else
-    pyr_launch_tails<N, 8>(A, nbin_ctas, s);
+  {
+    constexpr int CB = pyr_cols(N), threads = T * CB, groups = N / CB;
+    const size_t sm = sizeof(float2) * 2 * BS * CB;
+    auto kern = A.focal_work ? pyr_cols_kernel<N, true> : pyr_cols_kernel<N, false>;
+    pyr_smem(kern, sm);
+    // the points are split over as many CTAs per column group as give the
+    // shortest longest queue: points per CTA x waves (+ half a point of set-up)
+    const int slots = nsm * std::max(1, 512 / threads);
+    int split = 1;
+    double best = 1e30;
+    for (int ps = 1; ps <= A.npts; ++ps) {
+      const int per = (A.npts + ps - 1) / ps;
+      const double cost = (double)((groups * ps + slots - 1) / slots) * (per + 0.5);
+      if (cost < best) {
+        best = cost;
+        split = ps;
+      }
+    }
+    kern<<<dim3(groups, split), threads, sm, s>>>(A);
+    AOB_LAUNCH_CHECK("pyr_cols_kernel");
+  }
+  {
+    // groups of threads per row: one per point, in whole warps, up to PYR_THREADS
+    const int unit = T < 32 ? 32 / T : 1;
+    const int G = std::min(PYR_THREADS / T, (A.npts + unit - 1) / unit * unit);
+    const size_t sm = std::max(sizeof(float2) * 2 * BS * G, sizeof(float) * N * G);
+    pyr_smem(pyr_accum_kernel<N>, sm);
+    pyr_accum_kernel<N><<<N, G * T, sm, s>>>(A);
+    AOB_LAUNCH_CHECK("pyr_accum_kernel");
+  }
+  {
+    constexpr int CB = pyr_conv_cols(N);
+    const size_t sm = sizeof(float2) * 2 * BS * CB;
+    pyr_smem(pyr_conv_cols_kernel<N>, sm);
+    pyr_conv_cols_kernel<N><<<N / CB, T * CB, sm, s>>>(A);
+    AOB_LAUNCH_CHECK("pyr_conv_cols_kernel");
+  }
+  {
+    // as few rows per CTA as the binning and a whole warp allow (a power of two)
+    const int rows = std::max({A.nrebin, 2, 32 / T});
+    const int G = std::min(rows, PYR_THREADS / T);
+    const size_t sm = sizeof(float2) * 2 * BS * G + sizeof(float) * N * rows;
+    pyr_smem(pyr_bin_kernel<N>, sm);
+    pyr_bin_kernel<N><<<N / rows, G * T, sm, s>>>(A, rows);
+    AOB_LAUNCH_CHECK("pyr_bin_kernel");
+  }
 }
 
 }  // namespace aob
@@ -367,7 +417,7 @@ aob_pyr::aob_pyr(int device_, int nxsub_, int nvalid_, int npix_, int nphase_, i
   AOB_REQUIRE(nvalid > 0 && nrebin > 0 && ntot > 0 && npts > 0, "pyr: sizes must be > 0");
   AOB_REQUIRE(nfft >= 64 && nfft <= 2048 && (nfft & (nfft - 1)) == 0,
               "pyr: nfft must be a power of two in [64, 2048]");
-  AOB_REQUIRE(nrebin <= PYR_SEQ && (nrebin & (nrebin - 1)) == 0,
+  AOB_REQUIRE(nrebin <= PYR_MAX_REBIN && (nrebin & (nrebin - 1)) == 0,
               "pyr: nrebin must be a power of two <= 8 (the binning rows tile nfft)");
   AOB_REQUIRE(ntot <= nfft, "pyr: the phase grid (ntot) must fit in nfft");
   AOB_REQUIRE(nfft % nrebin == 0, "pyr: nfft must be a multiple of nrebin");
@@ -445,8 +495,6 @@ void aob_pyr::comp_image(bool with_noise, cudaStream_t s) {
   A.partial = partial.p;
   A.nrebin = nrebin;
   A.nb = nbin();
-  // binning rows per CTA: nrebin, at least 2 (a power of two dividing nfft)
-  A.rows_per_bin_cta = std::max(nrebin, 2);
   const int64_t n2 = (int64_t)nfft * nfft;
   A.focal_work = nullptr;
   if (compute_focalplane) {
@@ -455,12 +503,12 @@ void aob_pyr::comp_image(bool with_noise, cudaStream_t s) {
     A.focal_work = focal_work.p;
   }
   switch (nfft) {
-    case 64: pyr_launch<64>(A, npts, ntot, nrebin, s); break;
-    case 128: pyr_launch<128>(A, npts, ntot, nrebin, s); break;
-    case 256: pyr_launch<256>(A, npts, ntot, nrebin, s); break;
-    case 512: pyr_launch<512>(A, npts, ntot, nrebin, s); break;
-    case 1024: pyr_launch<1024>(A, npts, ntot, nrebin, s); break;
-    default: pyr_launch<2048>(A, npts, ntot, nrebin, s); break;
+    case 64: pyr_launch<64>(A, device, s); break;
+    case 128: pyr_launch<128>(A, device, s); break;
+    case 256: pyr_launch<256>(A, device, s); break;
+    case 512: pyr_launch<512>(A, device, s); break;
+    case 1024: pyr_launch<1024>(A, device, s); break;
+    default: pyr_launch<2048>(A, device, s); break;
   }
   if (compute_focalplane) {
     pyr_focal_sum_kernel<<<(int)std::min<int64_t>((n2 + 255) / 256, 8 * num_sms(device)), 256, 0, s>>>(
