@@ -276,46 +276,120 @@ __global__ void dm_shape_kernel(float *shape, int npix, const int32_t *rowptr, c
 }
 
 // ------------------------------------------------------------------ target PSF
-__global__ void target_fill_kernel(float2 *amp, const float *phase, const float *mask, float scale, int npup, int nfft) {
-  const int64_t n2 = (int64_t)nfft * nfft;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n2; t += (int64_t)gridDim.x * blockDim.x) {
-    const int i = (int)(t % nfft), j = (int)(t / nfft);
-    float2 v = make_float2(0.f, 0.f);
-    if (i < npup && j < npup) {
-      const int q = i + j * npup;
-      if (mask[q] > 0.f) {
-        float s, c;
-        sincosf(scale * phase[q], &s, &c);
-        v = make_float2(c, s);
-      }
+// The image of a target in two launches.  Rows: the field exp(i scale phase)
+// where the pupil is open, transformed along x straight from registers
+// (fft.cuh); only the npup rows that hold the pupil are formed.  Columns: the
+// rows beyond npup are zeros that are never loaded, and the finished spectrum
+// goes on to the short- and long-exposure images and their maxima in the same
+// pass.  At nfft = 512, npup = 240 the five launches this replaces (fill, two
+// transforms, |.|^2, a memset) took 24.5 us; see target_cols_kernel's rule for
+// the columns per CTA.  Bound: launch and memory latency (6 MB in L2).
+constexpr int TGT_THREADS = 256;
+
+template <int N>
+__global__ void __launch_bounds__(TGT_THREADS)
+    target_rows_kernel(float2 *amp, const float *phase, const float *mask, float scale, int npup, const float2 *tw,
+                       unsigned int *maxes) {
+  constexpr int T = N / 8, SEQ = TGT_THREADS / T, BS = fft_smem_elems(N);
+  __shared__ float2 s[BS > 0 ? SEQ * 2 * BS : 1];
+  if (blockIdx.x == 0 && threadIdx.x < 2) maxes[threadIdx.x] = 0u;
+  const int g = threadIdx.x / T, j = threadIdx.x % T;
+  const int y = blockIdx.x * SEQ + g;
+  float mk[8], ph[8];
+#pragma unroll
+  for (int m = 0; m < 8; ++m) {
+    const int x = j + T * m;
+    const bool in = x < npup && y < npup;
+    mk[m] = in ? mask[x + y * npup] : 0.f;
+    ph[m] = in ? phase[x + y * npup] : 0.f;
+  }
+  FftTw<N> W;
+  W.load(tw, j);
+  float2 v[8];
+#pragma unroll
+  for (int m = 0; m < 8; ++m) {
+    v[m] = make_float2(0.f, 0.f);
+    if (mk[m] > 0.f) {
+      float sn, cs;
+      sincosf(scale * ph[m], &sn, &cs);
+      v[m] = make_float2(cs, sn);
     }
-    amp[t] = v;
+  }
+  fft_regs<N, 1, BS, false>(v, W, j, s + g * 2 * BS, GroupSync<T>{g});
+  if (y < npup) {
+#pragma unroll
+    for (int m = 0; m < 8; ++m) amp[(size_t)y * N + j + T * m] = v[m];
   }
 }
 
-__global__ void target_abs2_kernel(float *se, float *le, const float2 *amp, int64_t n2, float norm, int comp_le,
-                                   unsigned int *max_se, unsigned int *max_le) {
+// columns per CTA: 4 up to nfft = 1024, so that the columns spread over 128 CTAs or
+// more where there are that many; the images' rows are then written in half sectors,
+// which L2 merges
+constexpr int target_cols(int n) { return n <= 1024 ? 4 : 2; }
+
+template <int N>
+__global__ void __launch_bounds__(N / 8 * target_cols(N))
+    target_cols_kernel(float *se, float *le, float2 *amp, int npup, float norm, int comp_le, const float2 *tw,
+                       unsigned int *maxes) {
+  extern __shared__ float2 sm[];
+  constexpr int T = N / 8, CB = target_cols(N), BS = fft_smem_elems(N) * CB;
+  __shared__ unsigned int red[2][32];
+  const int c = threadIdx.x % CB, j = threadIdx.x / CB;
+  const int x = blockIdx.x * CB + c;
+  float2 v[8];
+  float l[8];
+#pragma unroll
+  for (int m = 0; m < 8; ++m) {
+    const int y = j + T * m;
+    v[m] = y < npup ? __ldcg(amp + (size_t)y * N + x) : make_float2(0.f, 0.f);
+    l[m] = le[(size_t)y * N + x];
+  }
+  FftTw<N> W;
+  W.load(tw, j);
+  fft_regs<N, CB, BS, false>(v, W, j, sm + c, CtaSync{});
   unsigned int mse = 0, mle = 0;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n2; t += (int64_t)gridDim.x * blockDim.x) {
-    const float2 a = amp[t];
-    const float v = (a.x * a.x + a.y * a.y) * norm * norm;
-    se[t] = v;
-    float l = le[t];
+#pragma unroll
+  for (int m = 0; m < 8; ++m) {
+    const size_t o = (size_t)(j + T * m) * N + x;
+    amp[o] = v[m];
+    const float p = (v[m].x * v[m].x + v[m].y * v[m].y) * norm * norm;
+    se[o] = p;
     if (comp_le) {
-      l += v;
-      le[t] = l;
+      l[m] += p;
+      le[o] = l[m];
     }
-    mse = max(mse, __float_as_uint(v));
-    mle = max(mle, __float_as_uint(l));
+    mse = max(mse, __float_as_uint(p));
+    mle = max(mle, __float_as_uint(l[m]));
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    mse = max(mse, __shfl_xor_sync(0xffffffffu, mse, o));
-    mle = max(mle, __shfl_xor_sync(0xffffffffu, mle, o));
-  }
+  // one atomic per CTA (unsigned maxima of float bits, as the images are not negative)
+  const unsigned active = __activemask();
+  mse = __reduce_max_sync(active, mse);
+  mle = __reduce_max_sync(active, mle);
   if ((threadIdx.x & 31) == 0) {
-    atomicMax(max_se, mse);
-    atomicMax(max_le, mle);
+    red[0][threadIdx.x >> 5] = mse;
+    red[1][threadIdx.x >> 5] = mle;
   }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < (int)(blockDim.x + 31) / 32; ++w) {
+      mse = max(mse, red[0][w]);
+      mle = max(mle, red[1][w]);
+    }
+    atomicMax(maxes, mse);
+    atomicMax(maxes + 1, mle);
+  }
+}
+
+template <int N>
+static void target_image(float *se, float *le, float2 *amp, const float *phase, const float *mask, float scale,
+                         int npup, float norm, int comp_le, unsigned int *maxes, const float2 *tw, cudaStream_t s) {
+  constexpr int T = N / 8, SEQ = TGT_THREADS / T, CB = target_cols(N);
+  target_rows_kernel<N><<<(npup + SEQ - 1) / SEQ, TGT_THREADS, 0, s>>>(amp, phase, mask, scale, npup, tw, maxes);
+  AOB_LAUNCH_CHECK("target_rows_kernel");
+  constexpr int sm = (int)sizeof(float2) * 2 * fft_smem_elems(N) * CB;
+  smem_opt_in(reinterpret_cast<const void *>(target_cols_kernel<N>), std::max(sm, 48 * 1024));
+  target_cols_kernel<N><<<N / CB, T * CB, sm, s>>>(se, le, amp, npup, norm, comp_le, tw, maxes);
+  AOB_LAUNCH_CHECK("target_cols_kernel");
 }
 
 // Index of the largest value (the first one on ties, as cuBLAS Isamax used by
@@ -618,16 +692,24 @@ aob_target::aob_target(int device_, int npup_, int nfft_, const float *pupil, fl
 
 void aob_target::comp_image(const float *dev_phase, bool comp_le, cudaStream_t s) {
   AOB_CUDA(cudaSetDevice(device));
-  const int64_t n2 = (int64_t)nfft * nfft;
-  const float scale = (float)(2.0 * M_PI / (double)lambda);
-  target_fill_kernel<<<(int)std::min<int64_t>((n2 + 255) / 256, 8192), 256, 0, s>>>(
-      amp.p, dev_phase ? dev_phase : phase.p, mask.p, scale, npup, nfft);
-  AOB_LAUNCH_CHECK("target_fill_kernel");
-  fft2d(amp.p, nfft, 1, false, device, s);
-  AOB_CUDA(cudaMemsetAsync(maxes.p, 0, 2 * sizeof(unsigned int), s));
-  target_abs2_kernel<<<std::min<int64_t>((n2 + 255) / 256, 2 * 148), 256, 0, s>>>(
-      se.p, le.p, amp.p, n2, 1.0f / (float)npts, comp_le ? 1 : 0, maxes.p, maxes.p + 1);
-  AOB_LAUNCH_CHECK("target_abs2_kernel");
+  AOB_REQUIRE(nfft >= 8 && nfft <= 2048, "target: nfft must be a power of two in [8, 2048]");
+  const float scale = (float)(2.0 * M_PI / (double)lambda), norm = 1.0f / (float)npts;
+  const float2 *tw = fft_twiddles(device, nfft);
+  auto go = [&](auto size) {
+    target_image<decltype(size)::value>(se.p, le.p, amp.p, dev_phase ? dev_phase : phase.p, mask.p, scale, npup, norm,
+                                        comp_le ? 1 : 0, maxes.p, tw, s);
+  };
+  switch (nfft) {
+    case 8: go(std::integral_constant<int, 8>{}); break;
+    case 16: go(std::integral_constant<int, 16>{}); break;
+    case 32: go(std::integral_constant<int, 32>{}); break;
+    case 64: go(std::integral_constant<int, 64>{}); break;
+    case 128: go(std::integral_constant<int, 128>{}); break;
+    case 256: go(std::integral_constant<int, 256>{}); break;
+    case 512: go(std::integral_constant<int, 512>{}); break;
+    case 1024: go(std::integral_constant<int, 1024>{}); break;
+    default: go(std::integral_constant<int, 2048>{}); break;
+  }
   if (comp_le) ++le_count;
 }
 
