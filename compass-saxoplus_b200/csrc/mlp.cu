@@ -35,84 +35,107 @@ __global__ void f32_to_bf16_kernel(const float *src, __nv_bfloat16 *dst, int64_t
     dst[i] = __float2bfloat16_rn(src[i]);
 }
 
-// x [batch][nin] float -> xb [batch][pin] bf16 of x * scale, zero padding
-// (the row loops below take four elements per thread and pass, all loads
-// issued before any use, so that enough bytes are in flight per SM)
-__global__ void mlp_input_kernel(const float *x, int nin, int pin, int batch, float scale, __nv_bfloat16 *xb) {
-  const int nt = blockDim.x;
-  for (int b = blockIdx.x; b < batch; b += gridDim.x)
-    for (int i0 = threadIdx.x; i0 < pin; i0 += 4 * nt) {
-      float v[4];
+// x [batch][nin] float -> xb [batch][pin] bf16 of x * scale, zero padding.  A thread
+// takes groups of four elements, two groups' loads in flight (16-byte loads when
+// every row starts on 16 bytes).  Bound: DRAM (x is read once).
+__global__ void __launch_bounds__(256)
+    mlp_input_kernel(const float *x, int nin, int pin, int64_t ngrp, int vec, float scale, __nv_bfloat16 *xb) {
+  const int gpr = pin / 4;  // groups per row
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t g0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g0 < ngrp; g0 += 2 * stride) {
+    float4 v[2];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int i = i0 + k * nt;
-        v[k] = i < nin ? __ldcs(x + (int64_t)b * nin + i) : 0.f;
-      }
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int i = i0 + k * nt;
-        if (i < pin) xb[(int64_t)b * pin + i] = __float2bfloat16_rn(v[k] * scale);
+    for (int k = 0; k < 2; ++k) {
+      const int64_t g = g0 + k * stride;
+      v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (g < ngrp) {
+        const int64_t b = g / gpr;
+        const int i = 4 * (int)(g - b * gpr);
+        const float *row = x + b * nin + i;
+        if (vec) {
+          if (i < nin) v[k] = __ldcs(reinterpret_cast<const float4 *>(row));
+        } else {
+          if (i < nin) v[k].x = __ldcs(row);
+          if (i + 1 < nin) v[k].y = __ldcs(row + 1);
+          if (i + 2 < nin) v[k].z = __ldcs(row + 2);
+          if (i + 3 < nin) v[k].w = __ldcs(row + 3);
+        }
       }
     }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int64_t g = g0 + k * stride;
+      if (g >= ngrp) break;
+      __nv_bfloat162 q[2] = {__floats2bfloat162_rn(v[k].x * scale, v[k].y * scale),
+                             __floats2bfloat162_rn(v[k].z * scale, v[k].w * scale)};
+      *reinterpret_cast<uint2 *>(xb + 4 * g) = *reinterpret_cast<const uint2 *>(q);
+    }
+  }
 }
 
+// (after the mma.sync GEMMs; the tcgen05 GEMM stores the scaled outputs itself)
 __global__ void mlp_output_kernel(const float *y, int nout, int pout, int batch, float scale, float *out) {
   for (int b = blockIdx.x; b < batch; b += gridDim.x)
     for (int o = threadIdx.x; o < nout; o += blockDim.x) out[(int64_t)b * nout + o] = y[(int64_t)b * pout + o] * scale;
 }
 
 // Mean-squared error on the scaled outputs: d = y - t / out_scale; the loss
-// gradient 2 d / (batch * nout) goes to dy (bf16); per-block partial sums of d^2.
-__global__ void mlp_loss_kernel(const float *y, const float *t, int nout, int pout, int batch, float inv_out_scale,
-                                __nv_bfloat16 *dy, float *part) {
-  __shared__ float red[256];
+// gradient 2 d / (batch * nout) goes to dy (bf16).  A block takes 32 adjacent
+// columns and a chunk of rows (8 at a time, four rows' loads in flight per
+// thread); it leaves the column sums of the rounded gradient over its rows (the
+// output bias's gradient) and its sum of d^2, both added up by mlp_finish_kernel.
+constexpr int LOSS_ROWS = 64;  // rows per block
+__global__ void __launch_bounds__(256)
+    mlp_loss_kernel(const float *y, const float *t, int nout, int pout, int batch, float inv_out_scale,
+                    __nv_bfloat16 *dy, float *colpart, float *part) {
+  __shared__ float red[8][33], red2[8];
   const float g = 2.f / ((float)batch * (float)nout);
-  float acc = 0.f;
-  const int nt = blockDim.x;
-  for (int b = blockIdx.x; b < batch; b += gridDim.x)
-    for (int o0 = threadIdx.x; o0 < pout; o0 += 4 * nt) {
+  const int c = blockIdx.x * 32 + threadIdx.x;
+  const int r0 = blockIdx.y * LOSS_ROWS + threadIdx.y, r1 = min(batch, (int)(blockIdx.y + 1) * LOSS_ROWS);
+  float csum = 0.f, acc = 0.f;
+  if (c < pout)
+    for (int b0 = r0; b0 < r1; b0 += 32) {
       float yv[4], tv[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        const int o = o0 + k * nt;
-        yv[k] = o < nout ? y[(int64_t)b * pout + o] : 0.f;
-        tv[k] = o < nout ? __ldcs(t + (int64_t)b * nout + o) : 0.f;
+        const int b = b0 + 8 * k;
+        const bool in = b < r1 && c < nout;
+        yv[k] = in ? __ldcs(y + (int64_t)b * pout + c) : 0.f;
+        tv[k] = in ? __ldcs(t + (int64_t)b * nout + c) : 0.f;
       }
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        const int o = o0 + k * nt;
-        if (o >= pout) continue;
-        float d = 0.f;
-        if (o < nout) d = yv[k] - tv[k] * inv_out_scale;
-        dy[(int64_t)b * pout + o] = __float2bfloat16_rn(g * d);
+        const int b = b0 + 8 * k;
+        if (b >= r1) break;
+        const float d = c < nout ? yv[k] - tv[k] * inv_out_scale : 0.f;
+        const __nv_bfloat16 q = __float2bfloat16_rn(g * d);
+        dy[(int64_t)b * pout + c] = q;
+        csum += __bfloat162float(q);
         acc += d * d;
       }
     }
-  red[threadIdx.x] = acc;
+  red[threadIdx.y][threadIdx.x] = csum;
+  acc = warp_sum(acc);  // (a row of threads is a warp)
+  if (threadIdx.x == 0) red2[threadIdx.y] = acc;
   __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-    __syncthreads();
+  if (threadIdx.y == 0) {
+    float v = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v += red[k][threadIdx.x];
+    if (c < pout) colpart[(int64_t)blockIdx.y * pout + c] = v;
+    if (threadIdx.x == 0) {
+      v = 0.f;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v += red2[k];
+      part[blockIdx.y * gridDim.x + blockIdx.x] = v;
+    }
   }
-  if (threadIdx.x == 0) part[blockIdx.x] = red[0];
 }
 
-__global__ void mlp_loss_final_kernel(const float *part, int nblocks, float denom, float *loss) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    float s = 0.f;
-    for (int i = 0; i < nblocks; ++i) s += part[i];
-    *loss = s / denom;
-  }
-}
-
-// bias gradient: column sums of a [batch][cols] bf16 matrix, batch order
-// Column sums of d [batch][cols] (bias gradients) in two deterministic passes:
-// partial sums over row chunks (block 32 columns x 8 row lanes, coalesced
-// rows), then the chunks added in order.
+// Partial column sums of d [batch][cols] (cols even) over row chunks, for the
+// mma.sync path (the tcgen05 GEMM's epilogue leaves them itself): block 64
+// columns x 8 row lanes, two adjacent columns per thread, four rows in flight.
 constexpr int COLSUM_CHUNKS = 16;
-// Partial column sums over a chunk of rows: a thread takes two adjacent
-// columns (cols even: one 4-byte load per row, 128 bytes per warp) and rows
-// r0 + ty + 8 j, four rows' loads issued before they are added (in row order).
 __global__ void mlp_colsum_part_kernel(const __nv_bfloat16 *d, int batch, int cols, float *part) {
   __shared__ float red[8][2][33];
   const int c = 2 * (blockIdx.x * 32 + threadIdx.x);
@@ -148,26 +171,87 @@ __global__ void mlp_colsum_part_kernel(const __nv_bfloat16 *d, int batch, int co
     }
   }
 }
-__global__ void mlp_colsum_final_kernel(const float *part, int nchunk, int cols, float *out) {
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < cols; c += gridDim.x * blockDim.x) {
+
+// The small sums of a backward pass in one launch: the three bias gradients from
+// their partial column sums, and the loss.  A block adds up 32 columns of one
+// layer (8 lanes of parts, lane order fixed); the last block the loss.  (One thread
+// adding the loss's 1184 partial sums took 18 us.)
+struct FinishArgs {
+  const float *part[3];
+  float *out[3];
+  int nparts[3], cols[3], block0[4];  // layer l: blocks block0[l] .. block0[l + 1]
+  const float *loss_part;
+  int nloss;
+  float denom;
+  float *loss;  // or null
+};
+__global__ void __launch_bounds__(256) mlp_finish_kernel(const __grid_constant__ FinishArgs A) {
+  __shared__ float red[8][33];
+  if ((int)blockIdx.x == A.block0[3]) {
     float s = 0.f;
-    for (int y = 0; y < nchunk; ++y) s += part[(int64_t)y * cols + c];
-    out[c] = s;
+    for (int i = threadIdx.y * 32 + threadIdx.x; i < A.nloss; i += 256) s += A.loss_part[i];
+    s = warp_sum(s);
+    if (threadIdx.x == 0) red[0][threadIdx.y] = s;
+    __syncthreads();
+    if (threadIdx.x == 0 && threadIdx.y == 0) {
+      s = 0.f;
+      for (int w = 0; w < 8; ++w) s += red[0][w];
+      *A.loss = s / A.denom;
+    }
+    return;
+  }
+  int l = 0;
+  while (l < 2 && (int)blockIdx.x >= A.block0[l + 1]) ++l;
+  const int cols = A.cols[l], c = ((int)blockIdx.x - A.block0[l]) * 32 + threadIdx.x;
+  float s = 0.f;
+  if (c < cols)
+    for (int y = threadIdx.y; y < A.nparts[l]; y += 8) s += A.part[l][(int64_t)y * cols + c];
+  red[threadIdx.y][threadIdx.x] = s;
+  __syncthreads();
+  if (threadIdx.y == 0 && c < cols) {
+    s = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) s += red[k][threadIdx.x];
+    A.out[l][c] = s;
   }
 }
 
-// Adam (Kingma & Ba 2015) on FP32 masters; refreshes the BF16 copy.
-__global__ void mlp_adam_kernel(float *w, float *m, float *v, const float *g, __nv_bfloat16 *wb, int64_t n, float lr,
-                                float b1, float b2, float eps, float c1, float c2) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1.f - b1) * gi;
-    const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-    w[i] = wi;
-    if (wb) wb[i] = __float2bfloat16_rn(wi);
+// Adam (Kingma & Ba 2015) on the FP32 masters of every layer, four values per
+// thread; refreshes the BF16 copies.  One launch over the concatenated arrays
+// (all sizes are multiples of 8).  Bound: DRAM, 30 bytes per parameter.
+constexpr int ADAM_SEGS = 7;
+struct AdamArgs {
+  float *w[ADAM_SEGS], *m[ADAM_SEGS], *v[ADAM_SEGS];
+  const float *g[ADAM_SEGS];
+  __nv_bfloat16 *wb[ADAM_SEGS];  // or null
+  int64_t end[ADAM_SEGS];        // groups of four up to and including this array
+  float lr, b1, b2, eps, c1, c2;
+};
+__global__ void __launch_bounds__(256) mlp_adam_kernel(const __grid_constant__ AdamArgs A) {
+  const int64_t total = A.end[ADAM_SEGS - 1];
+  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
+    int l = 0;
+    while (q >= A.end[l]) ++l;
+    const int64_t i = q - (l ? A.end[l - 1] : 0);
+    float4 g4 = __ldcs(reinterpret_cast<const float4 *>(A.g[l]) + i);
+    float4 m4 = reinterpret_cast<const float4 *>(A.m[l])[i];
+    float4 v4 = reinterpret_cast<const float4 *>(A.v[l])[i];
+    float4 w4 = reinterpret_cast<const float4 *>(A.w[l])[i];
+    const float *g = &g4.x;
+    float *m = &m4.x, *v = &v4.x, *w = &w4.x;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      m[k] = A.b1 * m[k] + (1.f - A.b1) * g[k];
+      v[k] = A.b2 * v[k] + (1.f - A.b2) * g[k] * g[k];
+      w[k] = w[k] - A.lr * (m[k] / A.c1) / (sqrtf(v[k] / A.c2) + A.eps);
+    }
+    reinterpret_cast<float4 *>(A.m[l])[i] = m4;
+    reinterpret_cast<float4 *>(A.v[l])[i] = v4;
+    reinterpret_cast<float4 *>(A.w[l])[i] = w4;
+    if (A.wb[l]) {
+      __nv_bfloat162 b[2] = {__floats2bfloat162_rn(w[0], w[1]), __floats2bfloat162_rn(w[2], w[3])};
+      reinterpret_cast<uint2 *>(A.wb[l])[i] = *reinterpret_cast<const uint2 *>(b);
+    }
   }
 }
 
@@ -291,84 +375,118 @@ static void encode_map(CUtensorMap *m, const void *base, uint64_t inner, uint64_
   AOB_REQUIRE(r == CUDA_SUCCESS, "mlp gemm: tensor map encoding failed (" + std::to_string((int)r) + ")");
 }
 
-// kind 0: mma.sync kernel, 1: tcgen05 kernel.  P2 (tcgen05 only, same M, N
-// and layouts): a second product added in the same accumulator.
+// One product of a tcgen05 launch: the operands' layouts, an optional second product
+// added in the same accumulator (same M, N and layouts), the epilogue's extra outputs.
+struct TcOp {
+  GemmArgs P;
+  bool a_km, b_kn;
+  const GemmArgs *P2 = nullptr;
+  float *colpart = nullptr;
+  float *out = nullptr;
+  int out_n = 0;
+  float out_scale = 1.f;
+};
+
+// Launch up to TC_MAX_PROBS products of equal tile width as one list of tiles.
+// Tile width: the one with the smallest cost = rounds of tiles over the pairs of SMs
+// x (stages x time per stage + the tile's set-up), then one epilogue that nothing
+// overlaps.  A stage takes about 0.1 us plus the part that grows with the width
+// (0.3 us at 256); narrow tiles win where a product has few, wide ones where it
+// has many.  An N-contiguous B is loaded in boxes of 64, so its tiles are 128 or
+// 256 wide.
+static void tc_gemm(const TcOp *ops, int n, int device, uint32_t *status, cudaStream_t s) {
+  AOB_REQUIRE(n >= 1 && n <= TC_MAX_PROBS, "mlp gemm: bad product count");
+  const int pairs = std::max(1, num_sms(device) / 2);
+  int nk = 0;
+  bool boxes = false;
+  for (int i = 0; i < n; ++i) {
+    const GemmArgs &P = ops[i].P;
+    AOB_REQUIRE(P.M > 0 && P.N > 0 && P.K > 0, "mlp gemm: empty product");
+    AOB_REQUIRE(P.lda % 8 == 0 && P.ldb % 8 == 0 && ((ops[i].a_km && ops[i].b_kn) || P.K % 8 == 0),
+                "mlp gemm: contiguous dimensions must be multiples of 8");
+    int k = (P.K + TC_BK - 1) / TC_BK;
+    if (ops[i].P2) {
+      AOB_REQUIRE(n == 1, "mlp gemm: a second operand pair goes with a single product");
+      AOB_REQUIRE(ops[i].P2->M == P.M && ops[i].P2->N == P.N && ops[i].P2->K > 0 && ops[i].P2->lda % 8 == 0 &&
+                      ops[i].P2->ldb % 8 == 0,
+                  "mlp gemm: the second product must have the first's shape");
+      k += (ops[i].P2->K + TC_BK - 1) / TC_BK;
+    }
+    AOB_REQUIRE(P.N % 2 == 0 && P.ldc % 2 == 0 && P.ldp % 2 == 0 && !P.accumulate &&
+                    (P.epi == MG_EPI_NONE ? P.Cf && !P.Cb
+                     : P.epi == MG_EPI_GELU ? P.bias && P.pre_out && P.Cb && !P.Cf
+                                            : P.pre_in && P.Cb && !P.Cf && !P.bias && ops[i].colpart),
+                "mlp gemm: outputs that the epilogue does not have");
+    nk = std::max(nk, k);
+    boxes |= ops[i].b_kn;
+  }
+  auto tiles_of = [&](int bn) {
+    int64_t t = 0;
+    for (int i = 0; i < n; ++i)
+      t += (int64_t)((ops[i].P.M + TC_BM - 1) / TC_BM) * ((ops[i].P.N + bn - 1) / bn);
+    return t;
+  };
+  int bn = TC_MAX_BN;
+  double best = 1e30;
+  for (int w = TC_MAX_BN; w >= 64; w -= 32) {
+    if (boxes && w != 256 && w != 128) continue;
+    const double rounds = (double)((tiles_of(w) + pairs - 1) / pairs);
+    const double cost = rounds * (nk * (0.1 + 0.0008 * w) + 0.5) + 1.0 + 0.01 * w;
+    if (cost < best) {
+      best = cost;
+      bn = w;
+    }
+  }
+  TcArgs T{};
+  TcMaps M;
+  T.nprob = n;
+  T.bn = bn;
+  T.status = status;
+  int64_t tiles = 0;
+  auto maps = [bn](const GemmArgs &Q, bool a_km, bool b_kn, CUtensorMap *m) {
+    if (a_km)
+      encode_map(&m[0], Q.A, (uint64_t)Q.M, (uint64_t)Q.K, (uint64_t)Q.lda, 64u);
+    else
+      encode_map(&m[0], Q.A, (uint64_t)Q.K, (uint64_t)Q.M, (uint64_t)Q.lda, (uint32_t)TC_ROWS);
+    if (b_kn)
+      encode_map(&m[1], Q.B, (uint64_t)Q.N, (uint64_t)Q.K, (uint64_t)Q.ldb, 64u);
+    else
+      encode_map(&m[1], Q.B, (uint64_t)Q.K, (uint64_t)Q.N, (uint64_t)Q.ldb, (uint32_t)(bn / 2));
+  };
+  for (int i = 0; i < n; ++i) {
+    const TcOp &O = ops[i];
+    TcProb &Q = T.prob[i];
+    Q.P = O.P;
+    Q.a_mn = O.a_km ? 1 : 0;
+    Q.b_mn = O.b_kn ? 1 : 0;
+    Q.K2 = O.P2 ? O.P2->K : 0;
+    Q.tiles_m = (O.P.M + TC_BM - 1) / TC_BM;
+    Q.tile0 = (int)tiles;
+    Q.colpart = O.colpart;
+    Q.out = O.out;
+    Q.out_n = O.out_n;
+    Q.out_scale = O.out_scale;
+    tiles += (int64_t)Q.tiles_m * ((O.P.N + bn - 1) / bn);
+    maps(O.P, O.a_km, O.b_kn, &M.m[2 * i]);
+    if (O.P2) maps(*O.P2, O.a_km, O.b_kn, &M.m[2]);
+  }
+  AOB_REQUIRE(tiles < (int64_t)1 << 30, "mlp gemm: too many tiles");
+  T.ntiles = (int)tiles;
+  for (int i = n == 1 && ops[0].P2 ? 2 : n; i < TC_MAX_PROBS; ++i) {
+    M.m[2 * i] = M.m[0];
+    M.m[2 * i + 1] = M.m[1];
+  }
+  smem_opt_in(reinterpret_cast<const void *>(tc_gemm_kernel), (int)TC_SMEM_BYTES);
+  tc_gemm_kernel<<<2 * (int)std::min<int64_t>(tiles, pairs), TC_THREADS, TC_SMEM_BYTES, s>>>(M, T);
+  AOB_LAUNCH_CHECK("tc_gemm_kernel");
+}
+
+// The mma.sync kernel.
 template <bool A_KM, bool B_KN>
-static void gemm(const GemmArgs &P, cudaStream_t s, int kind, uint32_t *status, const GemmArgs *P2 = nullptr,
-                 aob::DevBuf<float> *work = nullptr) {
+static void gemm(const GemmArgs &P, cudaStream_t s) {
   AOB_REQUIRE(P.M > 0 && P.N > 0 && P.K > 0, "mlp gemm: empty product");
   AOB_REQUIRE(P.lda % 8 == 0 && P.ldb % 8 == 0 && ((A_KM && B_KN) || P.K % 8 == 0),
               "mlp gemm: contiguous dimensions must be multiples of 8");
-  if (kind == 1) {
-    TcArgs T{P, A_KM ? 1 : 0, B_KN ? 1 : 0, status, P2 ? P2->K : 0, 0, nullptr};
-    // split K when it shortens the product (plain float products only: no
-    // bias, no activation, no accumulate, no bf16 copy).  Cost model, measured
-    // on B200: a CTA alone on an SM takes ~0.5 us per 64-deep stage and two
-    // co-resident CTAs share the SM, so a product takes ~ceil(CTAs / SMs) x
-    // stages per slice x 0.5 us; the slice sum streams (n + 1) M N floats at
-    // ~4 TB/s.  Slices keep at least 8 stages.
-    const int tiles = ((P.N + TC_BN - 1) / TC_BN) * ((P.M + TC_BM - 1) / TC_BM);
-    int dev = 0;
-    AOB_CUDA(cudaGetDevice(&dev));
-    const int nsm = num_sms(dev);
-    int nsplit = 1;
-    if (work && !P2 && P.epi == MG_EPI_NONE && !P.bias && !P.accumulate && !P.Cb && P.Cf && P.ldc % 4 == 0 &&
-        reinterpret_cast<uintptr_t>(P.Cf) % 16 == 0) {
-      const int nkt = (P.K + TC_BK - 1) / TC_BK;
-      auto cost_us = [&](int n) {
-        const int per = (nkt + n - 1) / n, ns = (nkt + per - 1) / per;
-        const double waves = (double)((tiles * ns + nsm - 1) / nsm);
-        const double sum = ns > 1 ? (double)(ns + 1) * P.M * P.N * 4.0 / 4.0e6 : 0.0;
-        return waves * per * 0.5 + sum;
-      };
-      double best = cost_us(1);
-      for (int n = 2; n <= 16 && nkt / n >= 8; ++n)
-        if (cost_us(n) < best) {
-          best = cost_us(n);
-          nsplit = n;
-        }
-    }
-    if (nsplit > 1) {
-      const int per = (((P.K + TC_BK - 1) / TC_BK) + nsplit - 1) / nsplit;
-      nsplit = (((P.K + TC_BK - 1) / TC_BK) + per - 1) / per;
-      T.kchunk = per * TC_BK;
-      const int64_t need = (int64_t)nsplit * P.M * P.ldc;
-      if (work->n < need) work->alloc(need);
-      T.partial = work->p;
-    }
-    auto maps = [](const GemmArgs &Q, CUtensorMap &ma, CUtensorMap &mb) {
-      if (A_KM)
-        encode_map(&ma, Q.A, (uint64_t)Q.M, (uint64_t)Q.K, (uint64_t)Q.lda, 64u);
-      else
-        encode_map(&ma, Q.A, (uint64_t)Q.K, (uint64_t)Q.M, (uint64_t)Q.lda, (uint32_t)TC_BM);
-      if (B_KN)
-        encode_map(&mb, Q.B, (uint64_t)Q.N, (uint64_t)Q.K, (uint64_t)Q.ldb, 64u);
-      else
-        encode_map(&mb, Q.B, (uint64_t)Q.K, (uint64_t)Q.N, (uint64_t)Q.ldb, (uint32_t)TC_BN);
-    };
-    CUtensorMap ma, mb, ma2, mb2;
-    maps(P, ma, mb);
-    if (P2) {
-      AOB_REQUIRE(P2->M == P.M && P2->N == P.N && P2->K > 0 && P2->lda % 8 == 0 && P2->ldb % 8 == 0,
-                  "mlp gemm: the second product must have the first's shape");
-      maps(*P2, ma2, mb2);
-    } else {
-      ma2 = ma;
-      mb2 = mb;
-    }
-    smem_opt_in(reinterpret_cast<const void *>(tc_gemm_kernel), (int)TC_SMEM_BYTES);
-    dim3 grid((P.N + TC_BN - 1) / TC_BN, (P.M + TC_BM - 1) / TC_BM, nsplit);
-    tc_gemm_kernel<<<grid, TC_THREADS, TC_SMEM_BYTES, s>>>(ma, mb, ma2, mb2, T);
-    AOB_LAUNCH_CHECK("tc_gemm_kernel");
-    if (nsplit > 1) {
-      const int nq = (P.N + 3) / 4;
-      dim3 sgrid((nq + 255) / 256, (unsigned)std::min(P.M, 65535));
-      tc_splitk_sum_kernel<<<sgrid, 256, 0, s>>>(T.partial, nsplit, P.M, P.N, P.ldc, P.Cf);
-      AOB_LAUNCH_CHECK("tc_splitk_sum_kernel");
-    }
-    return;
-  }
-  AOB_REQUIRE(P2 == nullptr, "mlp gemm: a second product needs the tcgen05 kernel");
   dim3 grid((P.N + MG_BN - 1) / MG_BN, (P.M + MG_BM - 1) / MG_BM);
   mlp_gemm_kernel<A_KM, B_KN><<<grid, MG_THREADS, 0, s>>>(P);
   AOB_LAUNCH_CHECK("mlp_gemm_kernel");
@@ -474,7 +592,13 @@ void aob_mlp::ensure_batch(int batch) {
   dy.alloc((int64_t)cap * pout);
   dz2.alloc((int64_t)cap * ph2);
   dz1.alloc((int64_t)cap * ph1);
-  loss_part.alloc(8 * num_sms(device));
+  // partial sums: the loss kernel's blocks, and the bias gradients' (a row per 32
+  // samples, the output layer's per LOSS_ROWS; COLSUM_CHUNKS rows on the mma.sync path)
+  const int nchunk = (cap + LOSS_ROWS - 1) / LOSS_ROWS, rparts = std::max((cap + 31) / 32, COLSUM_CHUNKS);
+  loss_part.alloc((int64_t)nchunk * ((pout + 31) / 32));
+  colpart[0].alloc((int64_t)rparts * ph1);
+  colpart[1].alloc((int64_t)rparts * ph2);
+  colpart[2].alloc((int64_t)nchunk * pout);
 }
 
 static __nv_bfloat16 *bf(aob::DevBuf<uint16_t> &b) { return reinterpret_cast<__nv_bfloat16 *>(b.p); }
@@ -482,28 +606,39 @@ static __nv_bfloat16 *bf(aob::DevBuf<uint16_t> &b) { return reinterpret_cast<__n
 void aob_mlp::forward(const float *x, int batch, float *y_out, cudaStream_t s) {
   AOB_CUDA(cudaSetDevice(device));
   ensure_batch(batch);
-  mlp_input_kernel<<<std::min(batch, 8 * num_sms(device)), 256, 0, s>>>(x, nin, pin, batch, in_scale, bf(xb));
-  AOB_LAUNCH_CHECK("mlp_input_kernel");
-  GemmArgs P{};
-  // h1 = GELU(x W1^T + b1)
-  P = GemmArgs{batch, ph1, pin, bf(xb), pin, bf(wb[0]), pin, b[0].p, MG_EPI_GELU, nullptr, z1.p, ph1,
-               nullptr, bf(h1b), ph1, 0};
-  gemm<false, false>(P, s, gemm_kind, tc_status.p);
-  // h2 = GELU(h1 W2^T + b2)
-  P = GemmArgs{batch, ph2, ph1, bf(h1b), ph1, bf(wb[1]), ph1, b[1].p, MG_EPI_GELU, nullptr, z2.p, ph2,
-               nullptr, bf(h2b), ph2, 0};
-  gemm<false, false>(P, s, gemm_kind, tc_status.p);
-  // y = h2 W3^T + b3, then y += x Ws^T (skip path)
-  P = GemmArgs{batch, pout, ph2, bf(h2b), ph2, bf(wb[2]), ph2, b[2].p, MG_EPI_NONE, nullptr, nullptr, 0,
-               y.p, nullptr, pout, 0};
-  GemmArgs P2{batch, pout, pin, bf(xb), pin, bf(wb[3]), pin, nullptr, MG_EPI_NONE, nullptr, nullptr, 0,
+  {
+    const int64_t ngrp = (int64_t)batch * (pin / 4);
+    const int vec = nin % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+    mlp_input_kernel<<<(int)std::max<int64_t>(1, std::min<int64_t>((ngrp + 511) / 512, 8 * num_sms(device))), 256, 0, s>>>(
+        x, nin, pin, ngrp, vec, in_scale, bf(xb));
+    AOB_LAUNCH_CHECK("mlp_input_kernel");
+  }
+  // h1 = GELU(x W1^T + b1), h2 = GELU(h1 W2^T + b2), y = h2 W3^T + b3 + x Ws^T (the skip path)
+  const GemmArgs P1{batch, ph1, pin, bf(xb), pin, bf(wb[0]), pin, b[0].p, MG_EPI_GELU, nullptr, z1.p, ph1,
+                    nullptr, bf(h1b), ph1, 0};
+  const GemmArgs P2{batch, ph2, ph1, bf(h1b), ph1, bf(wb[1]), ph1, b[1].p, MG_EPI_GELU, nullptr, z2.p, ph2,
+                    nullptr, bf(h2b), ph2, 0};
+  const GemmArgs P3{batch, pout, ph2, bf(h2b), ph2, bf(wb[2]), ph2, b[2].p, MG_EPI_NONE, nullptr, nullptr, 0,
+                    y.p, nullptr, pout, 0};
+  GemmArgs PS{batch, pout, pin, bf(xb), pin, bf(wb[3]), pin, nullptr, MG_EPI_NONE, nullptr, nullptr, 0,
               y.p, nullptr, pout, 1};
   if (gemm_kind == 1) {
-    gemm<false, false>(P, s, gemm_kind, tc_status.p, &P2);  // one K loop over [h2 | x]
-  } else {
-    gemm<false, false>(P, s, gemm_kind, tc_status.p);
-    gemm<false, false>(P2, s, gemm_kind, tc_status.p);
+    TcOp O{P1, false, false};
+    tc_gemm(&O, 1, device, tc_status.p, s);
+    O.P = P2;
+    tc_gemm(&O, 1, device, tc_status.p, s);
+    O.P = P3;  // one K loop over [h2 | x]
+    O.P2 = &PS;
+    O.out = y_out;
+    O.out_n = nout;
+    O.out_scale = out_scale;
+    tc_gemm(&O, 1, device, tc_status.p, s);
+    return;
   }
+  gemm<false, false>(P1, s);
+  gemm<false, false>(P2, s);
+  gemm<false, false>(P3, s);
+  gemm<false, false>(PS, s);
   if (y_out) {
     mlp_output_kernel<<<std::min(batch, 8 * num_sms(device)), 256, 0, s>>>(y.p, nout, pout, batch, out_scale,
                                                                               y_out);
@@ -511,67 +646,94 @@ void aob_mlp::forward(const float *x, int batch, float *y_out, cudaStream_t s) {
   }
 }
 
-// bias gradient: column sums of a [batch][cols] bf16 matrix
-void aob_mlp::colsum(const __nv_bfloat16 *d, int batch, int cols, float *out, cudaStream_t s) {
-  if (colsum_part.n < (int64_t)COLSUM_CHUNKS * cols) colsum_part.alloc((int64_t)COLSUM_CHUNKS * cols);
-  AOB_REQUIRE(cols % 2 == 0, "mlp.colsum: padded column count must be even");
-  mlp_colsum_part_kernel<<<dim3((cols / 2 + 31) / 32, COLSUM_CHUNKS), dim3(32, 8), 0, s>>>(d, batch, cols,
-                                                                                        colsum_part.p);
-  mlp_colsum_final_kernel<<<(cols + 255) / 256, 256, 0, s>>>(colsum_part.p, COLSUM_CHUNKS, cols, out);
-  AOB_LAUNCH_CHECK("mlp_colsum_kernel");
-}
-
 // Gradients of the MSE after forward() on the same batch.
 void aob_mlp::backward(const float *target, int batch, float *loss, cudaStream_t s) {
   AOB_REQUIRE(batch <= cap, "mlp.backward: run forward on this batch first");
   AOB_CUDA(cudaSetDevice(device));
-  const int nb = (int)loss_part.n;
-  mlp_loss_kernel<<<nb, 256, 0, s>>>(y.p, target, nout, pout, batch, 1.f / out_scale, bf(dy), loss_part.p);
+  const dim3 lgrid((pout + 31) / 32, (batch + LOSS_ROWS - 1) / LOSS_ROWS);
+  mlp_loss_kernel<<<lgrid, dim3(32, 8), 0, s>>>(y.p, target, nout, pout, batch, 1.f / out_scale, bf(dy), colpart[2].p,
+                                                loss_part.p);
   AOB_LAUNCH_CHECK("mlp_loss_kernel");
-  if (loss) {
-    mlp_loss_final_kernel<<<1, 32, 0, s>>>(loss_part.p, nb, (float)batch * (float)nout, loss);
-    AOB_LAUNCH_CHECK("mlp_loss_final_kernel");
+  // data gradients: dz2 = (dy W3) * GELU'(z2), dz1 = (dz2 W2) * GELU'(z1)
+  const GemmArgs D2{batch, ph2, pout, bf(dy), pout, bf(wb[2]), ph2, nullptr, MG_EPI_DGELU, z2.p, nullptr, ph2,
+                    nullptr, bf(dz2), ph2, 0};
+  const GemmArgs D1{batch, ph1, ph2, bf(dz2), ph2, bf(wb[1]), ph1, nullptr, MG_EPI_DGELU, z1.p, nullptr, ph1,
+                    nullptr, bf(dz1), ph1, 0};
+  // weight gradients: dW3 = dy^T h2, dW2 = dz2^T h1, dW1 = dz1^T x, dWs = dy^T x
+  const GemmArgs G3{pout, ph2, batch, bf(dy), pout, bf(h2b), ph2, nullptr, MG_EPI_NONE, nullptr, nullptr, 0,
+                    gw[2].p, nullptr, ph2, 0};
+  const GemmArgs G2{ph2, ph1, batch, bf(dz2), ph2, bf(h1b), ph1, nullptr, MG_EPI_NONE, nullptr, nullptr, 0,
+                    gw[1].p, nullptr, ph1, 0};
+  const GemmArgs G1{ph1, pin, batch, bf(dz1), ph1, bf(xb), pin, nullptr, MG_EPI_NONE, nullptr, nullptr, 0,
+                    gw[0].p, nullptr, pin, 0};
+  const GemmArgs GS{pout, pin, batch, bf(dy), pout, bf(xb), pin, nullptr, MG_EPI_NONE, nullptr, nullptr, 0,
+                    gw[3].p, nullptr, pin, 0};
+  int rparts;
+  if (gemm_kind == 1) {
+    rparts = (batch + 31) / 32;
+    TcOp O{D2, false, true};
+    O.colpart = colpart[1].p;
+    tc_gemm(&O, 1, device, tc_status.p, s);
+    O.P = D1;
+    O.colpart = colpart[0].p;
+    tc_gemm(&O, 1, device, tc_status.p, s);
+    const TcOp W[4] = {{GS, true, true}, {G1, true, true}, {G3, true, true}, {G2, true, true}};
+    tc_gemm(W, 4, device, tc_status.p, s);
+  } else {
+    rparts = COLSUM_CHUNKS;
+    auto colsum = [&](const __nv_bfloat16 *d, int cols, float *part) {
+      mlp_colsum_part_kernel<<<dim3((cols / 2 + 31) / 32, COLSUM_CHUNKS), dim3(32, 8), 0, s>>>(d, batch, cols, part);
+      AOB_LAUNCH_CHECK("mlp_colsum_part_kernel");
+    };
+    gemm<true, true>(G3, s);
+    gemm<false, true>(D2, s);
+    colsum(bf(dz2), ph2, colpart[1].p);
+    gemm<true, true>(G2, s);
+    gemm<false, true>(D1, s);
+    colsum(bf(dz1), ph1, colpart[0].p);
+    gemm<true, true>(G1, s);
+    gemm<true, true>(GS, s);
   }
-  GemmArgs P{};
-  // layer 3: dW3 = dy^T h2, db3 = sum dy, dz2 = (dy W3) * GELU'(z2)
-  colsum(bf(dy), batch, pout, gb[2].p, s);
-  P = GemmArgs{pout, ph2, batch, bf(dy), pout, bf(h2b), ph2, nullptr, MG_EPI_NONE, nullptr, nullptr, 0,
-               gw[2].p, nullptr, ph2, 0};
-  gemm<true, true>(P, s, gemm_kind, tc_status.p, nullptr, &splitk);
-  P = GemmArgs{batch, ph2, pout, bf(dy), pout, bf(wb[2]), ph2, nullptr, MG_EPI_DGELU, z2.p, nullptr, ph2,
-               nullptr, bf(dz2), ph2, 0};
-  gemm<false, true>(P, s, gemm_kind, tc_status.p);
-  // layer 2
-  colsum(bf(dz2), batch, ph2, gb[1].p, s);
-  P = GemmArgs{ph2, ph1, batch, bf(dz2), ph2, bf(h1b), ph1, nullptr, MG_EPI_NONE, nullptr, nullptr, 0,
-               gw[1].p, nullptr, ph1, 0};
-  gemm<true, true>(P, s, gemm_kind, tc_status.p, nullptr, &splitk);
-  P = GemmArgs{batch, ph1, ph2, bf(dz2), ph2, bf(wb[1]), ph1, nullptr, MG_EPI_DGELU, z1.p, nullptr, ph1,
-               nullptr, bf(dz1), ph1, 0};
-  gemm<false, true>(P, s, gemm_kind, tc_status.p);
-  // layer 1
-  colsum(bf(dz1), batch, ph1, gb[0].p, s);
-  P = GemmArgs{ph1, pin, batch, bf(dz1), ph1, bf(xb), pin, nullptr, MG_EPI_NONE, nullptr, nullptr, 0,
-               gw[0].p, nullptr, pin, 0};
-  gemm<true, true>(P, s, gemm_kind, tc_status.p, nullptr, &splitk);
-  // skip path: dWs = dy^T x
-  P = GemmArgs{pout, pin, batch, bf(dy), pout, bf(xb), pin, nullptr, MG_EPI_NONE, nullptr, nullptr, 0,
-               gw[3].p, nullptr, pin, 0};
-  gemm<true, true>(P, s, gemm_kind, tc_status.p, nullptr, &splitk);
-  AOB_LAUNCH_CHECK("mlp_colsum_kernel");
+  FinishArgs F{};
+  const int cols[3] = {ph1, ph2, pout}, parts[3] = {rparts, rparts, (int)lgrid.y};
+  for (int l = 0; l < 3; ++l) {
+    F.part[l] = colpart[l].p;
+    F.out[l] = gb[l].p;
+    F.nparts[l] = parts[l];
+    F.cols[l] = cols[l];
+    F.block0[l + 1] = F.block0[l] + (cols[l] + 31) / 32;
+  }
+  F.loss_part = loss_part.p;
+  F.nloss = (int)(lgrid.x * lgrid.y);
+  F.denom = (float)batch * (float)nout;
+  F.loss = loss;
+  mlp_finish_kernel<<<F.block0[3] + (loss ? 1 : 0), dim3(32, 8), 0, s>>>(F);
+  AOB_LAUNCH_CHECK("mlp_finish_kernel");
 }
 
 void aob_mlp::adam(float lr, cudaStream_t s) {
   AOB_CUDA(cudaSetDevice(device));
   ++t;
-  const float c1 = 1.f - std::pow(beta1, (float)t), c2 = 1.f - std::pow(beta2, (float)t);
-  for (int l = 0; l < 4; ++l) {
-    mlp_adam_kernel<<<grid_for(w[l].n, device), 256, 0, s>>>(w[l].p, mw[l].p, vw[l].p, gw[l].p, bf(wb[l]), w[l].n,
-                                                             lr, beta1, beta2, eps, c1, c2);
-    if (l < 3)
-      mlp_adam_kernel<<<grid_for(b[l].n, device), 256, 0, s>>>(b[l].p, mb[l].p, vb[l].p, gb[l].p, nullptr, b[l].n,
-                                                               lr, beta1, beta2, eps, c1, c2);
+  AdamArgs A{};
+  A.lr = lr;
+  A.b1 = beta1;
+  A.b2 = beta2;
+  A.eps = eps;
+  A.c1 = 1.f - std::pow(beta1, (float)t);
+  A.c2 = 1.f - std::pow(beta2, (float)t);
+  int64_t end = 0;
+  for (int q = 0; q < ADAM_SEGS; ++q) {
+    const bool weight = q < 4;
+    const int l = weight ? q : q - 4;
+    A.w[q] = weight ? w[l].p : b[l].p;
+    A.m[q] = weight ? mw[l].p : mb[l].p;
+    A.v[q] = weight ? vw[l].p : vb[l].p;
+    A.g[q] = weight ? gw[l].p : gb[l].p;
+    A.wb[q] = weight ? bf(wb[l]) : nullptr;
+    end += (weight ? w[l].n : b[l].n) / 4;
+    A.end[q] = end;
   }
+  mlp_adam_kernel<<<(int)std::max<int64_t>(1, std::min<int64_t>((end + 255) / 256, 8 * num_sms(device))), 256, 0, s>>>(A);
   AOB_LAUNCH_CHECK("mlp_adam_kernel");
 }
 

@@ -1,36 +1,39 @@
 // BF16 GEMM on the fifth-generation tensor cores (tcgen05) for the learned
-// reconstructor's training step.  Same contract as mlp_gemm_kernel (GemmArgs:
+// reconstructor's batched products.  Same contract as mlp_gemm_kernel (GemmArgs:
 // A stored M x K ("MK") or K x M ("KM"), B stored N x K ("NK") or K x N
 // ("KN"), the same epilogue), so the three products of a training step run
 // without transposed copies: K-major operands use the K-major shared-memory
 // descriptor, M- or N-contiguous ones the MN-major descriptor.
 //
-// One CTA per 128 x 128 output tile, 16 warps, two CTAs per SM (97 KB of
-// shared memory and 128 TMEM columns each):
+// Two CTAs (a cluster, cta_group::2) form one 256 x bn tile: each loads its own
+// 128 rows of A and bn / 2 rows of B, 32 KB for a 64-deep stage at bn = 256,
+// two thirds of what two separate 128 x 256 tiles need from L2 and half of what
+// four 128 x 128 tiles do.  Bound: that traffic -- with either tile the SMs draw
+// 9 - 10 TB/s from L2 (0.42 us per stage at 256 x 256, 1.28 PFLOP/s in the main
+// loop; 128 x 128 tiles reached 0.68).  A training step at batch 4096 (2496 -> 1024
+// -> 1024 -> 1377) takes 315 us, 500 us with 128 x 128 tiles, split K and a
+// launch per bias and parameter array.  Pairs are persistent: pair p takes tiles p, p + pairs, ... of a list of up to
+// TC_MAX_PROBS products, so the four weight gradients of a training step
+// (independent, K = the batch) fill the GPU in one launch without split K.
+// Per CTA, 18 warps:
 //  * warp 0, one lane: TMA producer -- 2-D tensor loads with 128-byte swizzle
-//    (K-major tile: one box of 64 (K) x 128 rows; MN-major: two boxes of
-//    64 (M or N) x 64 (K)) into a 3-stage ring, each stage completing on its
-//    "full" mbarrier;
-//  * warp 1: allocates 128 TMEM columns (the 128 x 128 FP32 accumulator); one
-//    lane issues tcgen05.mma.cta_group::1.kind::f16 (M 128, N 128, K 16, four
-//    per 64-wide stage) and tcgen05.commit on the stage's "empty" mbarrier,
-//    which hands the stage back to the producer once those MMAs completed;
-//    after the last stage, a commit on the accumulator barrier;
-//  * all 16 warps: the epilogue -- warps w, w + 4, w + 8, w + 12 read TMEM
-//    lanes 32 (w & 3) .. + 31 (rows of the tile; a warp may only read its own
-//    lane quadrant), one 32-column chunk each, with tcgen05.ld 32x32b, transpose
-//    each 32 x 32 chunk through shared memory and apply bias / GELU / GELU'
-//    with coalesced row accesses.
-// Split K (blockIdx.z slices, each writing its plain FP32 product to a
-// workspace that tc_splitk_sum_kernel adds in slice order: deterministic) keeps
-// the SMs busy for the weight-gradient products, whose outputs have few tiles
-// and whose K is the batch.
+//    (K-major tile: one box of 64 (K) x rows; MN-major: boxes of 64 (M or N) x
+//    64 (K)) into a 5-stage ring; both CTAs' loads complete on the "full"
+//    mbarrier of the leader (cluster rank 0);
+//  * warp 1: allocates the TMEM (two 256-column FP32 accumulators); one lane of
+//    the leader issues tcgen05.mma.cta_group::2.kind::f16 (M 256, N bn, K 16) and
+//    commits each stage to both CTAs' "empty" mbarriers, and each finished
+//    tile to both CTAs' accumulator barriers;
+//  * 16 warps: the epilogue of a tile while the next one is multiplied -- a warp
+//    reads the TMEM lanes of its quadrant (warp & 3) in chunks of 16 columns,
+//    transposes each through shared memory and applies bias / GELU / GELU' with
+//    row accesses of whole sectors.
 // A second operand pair (A2, B2, same layouts, its own K) can follow the first
 // in the same K loop, so y = h2 W3^T + x Ws^T is one GEMM with no read-back of
 // the output.
-// Every mbarrier wait is bounded: on expiry a status bit is set, the kernel
-// still waits (bounded) for its MMAs, frees its TMEM and returns.  No cluster,
-// no multicast.
+// Every mbarrier wait is bounded: on expiry a status bit is set, nothing of the
+// tile is stored, and the CTA goes to its end, where it frees its TMEM.  No load
+// uses multicast.
 #pragma once
 
 #include <cuda.h>
@@ -41,23 +44,40 @@
 
 namespace aob {
 
-constexpr int TC_BM = 128, TC_BN = 128, TC_BK = 64, TC_STAGES = 3, TC_THREADS = 512;
-constexpr int TC_TILE_BYTES = TC_BM * TC_BK * 2;  // one operand tile of a stage (16 KB)
+constexpr int TC_BM = 256, TC_ROWS = 128, TC_MAX_BN = 256, TC_BK = 64, TC_STAGES = 5;
+constexpr int TC_EPI_WARPS = 16, TC_THREADS = 64 + 32 * TC_EPI_WARPS;
+constexpr int TC_TILE_BYTES = TC_ROWS * TC_BK * 2;  // one operand tile of a CTA and stage (16 KB)
 constexpr int TC_STAGE_BYTES = 2 * TC_TILE_BYTES;
-constexpr uint32_t TC_MAX_POLLS = 1u << 24;
+constexpr int TC_MAX_PROBS = 4;
+constexpr uint32_t TC_MAX_POLLS = 1u << 22;
 enum : uint32_t { ERR_TC_TIMEOUT = 8u };
 
-struct TcArgs {
+struct TcProb {
   GemmArgs P;
   int a_mn, b_mn;    // 1: the operand's M (N) index is the contiguous one (KM / KN)
-  uint32_t *status;  // error word (bounded waits that expired)
   int K2;            // > 0: a second product A2 B2^T over K2, summed in the same accumulator
-  int kchunk;        // split K: blockIdx.z covers K [z kchunk, (z + 1) kchunk) (0: all of K)
-  float *partial;    // split K: slice z writes its plain product to partial + z * M * ldc
+  int tiles_m;       // tiles along M; the tile index runs over M first
+  int tile0;         // first tile of this product in the launch's list
+  float *colpart;    // column sums of the bf16 output over each 32 rows (or null): [row / 32][ldc]
+  float *out;        // the output scaled by out_scale, without padding (or null): [M][out_n]
+  int out_n;
+  float out_scale;
+};
+struct TcArgs {
+  int nprob, ntiles, bn;
+  uint32_t *status;  // error word (bounded waits that expired)
+  TcProb prob[TC_MAX_PROBS];
+};
+// operand maps of product i at 2 i (A), 2 i + 1 (B); a second operand pair (single products) at 2, 3
+struct TcMaps {
+  CUtensorMap m[2 * TC_MAX_PROBS];
 };
 
-// shared memory bytes of the kernel (stages + barriers + 1024-byte alignment slack)
-constexpr size_t TC_SMEM_BYTES = (size_t)TC_STAGES * TC_STAGE_BYTES + 1024 + 256;
+constexpr int TC_STAGING_PITCH = 18;  // a warp's 32 x 16 chunk: 8-byte accesses, conflict-free writes
+constexpr int TC_STAGING_FLOATS = 32 * TC_STAGING_PITCH;
+// shared memory bytes of the kernel (stages, epilogue staging, barriers, 1024-byte alignment slack)
+constexpr size_t TC_SMEM_BYTES =
+    (size_t)TC_STAGES * TC_STAGE_BYTES + sizeof(float) * TC_STAGING_FLOATS * TC_EPI_WARPS + 1024 + 256;
 
 // UMMA shared-memory matrix descriptor: start address, leading / stride byte
 // offsets (16-byte units), descriptor version 1, 128-byte swizzle.
@@ -70,17 +90,36 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t saddr, uint32_t lbo
   return d;
 }
 
-// instruction descriptor of kind::f16: BF16 x BF16 -> F32, M = 128, N = 128
-__host__ __device__ constexpr uint32_t umma_idesc_bf16(int a_mn, int b_mn) {
+// instruction descriptor of kind::f16: BF16 x BF16 -> F32, M = 256 (the pair), N = bn
+__host__ __device__ constexpr uint32_t umma_idesc_bf16(int a_mn, int b_mn, int bn) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)a_mn << 15) | ((uint32_t)b_mn << 16) |
-         ((uint32_t)(TC_BN >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
+         ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
 }
 
-__device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int x, int y, uint64_t *bar) {
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// cluster address of this shared-memory address in the CTA of the given rank
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t a, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+// 2-D tensor load into this CTA's shared memory, completing on ``bar`` (a cluster address)
+__device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-          smem_addr(dst)),
-      "l"(map), "r"(x), "r"(y), "r"(smem_addr(bar))
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, "
+      "%3}], [%4];" ::"r"(smem_addr(dst)),
+      "l"(map), "r"(x), "r"(y), "r"(bar)
       : "memory");
 }
 
@@ -89,232 +128,284 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t da, uint64_t
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::"r"(tmem_d),
-      "l"(da), "l"(db), "r"(idesc), "r"(acc), "r"(z), "r"(z), "r"(z), "r"(z));
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}\n" ::"r"(tmem_d),
+      "l"(da), "l"(db), "r"(idesc), "r"(acc), "r"(z));
 }
 
-__device__ __forceinline__ void umma_commit(uint64_t *bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(bar))
-               : "memory");
+// arrives on the barrier at this offset in both CTAs once the MMAs issued so far have completed
+__device__ __forceinline__ void umma_commit_pair(uint64_t *bar) {
+  const uint16_t both = 3;
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+          smem_addr(bar)),
+      "h"(both)
+      : "memory");
 }
 
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
-      "%15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, "
+      "[%16];"
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr));
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// two CTAs per SM: one CTA's epilogue overlaps the other's main loop
-__global__ void __launch_bounds__(TC_THREADS, 2)
-    tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
-                   const __grid_constant__ CUtensorMap mapA2, const __grid_constant__ CUtensorMap mapB2, TcArgs T) {
+// The tile of a launch's list: its product and coordinates.
+struct TcTile {
+  int i, mt, nt, nk1, nk;
+  __device__ TcTile(const TcArgs &T, int t) {
+    i = 0;
+    while (i + 1 < T.nprob && t >= T.prob[i + 1].tile0) ++i;
+    const TcProb &Q = T.prob[i];
+    const int u = t - Q.tile0;
+    nt = u / Q.tiles_m;
+    mt = u - nt * Q.tiles_m;
+    nk1 = (Q.P.K + TC_BK - 1) / TC_BK;
+    nk = nk1 + (Q.K2 > 0 ? (Q.K2 + TC_BK - 1) / TC_BK : 0);
+  }
+};
+
+// The epilogue of one warp: its 32 rows from m0 on, 16-column chunks part, part + 4,
+// ... of the tile's bn columns from n0 on.  Each chunk goes TMEM -> registers
+// (thread = row) -> shared memory -> registers (lane: two columns of rows lane / 8,
+// + 4, ...), so global accesses are whole sectors, two values each.  The product's
+// parameters are copied to registers before the loops: read from the parameter
+// bank through a run-time index they cost more than the arithmetic (70 us per
+// product against 10).
+//   EPI none: Cf (+ bias), the scaled copy out; GELU: bias, pre_out, Cb; GELU': Cb
+//   and its column sums over the warp's rows.
+template <int EPI>
+__device__ __forceinline__ void tc_epilogue(const TcProb &Q, int m0, int n0, int bn, int part, uint32_t taddr,
+                                            float *stage, int lane) {
+  const int M = Q.P.M, N = Q.P.N, ldc = Q.P.ldc, ldp = Q.P.ldp, out_n = Q.out_n;
+  const float *__restrict__ bias = Q.P.bias;
+  const float *__restrict__ pre_in = Q.P.pre_in;
+  float *__restrict__ pre_out = Q.P.pre_out;
+  float *__restrict__ Cf = Q.P.Cf;
+  __nv_bfloat16 *__restrict__ Cb = Q.P.Cb;
+  float *__restrict__ out = Q.out;
+  float *__restrict__ colpart = Q.colpart;
+  const float oscale = Q.out_scale;
+  const int cp = 2 * (lane & 7), rq = lane >> 3;  // column pair, row offset
+  const bool full = m0 + 32 <= M;
+#pragma unroll 1
+  for (int c = part; c < bn / 16 && n0 + c * 16 < N; c += TC_EPI_WARPS / 4) {
+    uint32_t r[16];
+    tmem_ld16(taddr + (uint32_t)(c * 16), r);
+    const int cn = n0 + c * 16 + cp;
+    const bool in = cn < N;  // (N is even: both columns or neither)
+    // the chunk's global inputs go out before the transpose
+    float2 x[8];
+    if (EPI == MG_EPI_DGELU) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int m = m0 + 4 * i + rq;
+        x[i] = (in && (full || m < M)) ? __ldg(reinterpret_cast<const float2 *>(pre_in + (size_t)m * ldp + cn))
+                                       : make_float2(0.f, 0.f);
+      }
+    }
+    float2 bv = make_float2(0.f, 0.f);
+    if (EPI != MG_EPI_DGELU && bias && in) bv = __ldg(reinterpret_cast<const float2 *>(bias + cn));
+#pragma unroll
+    for (int j = 0; j < 16; j += 2)
+      *reinterpret_cast<float2 *>(stage + lane * TC_STAGING_PITCH + j) =
+          make_float2(__uint_as_float(r[j]), __uint_as_float(r[j + 1]));
+    __syncwarp();
+    float2 csum = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int row = 4 * i + rq, m = m0 + row;
+      float2 v = *reinterpret_cast<const float2 *>(stage + row * TC_STAGING_PITCH + cp);
+      if (!in || !(full || m < M)) continue;
+      const size_t o = (size_t)m * ldc + cn;
+      if (EPI == MG_EPI_DGELU) {
+        v.x *= gelu_grad_f(x[i].x);
+        v.y *= gelu_grad_f(x[i].y);
+      } else {
+        v.x += bv.x;
+        v.y += bv.y;
+      }
+      if (EPI == MG_EPI_GELU) {
+        *reinterpret_cast<float2 *>(pre_out + (size_t)m * ldp + cn) = v;
+        v.x = gelu_f(v.x);
+        v.y = gelu_f(v.y);
+      }
+      if (EPI == MG_EPI_NONE) {
+        *reinterpret_cast<float2 *>(Cf + o) = v;
+        if (out) {
+          if (cn < out_n) out[(size_t)m * out_n + cn] = v.x * oscale;
+          if (cn + 1 < out_n) out[(size_t)m * out_n + cn + 1] = v.y * oscale;
+        }
+      } else {
+        const __nv_bfloat162 q = __floats2bfloat162_rn(v.x, v.y);
+        *reinterpret_cast<__nv_bfloat162 *>(Cb + o) = q;
+        if (EPI == MG_EPI_DGELU) {
+          const float2 f = __bfloat1622float2(q);
+          csum.x += f.x;
+          csum.y += f.y;
+        }
+      }
+    }
+    if (EPI == MG_EPI_DGELU) {
+#pragma unroll
+      for (int o = 8; o < 32; o <<= 1) {
+        csum.x += __shfl_xor_sync(0xffffffffu, csum.x, o);
+        csum.y += __shfl_xor_sync(0xffffffffu, csum.y, o);
+      }
+      if (rq == 0 && in && m0 < M) *reinterpret_cast<float2 *>(colpart + (size_t)(m0 / 32) * ldc + cn) = csum;
+    }
+    __syncwarp();
+  }
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
+    tc_gemm_kernel(const __grid_constant__ TcMaps maps, const __grid_constant__ TcArgs T) {
   extern __shared__ __align__(1024) unsigned char tc_raw[];
   unsigned char *sm = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(tc_raw) + 1023) & ~uintptr_t(1023));
-  const GemmArgs &P = T.P;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m0 = blockIdx.y * TC_BM, n0 = blockIdx.x * TC_BN;
-  // K range of this CTA: the whole K (plus K2), or one split-K slice
-  int kt0 = 0, nk1 = (P.K + TC_BK - 1) / TC_BK;
-  if (T.kchunk > 0) {
-    kt0 = (int)blockIdx.z * (T.kchunk / TC_BK);
-    nk1 = min(nk1, kt0 + T.kchunk / TC_BK);
-  }
-  const int nk = nk1 - kt0 + (T.K2 > 0 ? (T.K2 + TC_BK - 1) / TC_BK : 0);
-  uint64_t *full = reinterpret_cast<uint64_t *>(sm + TC_STAGES * TC_STAGE_BYTES);
+  const uint32_t rank = cluster_rank();
+  const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
+  float *staging = reinterpret_cast<float *>(sm + TC_STAGES * TC_STAGE_BYTES);
+  uint64_t *full = reinterpret_cast<uint64_t *>(staging + TC_STAGING_FLOATS * TC_EPI_WARPS);
   uint64_t *empty = full + TC_STAGES;
-  uint64_t *accb = empty + TC_STAGES;
-  uint32_t *tslot = reinterpret_cast<uint32_t *>(accb + 1);
+  uint64_t *accfull = empty + TC_STAGES, *accempty = accfull + 2;
+  uint32_t *tslot = reinterpret_cast<uint32_t *>(accempty + 2);
   if (threadIdx.x == 0) {
     for (int s = 0; s < TC_STAGES; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
-    mbar_init(accb, 1);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&accfull[b], 1);
+      mbar_init(&accempty[b], 2 * TC_EPI_WARPS);
+    }
     fence_mbar_init();
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tslot)),
-                 "r"((uint32_t)TC_BN));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tslot)),
+                 "r"(512u));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::);
     tc_fence_before();
   }
   __syncthreads();
+  cluster_sync();  // both CTAs' barriers exist before either's loads, MMAs or arrivals
   tc_fence_after();
   const uint32_t tmem = *tslot;
+  const int bn = T.bn, bh = bn / 2;
   bool ok = true;
   // the other lanes of the two role warps wait at the warp barrier (not in a
   // polling loop that would share the warp's issue slots with the role lane)
   if (warp == 0) {
     if (lane == 0) {
       // ---- TMA producer ----
-      for (int kt = 0; kt < nk; ++kt) {
-        const int s = kt % TC_STAGES;
-        const uint32_t round = (uint32_t)(kt / TC_STAGES);
-        if (kt >= TC_STAGES && !mbar_wait(&empty[s], (round - 1u) & 1u, TC_MAX_POLLS)) {
-          ok = false;
-          break;
+      int it = 0;
+      for (int t = pair; ok && t < T.ntiles; t += npairs) {
+        const TcTile X(T, t);
+        const bool a_mn = T.prob[X.i].a_mn, b_mn = T.prob[X.i].b_mn;
+        const int m0 = X.mt * TC_BM + (int)rank * TC_ROWS, n0 = X.nt * bn + (int)rank * bh;
+        for (int kt = 0; kt < X.nk; ++kt, ++it) {
+          const int s = it % TC_STAGES;
+          if (it >= TC_STAGES && !mbar_wait(&empty[s], (uint32_t)(it / TC_STAGES - 1) & 1u, TC_MAX_POLLS)) {
+            ok = false;
+            break;
+          }
+          unsigned char *sa = sm + s * TC_STAGE_BYTES, *sb = sa + TC_TILE_BYTES;
+          if (rank == 0) mbar_expect_tx(&full[s], 2u * (uint32_t)(TC_TILE_BYTES + bh * TC_BK * 2));
+          const uint32_t bar = cluster_addr(smem_addr(&full[s]), 0);
+          const bool second = kt >= X.nk1;
+          const CUtensorMap *ma = &maps.m[second ? 2 : 2 * X.i], *mb = ma + 1;
+          const int k0 = (second ? kt - X.nk1 : kt) * TC_BK;
+          if (a_mn) {
+            tma_load_2d(sa, ma, m0, k0, bar);
+            tma_load_2d(sa + TC_TILE_BYTES / 2, ma, m0 + 64, k0, bar);
+          } else {
+            tma_load_2d(sa, ma, k0, m0, bar);
+          }
+          if (b_mn) {
+            for (int h = 0; h < bh; h += 64) tma_load_2d(sb + h * TC_BK * 2, mb, n0 + h, k0, bar);
+          } else {
+            tma_load_2d(sb, mb, k0, n0, bar);
+          }
         }
-        unsigned char *sa = sm + s * TC_STAGE_BYTES, *sb = sa + TC_TILE_BYTES;
-        mbar_expect_tx(&full[s], (uint32_t)TC_STAGE_BYTES);
-        const bool second = kt0 + kt >= nk1;
-        const CUtensorMap *ma = second ? &mapA2 : &mapA, *mb = second ? &mapB2 : &mapB;
-        const int k0 = (second ? kt0 + kt - nk1 : kt0 + kt) * TC_BK;
-        if (T.a_mn) {
-          tma_load_2d(sa, ma, m0, k0, &full[s]);
-          tma_load_2d(sa + TC_TILE_BYTES / 2, ma, m0 + 64, k0, &full[s]);
-        } else {
-          tma_load_2d(sa, ma, k0, m0, &full[s]);
-        }
-        if (T.b_mn) {
-          tma_load_2d(sb, mb, n0, k0, &full[s]);
-          tma_load_2d(sb + TC_TILE_BYTES / 2, mb, n0 + 64, k0, &full[s]);
-        } else {
-          tma_load_2d(sb, mb, k0, n0, &full[s]);
-        }
-    }
+      }
+      // the last stages' hand-backs have arrived before the CTA may end
+      for (int k = max(0, it - TC_STAGES); ok && k < it; ++k)
+        ok = mbar_wait(&empty[k % TC_STAGES], (uint32_t)(k / TC_STAGES) & 1u, TC_MAX_POLLS);
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (lane == 0 && rank == 0) {
       // ---- MMA issuer ----
-      const uint32_t idesc = umma_idesc_bf16(T.a_mn, T.b_mn);
-      int issued = 0;
-      for (int kt = 0; kt < nk; ++kt) {
-        const int s = kt % TC_STAGES;
-        if (!mbar_wait(&full[s], (uint32_t)(kt / TC_STAGES) & 1u, TC_MAX_POLLS)) {
+      int it = 0, n = 0;
+      for (int t = pair; ok && t < T.ntiles; t += npairs, ++n) {
+        const TcTile X(T, t);
+        const int a_mn = T.prob[X.i].a_mn, b_mn = T.prob[X.i].b_mn;
+        const uint32_t idesc = umma_idesc_bf16(a_mn, b_mn, bn);
+        // K-major: 16 elements = 32 bytes along the swizzled row; MN-major: 16 rows of 128
+        // bytes (descriptor addresses count 16 bytes)
+        const uint64_t da0 = umma_desc_sw128(smem_addr(sm), a_mn ? TC_TILE_BYTES / 2 : 16, 1024);
+        const uint64_t db0 = umma_desc_sw128(smem_addr(sm) + TC_TILE_BYTES, b_mn ? TC_TILE_BYTES / 2 : 16, 1024);
+        const uint32_t ka = a_mn ? 128 : 2, kb = b_mn ? 128 : 2;
+        const uint32_t acc = tmem + (uint32_t)(n & 1) * TC_MAX_BN;
+        if (n >= 2 && !mbar_wait(&accempty[n & 1], (uint32_t)(n / 2 - 1) & 1u, TC_MAX_POLLS)) {
           ok = false;
           break;
         }
         tc_fence_after();
-        const uint32_t sa = smem_addr(sm + s * TC_STAGE_BYTES), sb = sa + TC_TILE_BYTES;
-  #pragma unroll
-        for (int k = 0; k < TC_BK / 16; ++k) {
-          // K-major: 16 elements = 32 bytes along the swizzled row; MN-major: 16 rows of 128 bytes
-          const uint64_t da = T.a_mn ? umma_desc_sw128(sa + k * 2048, TC_TILE_BYTES / 2, 1024)
-                                     : umma_desc_sw128(sa + k * 32, 16, 1024);
-          const uint64_t db = T.b_mn ? umma_desc_sw128(sb + k * 2048, TC_TILE_BYTES / 2, 1024)
-                                     : umma_desc_sw128(sb + k * 32, 16, 1024);
-          umma_bf16(tmem, da, db, idesc, (kt > 0 || k > 0) ? 1u : 0u);
-        }
-        umma_commit(&empty[s]);
-        ++issued;
-    }
-    umma_commit(accb);  // arrives once every MMA issued above has completed
-    (void)issued;
-    }
-    __syncwarp();
-  }
-  // ---- epilogue: warp w owns TMEM lanes (tile rows) 32w .. 32w + 31.  Each
-  //      32-column chunk goes TMEM -> registers (thread = row) -> shared memory
-  //      (the idle stage buffers; padded rows) -> registers (lane = column), so
-  //      that every global load and store of the epilogue is a coalesced row ----
-  ok &= mbar_wait(accb, 0, TC_MAX_POLLS);
-  __syncwarp();
-  tc_fence_after();
-  // warps w, w + 4, w + 8 and w + 12 share TMEM lane quadrant w & 3 (a warp
-  // may only read its own quadrant) and take one 32-column chunk each
-  const int quad = warp & 3, part = warp >> 2;
-  float *stage = reinterpret_cast<float *>(sm) + warp * 32 * 33;
-  const int n_lane = lane;
-#pragma unroll 1
-  for (int c = part * (TC_BN / 128); c < (part + 1) * (TC_BN / 128); ++c) {
-    uint32_t r[32];
-    tmem_ld32(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(c * 32), r);
+        for (int kt = 0; kt < X.nk; ++kt, ++it) {
+          const int s = it % TC_STAGES;
+          if (!mbar_wait(&full[s], (uint32_t)(it / TC_STAGES) & 1u, TC_MAX_POLLS)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint64_t off = (uint64_t)(s * (TC_STAGE_BYTES / 16));
 #pragma unroll
-    for (int j = 0; j < 32; ++j) stage[lane * 33 + j] = __uint_as_float(r[j]);
-    __syncwarp();
-    const int n = n0 + c * 32 + n_lane;
-    const float bn = (P.bias && n < P.N) ? P.bias[n] : 0.f;
-    if (P.epi == MG_EPI_DGELU && T.kchunk == 0 && !P.accumulate && !P.bias) {
-      // GELU' epilogue (the data gradients): rows in blocks of 8 whose
-      // pre-activations are all requested before any is used, one memory
-      // latency per block instead of one per row
-#pragma unroll 1
-      for (int i0 = 0; i0 < 32; i0 += 8) {
-        float pin[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int m = m0 + quad * 32 + i0 + j;
-          pin[j] = (ok && m < P.M && n < P.N) ? __ldg(P.pre_in + (size_t)m * P.ldp + n) : 0.f;
+          for (int k = 0; k < TC_BK / 16; ++k)
+            umma_bf16(acc, da0 + off + k * ka, db0 + off + k * kb, idesc, (kt > 0 || k > 0) ? 1u : 0u);
+          umma_commit_pair(&empty[s]);
         }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int m = m0 + quad * 32 + i0 + j;
-          if (!ok || m >= P.M || n >= P.N) continue;
-          const float v = stage[(i0 + j) * 33 + n_lane] * gelu_grad_f(pin[j]);
-          const size_t o = (size_t)m * P.ldc + n;
-          if (P.Cf) P.Cf[o] = v;
-          if (P.Cb) P.Cb[o] = __float2bfloat16_rn(v);
-        }
-      }
-    } else {
-#pragma unroll 4
-      for (int i = 0; i < 32; ++i) {
-        const int m = m0 + quad * 32 + i;
-        if (!ok || m >= P.M || n >= P.N) continue;
-        float v = stage[i * 33 + n_lane];
-        const size_t o = (size_t)m * P.ldc + n;
-        if (T.kchunk > 0) {  // split K: the plain product of this slice (summed later in slice order)
-          T.partial[(size_t)blockIdx.z * P.M * P.ldc + o] = v;
-          continue;
-        }
-        if (P.accumulate) v += P.Cf[o];
-        if (P.bias) v += bn;
-        if (P.epi == MG_EPI_GELU) {
-          if (P.pre_out) P.pre_out[(size_t)m * P.ldp + n] = v;
-          v = gelu_f(v);
-        } else if (P.epi == MG_EPI_DGELU) {
-          v *= gelu_grad_f(P.pre_in[(size_t)m * P.ldp + n]);
-        }
-        if (P.Cf) P.Cf[o] = v;
-        if (P.Cb) P.Cb[o] = __float2bfloat16_rn(v);
+        if (ok) umma_commit_pair(&accfull[n & 1]);
       }
     }
     __syncwarp();
+  } else {
+    // ---- epilogue ----
+    const int quad = warp & 3, part = (warp - 2) >> 2;
+    float *stage = staging + (warp - 2) * TC_STAGING_FLOATS;
+    int n = 0;
+    for (int t = pair; t < T.ntiles; t += npairs, ++n) {
+      const TcTile X(T, t);
+      const TcProb &Q = T.prob[X.i];
+      const int m0 = X.mt * TC_BM + (int)rank * TC_ROWS + quad * 32, n0 = X.nt * bn;
+      ok = mbar_wait(&accfull[n & 1], (uint32_t)(n / 2) & 1u, TC_MAX_POLLS);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(n & 1) * TC_MAX_BN;
+      const int epi = Q.P.epi;
+      if (epi == MG_EPI_GELU)
+        tc_epilogue<MG_EPI_GELU>(Q, m0, n0, bn, part, taddr, stage, lane);
+      else if (epi == MG_EPI_DGELU)
+        tc_epilogue<MG_EPI_DGELU>(Q, m0, n0, bn, part, taddr, stage, lane);
+      else
+        tc_epilogue<MG_EPI_NONE>(Q, m0, n0, bn, part, taddr, stage, lane);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(cluster_addr(smem_addr(&accempty[n & 1]), 0));
+    }
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)TC_BN));
+  cluster_sync();  // the pair's MMAs, loads and arrivals are done (or its bounded waits have expired)
+  if (warp == 1)
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
   if (!ok && lane == 0 && T.status) atomicOr(T.status, (uint32_t)ERR_TC_TIMEOUT);
-}
-
-// out[m][n] = sum over slices z (in order) of part[z][m][n], n < N (rows of
-// stride ld): the split-K reduction.  Rows over blockIdx.y, 16-byte column
-// groups over x (ld a multiple of 4, 16-byte aligned buffers: checked on the
-// host); the slices are read streaming, the sum keeps the slice order.
-__global__ void tc_splitk_sum_kernel(const float *part, int nslice, int M, int N, int ld, float *out) {
-  const int64_t total = (int64_t)M * ld;
-  const int nq = (N + 3) >> 2;
-  for (int m = blockIdx.y; m < M; m += gridDim.y) {
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x) {
-      const int64_t o = (int64_t)m * ld + 4 * q;
-      float4 v = __ldcs(reinterpret_cast<const float4 *>(part + o));
-      for (int z = 1; z < nslice; ++z) {
-        const float4 w = __ldcs(reinterpret_cast<const float4 *>(part + (int64_t)z * total + o));
-        v.x += w.x;
-        v.y += w.y;
-        v.z += w.z;
-        v.w += w.w;
-      }
-      const int n = 4 * q;
-      if (n + 3 < N) {
-        *reinterpret_cast<float4 *>(out + o) = v;
-      } else {
-        out[o] = v.x;
-        if (n + 1 < N) out[o + 1] = v.y;
-        if (n + 2 < N) out[o + 2] = v.z;
-      }
-    }
-  }
 }
 
 }  // namespace aob
