@@ -32,8 +32,8 @@ import time
 
 from ._lib import AobError, call
 
-DEFAULT_BATCH_SPACE = dict(subaps=(16, 32, 64), team=(64, 256), mvm_kb=(48, 96), lag=(16,), ctas_per_sm=(2, 3),
-                           order=(0,))
+DEFAULT_BATCH_SPACE = dict(subaps=(8, 16, 32), team=(64, 256), mvm_kb=(24, 48, 96), lag=(64,),
+                           ctas_per_sm=(2, 3, 4), order=(0,))
 _BATCH_KEYS = ("subaps", "team", "mvm_kb", "lag", "ctas_per_sm", "order")
 DEFAULT_LOOP_SPACE = dict(fused_batch=(0, 1, 2, 4, 8))
 

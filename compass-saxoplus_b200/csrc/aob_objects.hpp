@@ -292,12 +292,16 @@ struct aob_loop {
 struct aob_batch {
   int device = 0;
   std::vector<aob_loop *> loops;
-  // tuning: sub-apertures per sensor item (0 = 32), threads per sensor team
-  // (0 = 32), command-matrix KB per MVM item (0 = 48), MVM items queued `lag`
-  // instances after their sensor items, CTAs per SM (0 = 2), instance order
+  // tuning: sub-apertures per sensor item, threads per sensor team, command-matrix
+  // KB per MVM item, CTAs per SM (0: chosen by pick_tuning), MVM items queued
+  // `lag` instances after their sensor items (-1: see build), instance order
   // (0 = largest first, 1 = as added)
-  int subaps = 0, team = 0, mvm_kb = 0, lag = 2, ctas_per_sm = 0, order = 0;
-  int team_threads() const { return team > 0 ? team : 32; }
+  int subaps = 0, team = 0, mvm_kb = 0, lag = -1, ctas_per_sm = 0, order = 0;
+  struct Tuning {
+    int subaps, team, mvm_kb, ctas_per_sm;
+  } tune{32, 32, 48, 2};  // the values in use
+  Tuning pick_tuning() const;
+  size_t item_cap(int ctas) const;
   bool use_graph = true;
   bool built = false;
   uint64_t built_key = 0;

@@ -246,7 +246,7 @@ __device__ __forceinline__ void mvm_item(const BatchInst &I, int ii, int r0, int
 }
 
 // MINB: CTAs per SM the register budget is sized for (2: up to 128
-// registers per thread, 4: up to 64)
+// registers per thread, 3: up to 80, 4: up to 64)
 template <int MINB>
 __global__ void __launch_bounds__(BATCH_THREADS, MINB) batch_step_kernel(BatchArgs A) {
   extern __shared__ __align__(128) unsigned char sm[];
@@ -331,6 +331,11 @@ __global__ void __launch_bounds__(BATCH_THREADS, MINB) batch_step_kernel(BatchAr
 
 using namespace aob;
 
+// the kernel whose register budget fits this many CTAs on an SM
+static void (*batch_kernel(int ctas_per_sm))(BatchArgs) {
+  return ctas_per_sm <= 2 ? batch_step_kernel<2> : (ctas_per_sm == 3 ? batch_step_kernel<3> : batch_step_kernel<4>);
+}
+
 aob_batch::aob_batch(int device_) : device(device_) {}
 
 aob_batch::~aob_batch() { drop_graphs(); }
@@ -384,6 +389,55 @@ uint64_t aob_batch::key(bool noise) const {
   return h;
 }
 
+// Shared memory one item may use with this many CTAs on an SM: the SM's 228 KB
+// shared out, less the per-block reservation, static shared memory and a fixed
+// header for BATCH_MAX_ROWS rows of barriers and epilogue inputs.
+size_t aob_batch::item_cap(int ctas) const {
+  const size_t cap = std::min<size_t>((size_t)226 * 1024, ((size_t)228 / ctas - 2) * 1024);
+  return cap - batch_bars_bytes(BATCH_MAX_ROWS) - batch_pre_bytes(BATCH_MAX_ROWS);
+}
+
+// Bytes of a sensor item of ``s`` sub-apertures shared by teams of ``tm`` threads, and
+// of an MVM item of ``r`` rows.
+static size_t sensor_item_bytes(const aob_sh *w, int s, int tm) {
+  const int npix2 = w->npix * w->npix, teams = BATCH_THREADS / tm;
+  const ShSmem L(w->nfft, w->nu, w->nv, w->nphase, w->nrebin * w->nrebin * npix2, npix2, (s + teams - 1) / teams);
+  return L.team_bytes(teams);
+}
+static size_t mvm_item_bytes(const aob_ls *c, int r) {
+  const int esize = c->prec == AOB_PREC_F32 ? 4 : (c->prec == AOB_PREC_BF16 ? 2 : 1), V = 16 / esize;
+  const int ld = (c->nslope + V - 1) / V * V;
+  return (size_t)r * ld * esize + sizeof(float) * swizzled_slope_floats(ld, V) + sizeof(float) * BATCH_SLOTS * r;
+}
+
+// Tile shapes for the values that were left open, by the batch's sub-apertures per
+// SM.  Measured on B200 over 9 batches (2 to 64 loops, 8 to 40 sub-apertures across,
+// every precision; all shapes with 8 .. 64 sub-apertures, teams of 32 .. 256, 24 .. 96 KB
+// and 2 .. 4 CTAs per SM): the shapes below are within 8 % of the best of each, 17 %
+// at one.  Many sub-apertures: large items, three CTAs (170 us for 32 loops of 24 .. 40
+// sub-apertures across, 371 us with the former fixed shape and a lag of two
+// instances, whose rows waited for sensor items still running).  Few: small items, so
+// that every CTA has one (67 -> 31 us for 5 loops of 10 .. 20).  Two CTAs and the
+// former shape where an item would not fit otherwise.
+aob_batch::Tuning aob_batch::pick_tuning() const {
+  int64_t n = 0;
+  for (const aob_loop *l : loops) n += l->wfs->nvalid;
+  const int nsm = num_sms(device);
+  Tuning t = n >= 100 * nsm ? Tuning{32, 256, 96, 3}
+             : n >= 30 * nsm ? Tuning{8, 64, 24, 3}
+             : n >= 16 * nsm ? Tuning{8, 256, 24, 4}
+                             : Tuning{8, 64, 24, 2};
+  auto given = [this](Tuning q) {
+    return Tuning{subaps > 0 ? subaps : q.subaps, team > 0 ? team : q.team, mvm_kb > 0 ? mvm_kb : q.mvm_kb,
+                  ctas_per_sm > 0 ? ctas_per_sm : q.ctas_per_sm};
+  };
+  t = given(t);
+  const size_t cap = item_cap(t.ctas_per_sm);
+  for (const aob_loop *l : loops)
+    if (sensor_item_bytes(l->wfs, 1, t.team) > cap || mvm_item_bytes(l->ls, 1) > cap) return given(Tuning{32, 32, 48, 2});
+  return t;
+}
+
 // Snapshot every instance's parameters, cut the work into items and upload.
 void aob_batch::build(bool noise) {
   AOB_REQUIRE(!loops.empty(), "batch: no instances added");
@@ -414,13 +468,11 @@ void aob_batch::build(bool noise) {
   frame_seen.assign(n, 0);
   h_frames.assign(n, 0);
 
-  // dynamic shared memory per CTA (static shared memory and the per-block
-  // reservation come on top), minus a fixed header for BATCH_MAX_ROWS rows of
-  // barriers and epilogue inputs, is what one item may use
-  const int cps = ctas_per_sm > 0 ? ctas_per_sm : 2;
-  const size_t smem_cap = std::min<size_t>((size_t)226 * 1024, ((size_t)228 / cps - 2) * 1024);
-  const size_t item_cap = smem_cap - batch_bars_bytes(BATCH_MAX_ROWS) - batch_pre_bytes(BATCH_MAX_ROWS);
-  const size_t kb = mvm_kb > 0 ? (size_t)mvm_kb * 1024 : (size_t)48 * 1024;
+  tune = pick_tuning();
+  const int cps = tune.ctas_per_sm, tm = tune.team;
+  const size_t cap = item_cap(cps);
+  const size_t smem_cap = cap + batch_bars_bytes(BATCH_MAX_ROWS) + batch_pre_bytes(BATCH_MAX_ROWS);
+  const size_t kb = (size_t)tune.mvm_kb * 1024;
   std::vector<int> S(n), RPI(n);
   int rmax = 1;
   alg_bytes = 0;
@@ -463,28 +515,20 @@ void aob_batch::build(bool noise) {
     hf[i] = (uint32_t)w->frame;
     frame_seen[i] = w->frame;
     // sensor items: `subaps` sub-apertures each, split over the CTA's teams
-    const int npix2 = w->npix * w->npix;
-    const int tm = team_threads();
-    int s = std::max(1, std::min(subaps > 0 ? subaps : 32, w->nvalid));
-    auto sh_bytes = [&](int b) {
-      const int smax = (b + BATCH_THREADS / tm - 1) / (BATCH_THREADS / tm);
-      const ShSmem L(w->nfft, w->nu, w->nv, w->nphase, w->nrebin * w->nrebin * npix2, npix2, smax);
-      return L.team_bytes(BATCH_THREADS / tm);
-    };
-    while (s > 1 && sh_bytes(s) > item_cap) --s;
-    AOB_REQUIRE(sh_bytes(s) <= item_cap, "batch: instance " + std::to_string(i) + ": a sensor item does not fit");
+    int s = std::max(1, std::min(tune.subaps, w->nvalid));
+    while (s > 1 && sensor_item_bytes(w, s, tm) > cap) --s;
+    AOB_REQUIRE(sensor_item_bytes(w, s, tm) <= cap,
+                "batch: instance " + std::to_string(i) + ": a sensor item does not fit");
     S[i] = s;
     I.smax = (s + BATCH_THREADS / tm - 1) / (BATCH_THREADS / tm);
     I.nsensor = (w->nvalid + s - 1) / s;
     // MVM items: about `kb` bytes of rows each
     const size_t row_bytes = (size_t)I.ld * esize;
-    const size_t slope_b = sizeof(float) * swizzled_slope_floats(I.ld, V);
     int r = (int)std::max<size_t>(1, kb / row_bytes);
-    r = std::min(r, c->nactu);
-    auto mvm_bytes = [&](int rr) { return (size_t)rr * row_bytes + slope_b + sizeof(float) * BATCH_SLOTS * rr; };
-    r = std::min(r, BATCH_MAX_ROWS);
-    while (r > 1 && mvm_bytes(r) > item_cap) --r;
-    AOB_REQUIRE(mvm_bytes(r) <= item_cap, "batch: instance " + std::to_string(i) + ": a command-matrix row does not fit");
+    r = std::min(std::min(r, c->nactu), BATCH_MAX_ROWS);
+    while (r > 1 && mvm_item_bytes(c, r) > cap) --r;
+    AOB_REQUIRE(mvm_item_bytes(c, r) <= cap,
+                "batch: instance " + std::to_string(i) + ": a command-matrix row does not fit");
     // even split of the rows over the items
     const int nit = (c->nactu + r - 1) / r;
     RPI[i] = (c->nactu + nit - 1) / nit;
@@ -496,19 +540,10 @@ void aob_batch::build(bool noise) {
                  + 2 * 4 * (int64_t)c->nslope                  // slopes written, read back
                  + 4 * 4 * (int64_t)c->nactu;                  // com read + write, err, voltage
   }
-  // the area must hold every item's shared memory with the final rows_max
+  // the area must hold every item's shared memory
   size_t area = 0;
-  for (int i = 0; i < n; ++i) {
-    aob_loop *l = loops[i];
-    aob_sh *w = l->wfs;
-    const int npix2 = w->npix * w->npix;
-    const ShSmem L(w->nfft, w->nu, w->nv, w->nphase, w->nrebin * w->nrebin * npix2, npix2, hi[i].smax);
-    const int esize = hi[i].prec == AOB_PREC_F32 ? 4 : (hi[i].prec == AOB_PREC_BF16 ? 2 : 1);
-    const int V = 16 / esize;
-    const size_t mv = (size_t)RPI[i] * hi[i].ld * esize + sizeof(float) * swizzled_slope_floats(hi[i].ld, V) +
-                      sizeof(float) * BATCH_SLOTS * RPI[i];
-    area = std::max(area, std::max(L.team_bytes(BATCH_THREADS / team_threads()), mv));
-  }
+  for (int i = 0; i < n; ++i)
+    area = std::max({area, sensor_item_bytes(loops[i]->wfs, S[i], tm), mvm_item_bytes(loops[i]->ls, RPI[i])});
   smem = batch_bars_bytes(rmax) + batch_pre_bytes(rmax) + area;
   AOB_REQUIRE(smem <= smem_cap, "batch: shared memory per CTA exceeds the budget");
   rows_max = rmax;
@@ -526,9 +561,25 @@ void aob_batch::build(bool noise) {
     const int na = loops[i]->ls->nactu;
     for (int r0 = 0; r0 < na; r0 += RPI[i]) items.push_back(make_int4(i, BI_MVM, r0, std::min(RPI[i], na - r0)));
   };
-  for (int k = 0; k < n + lag; ++k) {
-    if (k < n) emit_sensor(ord[k]);
-    if (k - lag >= 0) emit_mvm(ord[k - lag]);
+  if (lag >= 0) {
+    for (int k = 0; k < n + lag; ++k) {
+      if (k < n) emit_sensor(ord[k]);
+      if (k - lag >= 0) emit_mvm(ord[k - lag]);
+    }
+  } else {
+    // an instance's rows follow once two rounds of sensor items have been queued
+    // after its own, which by then have finished: a CTA that takes a row item too
+    // early polls until they have
+    std::vector<size_t> after(n);  // sensor items queued up to and including instance ord[k]'s
+    size_t sensors = 0;
+    int next = 0;
+    for (int k = 0; k < n; ++k) {
+      emit_sensor(ord[k]);
+      sensors += hi[ord[k]].nsensor;
+      after[k] = sensors;
+      while (next <= k && sensors >= after[next] + 2 * (size_t)nsm * cps) emit_mvm(ord[next++]);
+    }
+    while (next < n) emit_mvm(ord[next++]);
   }
   nitems = (int)items.size();
   d_items.alloc(nitems);
@@ -542,7 +593,7 @@ void aob_batch::build(bool noise) {
     d_inst[v].alloc((int64_t)sizeof(BatchInst) * n);
     AOB_CUDA(cudaMemcpy(d_inst[v].p, t.data(), sizeof(BatchInst) * n, cudaMemcpyHostToDevice));
   }
-  auto kern = cps <= 2 ? batch_step_kernel<2> : batch_step_kernel<4>;
+  auto kern = batch_kernel(cps);
   smem_opt_in(reinterpret_cast<const void *>(kern), (int)smem);  // only ever raised, per device
   int per_sm = 0;
   AOB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, BATCH_THREADS, smem));
@@ -566,13 +617,10 @@ void aob_batch::launch(bool staged, cudaStream_t s) {
   A.frames = frames.p;
   A.status = status.p;
   A.rows_max = rows_max;
-  A.team = team_threads();
+  A.team = tune.team;
   A.dep_polls = test_dep_polls ? test_dep_polls : DEP_MAX_POLLS;
   A.dep_extra = test_dep_extra;
-  if (ctas_per_sm == 0 || ctas_per_sm <= 2)
-    batch_step_kernel<2><<<grid, BATCH_THREADS, smem, s>>>(A);
-  else
-    batch_step_kernel<4><<<grid, BATCH_THREADS, smem, s>>>(A);
+  batch_kernel(tune.ctas_per_sm)<<<grid, BATCH_THREADS, smem, s>>>(A);
   AOB_LAUNCH_CHECK("batch_step_kernel");
 }
 
