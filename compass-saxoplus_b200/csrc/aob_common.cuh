@@ -49,6 +49,40 @@ inline void smem_opt_in(const void *fn, int bytes) {
   }
 }
 
+// Programmatic dependent launch.  The step of a controller is a chain of kernels of
+// a few microseconds each; started one after the other's end, every link costs
+// 1.5 - 2 us of launch latency (image, slopes, commands and voltages of a 40 x 40
+// sensor as four calls: 26.2 us a pass, 17.3 us started this way; a 512 x 512 pyramid
+// with its command matrix, nine kernels: 111.6 and 88.4 us).  A kernel started by launch_after may become
+// resident while the kernel before it on the stream still runs, once all of that
+// one's CTAs have said so (dep_launch, at their start) or ended, and waits in
+// dep_wait until it has completed and its writes are visible.  Every such
+// kernel calls dep_wait in every CTA before it reads anything another kernel
+// may write and before it writes anything; ahead of it are only index arithmetic,
+// barrier set-up and reads of tables and matrices that no kernel writes.  So a
+// kernel that completes has seen all its predecessors complete, and launches of
+// any other kind (copies, events, other libraries' kernels) order as always.
+__device__ __forceinline__ void dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void dep_sync() {
+  dep_launch();
+  dep_wait();
+}
+template <class... P, class... A>
+inline void launch_after(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  AOB_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<P>(std::forward<A>(args))...));
+}
+
 // RAII device buffer
 template <typename T>
 struct DevBuf {

@@ -34,6 +34,7 @@ struct CogArgs {
 };
 
 __global__ void cog_kernel(CogArgs A) {
+  dep_sync();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -71,6 +72,7 @@ __global__ void cog_kernel(CogArgs A) {
 // store the thresholded pixels of every valid sub-aperture into the image.
 __global__ void tcog_writeback_kernel(float *img, int size, const int32_t *validx, const int32_t *validy,
                                       int nvalid, int npix, float thresh) {
+  dep_sync();
   const int npix2 = npix * npix;
   const int64_t lim = (int64_t)size * size;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < npix2 * nvalid; t += gridDim.x * blockDim.x) {
@@ -104,6 +106,7 @@ __device__ __forceinline__ void pyr_quad(const float *img, int ns, const int32_t
 __global__ void __launch_bounds__(PYR_SLOPE_THREADS)
     pyr_flux_kernel(const float *img, int ns, const int32_t *vx, const int32_t *vy, int nvalid, float *inten,
                     float *partial) {
+  dep_sync();
   __shared__ float red[PYR_SLOPE_THREADS / 32];
   const int i = blockIdx.x * PYR_SLOPE_THREADS + threadIdx.x;
   float f = 0.f;
@@ -126,6 +129,7 @@ __global__ void __launch_bounds__(PYR_SLOPE_THREADS)
     pyr_slopes_kernel(const float *img, int ns, const int32_t *vx, const int32_t *vy, int nvalid, float scale,
                       float thresh, int method, const float *ref, int order, const float *partial, int nparts,
                       float *slopes, float *inten) {
+  dep_sync();
   __shared__ float s_mean;
   const bool sinus = (method & 1) == 0, local = method > 1;
   if (threadIdx.x < 32) {
@@ -268,6 +272,7 @@ static int bpcog_block(int n) {
 template <typename Tin>
 __global__ void calib_kernel(const Tin *raw, float *cal, const float *dark, const float *flat, const int32_t *lut,
                              int64_t n) {
+  dep_sync();
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x)
     cal[t] = ((float)raw[lut[t]] - dark[t]) * flat[t];
 }
@@ -280,6 +285,7 @@ template <typename Tin>
 __global__ void calib_valid_kernel(const Tin *raw, float *cal, const float *dark, const float *flat,
                                    const int32_t *lut, const int32_t *vx, const int32_t *vy, int nvalid, int npix,
                                    int size) {
+  dep_sync();
   const int npix2 = npix * npix;
   const int64_t lim = (int64_t)size * size;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < (int64_t)nvalid * npix2;
@@ -340,9 +346,9 @@ void aob_centro::calibrate(cudaStream_t s, bool valid_only) {
   if (!valid_only) {
     const int grid = (int)std::min<int64_t>((n + 255) / 256, 4096);
     if (raw_u16)
-      calib_kernel<uint16_t><<<grid, 256, 0, s>>>(img_raw_u16.p, img.p, dark.p, flat.p, lut.p, n);
+      launch_after(calib_kernel<uint16_t>, grid, 256, 0, s, img_raw_u16.p, img.p, dark.p, flat.p, lut.p, n);
     else
-      calib_kernel<float><<<grid, 256, 0, s>>>(img_raw.p, img.p, dark.p, flat.p, lut.p, n);
+      launch_after(calib_kernel<float>, grid, 256, 0, s, img_raw.p, img.p, dark.p, flat.p, lut.p, n);
     AOB_LAUNCH_CHECK("calib_kernel");
     return;
   }
@@ -355,10 +361,10 @@ void aob_centro::calibrate(cudaStream_t s, bool valid_only) {
   const int64_t work = (int64_t)nv * np * np;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((work + 255) / 256, 4096));
   if (raw_u16)
-    calib_valid_kernel<uint16_t><<<grid, 256, 0, s>>>(img_raw_u16.p, img.p, dark.p, flat.p, lut.p, validx.p,
+    launch_after(calib_valid_kernel<uint16_t>, grid, 256, 0, s, img_raw_u16.p, img.p, dark.p, flat.p, lut.p, validx.p,
                                                       validy.p, nv, np, img_m);
   else
-    calib_valid_kernel<float><<<grid, 256, 0, s>>>(img_raw.p, img.p, dark.p, flat.p, lut.p, validx.p, validy.p, nv,
+    launch_after(calib_valid_kernel<float>, grid, 256, 0, s, img_raw.p, img.p, dark.p, flat.p, lut.p, validx.p, validy.p, nv,
                                                    np, img_m);
   AOB_LAUNCH_CHECK("calib_valid_kernel");
 }
@@ -420,10 +426,10 @@ void aob_centro::get_cog(float *dev_slopes, cudaStream_t s) {
     AOB_CUDA(cudaSetDevice(device));
     const int nparts = (nvalid + PYR_SLOPE_THREADS - 1) / PYR_SLOPE_THREADS;
     if (pyr_partial.n < nparts) pyr_partial.alloc(nparts);
-    pyr_flux_kernel<<<nparts, PYR_SLOPE_THREADS, 0, s>>>(im, ns, validx.p, validy.p, nvalid, intensities.p,
+    launch_after(pyr_flux_kernel, nparts, PYR_SLOPE_THREADS, 0, s, im, ns, validx.p, validy.p, nvalid, intensities.p,
                                                         pyr_partial.p);
     AOB_LAUNCH_CHECK("pyr_flux_kernel");
-    pyr_slopes_kernel<<<nparts, PYR_SLOPE_THREADS, 0, s>>>(im, ns, validx.p, validy.p, nvalid, scale, valid_thresh,
+    launch_after(pyr_slopes_kernel, nparts, PYR_SLOPE_THREADS, 0, s, im, ns, validx.p, validy.p, nvalid, scale, valid_thresh,
                                                           pyr_method, ref.p, order, pyr_partial.p, nparts, dev_slopes,
                                                           intensities.p);
     AOB_LAUNCH_CHECK("pyr_slopes_kernel");
@@ -439,7 +445,7 @@ void aob_centro::get_cog(float *dev_slopes, cudaStream_t s) {
                              cudaMemcpyDeviceToDevice, s));
     if (type == 1) {
       const int n = npix * npix * nvalid;
-      tcog_writeback_kernel<<<std::min((n + 255) / 256, 4096), 256, 0, s>>>(
+      launch_after(tcog_writeback_kernel, std::min((n + 255) / 256, 4096), 256, 0, s, 
           wfs->binimg.p, wfs->npix * wfs->nxsub, validx.p, validy.p, nvalid, npix, threshold);
       AOB_LAUNCH_CHECK("tcog_writeback_kernel");
       ++wfs->image_gen;  // a second get_cog thresholds again, as the reference does
@@ -472,7 +478,7 @@ void aob_centro::get_cog(float *dev_slopes, cudaStream_t s) {
   A.intens = intensities.p;
   const int warps_per_block = 8;
   const int grid = std::max(1, std::min((nvalid + warps_per_block - 1) / warps_per_block, num_sms(device) * 8));
-  cog_kernel<<<grid, warps_per_block * 32, 0, s>>>(A);
+  launch_after(cog_kernel, grid, warps_per_block * 32, 0, s, A);
   AOB_LAUNCH_CHECK("cog_kernel");
   if (wfs && type == 1) ++wfs->image_gen;
 }

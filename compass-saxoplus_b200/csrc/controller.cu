@@ -118,6 +118,7 @@ __host__ __device__ inline int mvm_smem_floats(int ld, int v) { return ((ld / v 
 
 template <typename T>
 __global__ void __launch_bounds__(MVM_THREADS) ls_mvm_kernel(MvmArgs A) {
+  dep_sync();
   extern __shared__ __align__(16) float s_sh[];
   if (A.use && *A.use == 0u) return;
   constexpr int V = Pack<T>::N;
@@ -197,7 +198,11 @@ __global__ void __launch_bounds__(MVM_THREADS) ls_mvm_bulk_kernel(MvmArgs A) {
   const int r0 = (int)((blockIdx.x * (uint32_t)A.nrow) / gridDim.x);  // 32-bit: host-checked range
   const int r1 = (int)(((blockIdx.x + 1) * (uint32_t)A.nrow) / gridDim.x);
   const int R = r1 - r0;
-  if (A.use && *A.use == 0u) return;
+  dep_launch();
+  if (A.use) {
+    dep_wait();
+    if (*A.use == 0u) return;
+  }
   // shared memory: barriers | slopes | rows | per-warp partial sums
   uint64_t *bars = reinterpret_cast<uint64_t *>(sm);
   float *s_sh = reinterpret_cast<float *>(sm + mvm_bars_bytes(A.rows_per_cta));
@@ -214,6 +219,7 @@ __global__ void __launch_bounds__(MVM_THREADS) ls_mvm_bulk_kernel(MvmArgs A) {
     for (int r = 0; r < R; ++r)
       bulk_g2s(rows + (size_t)r * row_bytes, src + (size_t)r * row_bytes, row_bytes, &bars[0]);
   }
+  dep_wait();  // (the rows, which no kernel writes, are on their way while the slopes' producer ends)
   if (A.bump && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(A.bump, 1u);
   // epilogue inputs of this thread's row (R <= blockDim), fetched now
   float e_sc = 1.f, e_mg = 1.f, e_cm = 0.f;
@@ -291,6 +297,7 @@ __global__ void __launch_bounds__(MVM_THREADS) ls_mvm_bulk_kernel(MvmArgs A) {
 // One warp per row; the row sum runs lane-strided, then a butterfly.
 __global__ void gemv_rows_kernel(const float *A, int lda, int nrow, int ncol, const float *x, float alpha, float beta,
                                  float *y) {
+  dep_sync();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const int nw = (gridDim.x * blockDim.x) >> 5;
@@ -305,10 +312,12 @@ __global__ void gemv_rows_kernel(const float *A, int lda, int nrow, int ncol, co
 
 // x[i] = x[i] * scale[i] * gain (mult_krnl, libsutra/src.cu/sutra_utils.cu:603-610)
 __global__ void mult_vec_kernel(float *x, const float *scale, float gain, int n) {
+  dep_sync();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) x[i] = x[i] * scale[i] * gain;
 }
 // y[i] += x[i] (axpy with alpha 1)
 __global__ void add_vec_kernel(float *y, const float *x, int n) {
+  dep_sync();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) y[i] += x[i];
 }
 
@@ -329,6 +338,7 @@ struct VoltArgs {
 };
 
 __global__ void voltage_kernel(VoltArgs A) {
+  dep_sync();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < A.n; i += gridDim.x * blockDim.x) {
     float v;
     if (A.delayed) {
@@ -344,11 +354,13 @@ __global__ void voltage_kernel(VoltArgs A) {
 }
 
 __global__ void add_perturb_kernel(float *y, const float *buf, int cpt, int nper, int n) {
+  dep_sync();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     y[i] += buf[cpt + (int64_t)i * nper];
 }
 
 __global__ void clip_kernel(float *x, int n, float lo, float hi) {
+  dep_sync();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     x[i] = fminf(fmaxf(x[i], lo), hi);
 }
@@ -488,11 +500,11 @@ void launch_mvm_t(const MvmArgs &A0, int grid, bool bulk, cudaStream_t s) {
     const size_t sm = mvm_bars_bytes(A.rows_per_cta) + slope_bytes + (size_t)A.rows_per_cta * A.ld * sizeof(T) +
                       sizeof(float) * (MVM_THREADS / 32) * A.rows_per_cta;
     smem_opt_in(reinterpret_cast<const void *>(ls_mvm_bulk_kernel<T>), (int)sm);
-    ls_mvm_bulk_kernel<T><<<grid, MVM_THREADS, sm, s>>>(A);
+    launch_after(ls_mvm_bulk_kernel<T>, grid, MVM_THREADS, sm, s, A);
     AOB_LAUNCH_CHECK("ls_mvm_bulk_kernel");
   } else {
     smem_opt_in(reinterpret_cast<const void *>(ls_mvm_kernel<T>), (int)slope_bytes);
-    ls_mvm_kernel<T><<<grid, MVM_THREADS, slope_bytes, s>>>(A);
+    launch_after(ls_mvm_kernel<T>, grid, MVM_THREADS, slope_bytes, s, A);
     AOB_LAUNCH_CHECK("ls_mvm_kernel");
   }
 }
@@ -541,7 +553,7 @@ void aob_ls::generic_comp_com(cudaStream_t s, uint32_t *bump) {
   if (polc) {
     AOB_REQUIRE(imat_rows.p != nullptr, "comp_com: polc needs the interaction matrix (set_imat)");
     AOB_CUDA(cudaMemcpyAsync(ol_meas.p, centroids.p, sizeof(float) * nslope, cudaMemcpyDeviceToDevice, s));
-    gemv_rows_kernel<<<std::max(1, std::min((nslope + 7) / 8, 4096)), 256, 0, s>>>(
+    launch_after(gemv_rows_kernel, std::max(1, std::min((nslope + 7) / 8, 4096)), 256, 0, s, 
         imat_rows.p, nactu, nslope, nactu, com_clipped.p, -1.f, 1.f, ol_meas.p);
     AOB_LAUNCH_CHECK("gemv_rows_kernel (polc)");
     sin = ol_meas.p;
@@ -574,11 +586,11 @@ void aob_ls::generic_comp_com(cudaStream_t s, uint32_t *bump) {
   if (law == AOB_LAW_INTEGRATOR) return;
   // err = -(cmat s); buff = err * modal gains
   AOB_REQUIRE(matE_rows.p != nullptr, "comp_com: this command law needs matE (set_matE)");
-  mult_vec_kernel<<<grid_v, thr, 0, s>>>(err.p, gains.p, 1.f, nactu);
+  launch_after(mult_vec_kernel, grid_v, thr, 0, s, err.p, gains.p, 1.f, nactu);
   AOB_LAUNCH_CHECK("mult_vec_kernel");
   const int grid_r = std::max(1, std::min((nactu + 7) / 8, 4096));
   if (law == AOB_LAW_MODAL_INTEGRATOR) {
-    gemv_rows_kernel<<<grid_r, 256, 0, s>>>(matE_rows.p, nactu, nactu, nactu, err.p, gain, berta, com());
+    launch_after(gemv_rows_kernel, grid_r, 256, 0, s, matE_rows.p, nactu, nactu, nactu, err.p, gain, berta, com());
     AOB_LAUNCH_CHECK("gemv_rows_kernel (modal integrator)");
     return;
   }
@@ -590,10 +602,10 @@ void aob_ls::generic_comp_com(cudaStream_t s, uint32_t *bump) {
     AOB_CUDA(cudaMemcpyAsync(com1_tmp.p, com(), sizeof(float) * nactu, cudaMemcpyDeviceToDevice, s));
     com1 = com1_tmp.p;
   }
-  gemv_rows_kernel<<<grid_r, 256, 0, s>>>(matE_rows.p, nactu, nactu, nactu, com1, 1.f, 0.f, com());
+  launch_after(gemv_rows_kernel, grid_r, 256, 0, s, matE_rows.p, nactu, nactu, nactu, com1, 1.f, 0.f, com());
   AOB_LAUNCH_CHECK("gemv_rows_kernel (2matrices)");
-  mult_vec_kernel<<<grid_v, thr, 0, s>>>(com(), decay.p, 1.f, nactu);
-  add_vec_kernel<<<grid_v, thr, 0, s>>>(com(), err.p, nactu);
+  launch_after(mult_vec_kernel, grid_v, thr, 0, s, com(), decay.p, 1.f, nactu);
+  launch_after(add_vec_kernel, grid_v, thr, 0, s, com(), err.p, nactu);
   AOB_LAUNCH_CHECK("2matrices update");
 }
 
@@ -651,7 +663,7 @@ void aob_ls::comp_voltage(cudaStream_t s) {
   A.do_clip = volt_min < volt_max ? 1 : 0;
   A.out = com_clipped.p;
   A.n = nactu;
-  voltage_kernel<<<std::max(1, std::min((nactu + 255) / 256, 1024)), 256, 0, s>>>(A);
+  launch_after(voltage_kernel, std::max(1, std::min((nactu + 255) / 256, 1024)), 256, 0, s, A);
   AOB_LAUNCH_CHECK("voltage_kernel");
   if (A.delayed) {
     // the oldest buffer now holds a copy of the current command and becomes it
@@ -669,7 +681,7 @@ void aob_ls::apply_perturb(cudaStream_t s) {
   for (auto &kv : perturb) {
     Perturb &p = kv.second;
     if (!p.on) continue;
-    add_perturb_kernel<<<grid, 256, 0, s>>>(com_clipped.p, p.buf.p, p.cpt, p.n, nactu);
+    launch_after(add_perturb_kernel, grid, 256, 0, s, com_clipped.p, p.buf.p, p.cpt, p.n, nactu);
     AOB_LAUNCH_CHECK("add_perturb_kernel");
     p.cpt = (p.cpt < p.n - 1) ? p.cpt + 1 : 0;
   }
@@ -678,7 +690,7 @@ void aob_ls::apply_perturb(cudaStream_t s) {
 void aob_ls::clip(cudaStream_t s) {
   if (!(volt_min < volt_max)) return;
   AOB_CUDA(cudaSetDevice(device));
-  clip_kernel<<<std::max(1, std::min((nactu + 255) / 256, 1024)), 256, 0, s>>>(com_clipped.p, nactu, volt_min, volt_max);
+  launch_after(clip_kernel, std::max(1, std::min((nactu + 255) / 256, 1024)), 256, 0, s, com_clipped.p, nactu, volt_min, volt_max);
   AOB_LAUNCH_CHECK("clip_kernel");
 }
 

@@ -40,6 +40,7 @@ __global__ void f32_to_bf16_kernel(const float *src, __nv_bfloat16 *dst, int64_t
 // every row starts on 16 bytes).  Bound: DRAM (x is read once).
 __global__ void __launch_bounds__(256)
     mlp_input_kernel(const float *x, int nin, int pin, int64_t ngrp, int vec, float scale, __nv_bfloat16 *xb) {
+  dep_sync();
   const int gpr = pin / 4;  // groups per row
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t g0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g0 < ngrp; g0 += 2 * stride) {
@@ -88,6 +89,7 @@ constexpr int LOSS_ROWS = 64;  // rows per block
 __global__ void __launch_bounds__(256)
     mlp_loss_kernel(const float *y, const float *t, int nout, int pout, int batch, float inv_out_scale,
                     __nv_bfloat16 *dy, float *colpart, float *part) {
+  dep_sync();
   __shared__ float red[8][33], red2[8];
   const float g = 2.f / ((float)batch * (float)nout);
   const int c = blockIdx.x * 32 + threadIdx.x;
@@ -186,6 +188,7 @@ struct FinishArgs {
   float *loss;  // or null
 };
 __global__ void __launch_bounds__(256) mlp_finish_kernel(const __grid_constant__ FinishArgs A) {
+  dep_sync();
   __shared__ float red[8][33];
   if ((int)blockIdx.x == A.block0[3]) {
     float s = 0.f;
@@ -228,6 +231,7 @@ struct AdamArgs {
   float lr, b1, b2, eps, c1, c2;
 };
 __global__ void __launch_bounds__(256) mlp_adam_kernel(const __grid_constant__ AdamArgs A) {
+  dep_sync();
   const int64_t total = A.end[ADAM_SEGS - 1];
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
     int l = 0;
@@ -477,7 +481,7 @@ static void tc_gemm(const TcOp *ops, int n, int device, uint32_t *status, cudaSt
     M.m[2 * i + 1] = M.m[1];
   }
   smem_opt_in(reinterpret_cast<const void *>(tc_gemm_kernel), (int)TC_SMEM_BYTES);
-  tc_gemm_kernel<<<2 * (int)std::min<int64_t>(tiles, pairs), TC_THREADS, TC_SMEM_BYTES, s>>>(M, T);
+  launch_after(tc_gemm_kernel, 2 * (int)std::min<int64_t>(tiles, pairs), TC_THREADS, TC_SMEM_BYTES, s, M, T);
   AOB_LAUNCH_CHECK("tc_gemm_kernel");
 }
 
@@ -609,7 +613,7 @@ void aob_mlp::forward(const float *x, int batch, float *y_out, cudaStream_t s) {
   {
     const int64_t ngrp = (int64_t)batch * (pin / 4);
     const int vec = nin % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
-    mlp_input_kernel<<<(int)std::max<int64_t>(1, std::min<int64_t>((ngrp + 511) / 512, 8 * num_sms(device))), 256, 0, s>>>(
+    launch_after(mlp_input_kernel, (int)std::max<int64_t>(1, std::min<int64_t>((ngrp + 511) / 512, 8 * num_sms(device))), 256, 0, s, 
         x, nin, pin, ngrp, vec, in_scale, bf(xb));
     AOB_LAUNCH_CHECK("mlp_input_kernel");
   }
@@ -651,7 +655,7 @@ void aob_mlp::backward(const float *target, int batch, float *loss, cudaStream_t
   AOB_REQUIRE(batch <= cap, "mlp.backward: run forward on this batch first");
   AOB_CUDA(cudaSetDevice(device));
   const dim3 lgrid((pout + 31) / 32, (batch + LOSS_ROWS - 1) / LOSS_ROWS);
-  mlp_loss_kernel<<<lgrid, dim3(32, 8), 0, s>>>(y.p, target, nout, pout, batch, 1.f / out_scale, bf(dy), colpart[2].p,
+  launch_after(mlp_loss_kernel, lgrid, dim3(32, 8), 0, s, y.p, target, nout, pout, batch, 1.f / out_scale, bf(dy), colpart[2].p,
                                                 loss_part.p);
   AOB_LAUNCH_CHECK("mlp_loss_kernel");
   // data gradients: dz2 = (dy W3) * GELU'(z2), dz1 = (dz2 W2) * GELU'(z1)
@@ -707,7 +711,7 @@ void aob_mlp::backward(const float *target, int batch, float *loss, cudaStream_t
   F.nloss = (int)(lgrid.x * lgrid.y);
   F.denom = (float)batch * (float)nout;
   F.loss = loss;
-  mlp_finish_kernel<<<F.block0[3] + (loss ? 1 : 0), dim3(32, 8), 0, s>>>(F);
+  launch_after(mlp_finish_kernel, F.block0[3] + (loss ? 1 : 0), dim3(32, 8), 0, s, F);
   AOB_LAUNCH_CHECK("mlp_finish_kernel");
 }
 
@@ -733,7 +737,7 @@ void aob_mlp::adam(float lr, cudaStream_t s) {
     end += (weight ? w[l].n : b[l].n) / 4;
     A.end[q] = end;
   }
-  mlp_adam_kernel<<<(int)std::max<int64_t>(1, std::min<int64_t>((end + 255) / 256, 8 * num_sms(device))), 256, 0, s>>>(A);
+  launch_after(mlp_adam_kernel, (int)std::max<int64_t>(1, std::min<int64_t>((end + 255) / 256, 8 * num_sms(device))), 256, 0, s, A);
   AOB_LAUNCH_CHECK("mlp_adam_kernel");
 }
 

@@ -275,6 +275,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
   uint64_t *empty = full + TC_STAGES;
   uint64_t *accfull = empty + TC_STAGES, *accempty = accfull + 2;
   uint32_t *tslot = reinterpret_cast<uint32_t *>(accempty + 2);
+  dep_launch();
   if (threadIdx.x == 0) {
     for (int s = 0; s < TC_STAGES; ++s) {
       mbar_init(&full[s], 1);
@@ -295,6 +296,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
   __syncthreads();
   cluster_sync();  // both CTAs' barriers exist before either's loads, MMAs or arrivals
   tc_fence_after();
+  dep_wait();
   const uint32_t tmem = *tslot;
   const int bn = T.bn, bh = bn / 2;
   bool ok = true;

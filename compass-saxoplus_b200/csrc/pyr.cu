@@ -78,7 +78,9 @@ __global__ void __launch_bounds__(PYR_ROW_THREADS) pyr_rows_kernel(PyrArgs A) {
   const bool active = q < A.npts * A.ntot;
   const int p = active ? q / A.ntot : 0, yb = active ? q - p * A.ntot : 0;
   FftTw<N> W;
+  dep_launch();
   W.load(A.tw, j);
+  dep_wait();
   const float cxp = A.cx[p], cyp = A.cy[p];
   const float yy = (float)yb - A.ntot / 2.0f;
   float2 v[8];
@@ -124,6 +126,7 @@ __global__ void __launch_bounds__(N / 8 * pyr_cols(N)) pyr_cols_kernel(PyrArgs A
   const int x = blockIdx.x * CB + c;
   float2 *s = sm + c;
   FftTw<N> W;
+  dep_launch();
   W.load(A.tw, j);
   float2 mask[8];
 #pragma unroll
@@ -144,6 +147,7 @@ __global__ void __launch_bounds__(N / 8 * pyr_cols(N)) pyr_cols_kernel(PyrArgs A
   // rows [0, ntot) hold the input and are overwritten by the output: every
   // thread of the column has its input in registers by the first barrier
   float2 nxt[8];
+  dep_wait();
   load(nxt, blockIdx.y);
   for (int p = blockIdx.y; p < A.npts; p += gridDim.y) {
     float2 v[8];
@@ -184,7 +188,9 @@ __global__ void __launch_bounds__(PYR_THREADS) pyr_accum_kernel(PyrArgs A) {
   const GroupSync<T> sync{g};
   float2 *s = sm + g * 2 * BS;
   FftTw<N> W;
+  dep_launch();
   W.load(A.tw, j);
+  dep_wait();
   float acc[8];
 #pragma unroll
   for (int m = 0; m < 8; ++m) acc[m] = 0.f;
@@ -248,13 +254,14 @@ __global__ void __launch_bounds__(N / 8 * pyr_conv_cols(N)) pyr_conv_cols_kernel
   float2 *s = sm + c;
   float2 v[8];
   float msk[8];
-#pragma unroll
-  for (int m = 0; m < 8; ++m) {
-    v[m] = A.conv[x + (size_t)(j + T * m) * N];
-    msk[m] = A.sincar[x + (size_t)(j + T * m) * N];
-  }
   FftTw<N> W;
+  dep_launch();
   W.load(A.tw, j);
+#pragma unroll
+  for (int m = 0; m < 8; ++m) msk[m] = A.sincar[x + (size_t)(j + T * m) * N];
+  dep_wait();
+#pragma unroll
+  for (int m = 0; m < 8; ++m) v[m] = A.conv[x + (size_t)(j + T * m) * N];
   fft_regs<N, CB, BS, true>(v, W, j, s, CtaSync{});
   if (fft_odd_exchanges(N)) __syncthreads();
 #pragma unroll
@@ -277,7 +284,9 @@ __global__ void __launch_bounds__(PYR_THREADS) pyr_bin_kernel(PyrArgs A, int row
   float *real = reinterpret_cast<float *>(sm + G * 2 * BS);  // rows x N
   const int y0 = blockIdx.x * rows;
   FftTw<N> W;
+  dep_launch();
   W.load(A.tw, j);
+  dep_wait();
   for (int r = g; r < rows; r += G) {  // rows is a multiple of G
     float2 v[8];
 #pragma unroll
@@ -309,6 +318,7 @@ __global__ void __launch_bounds__(PYR_THREADS) pyr_bin_kernel(PyrArgs A, int row
 // 6. normalisation to nphot (sum of the row sums in row order) and noise.
 __global__ void pyr_norm_noise_kernel(float *binimg, const float *partial, int nb, float nphot, int noise_mode,
                                       float noise, uint32_t frame, uint32_t k0, uint32_t k1) {
+  dep_sync();
   __shared__ float s_fact;
   __shared__ float rk[AOB_POISSON_INV_KMAX + 1];
   if (noise_mode >= 1)
@@ -337,6 +347,7 @@ __global__ void pyr_norm_noise_kernel(float *binimg, const float *partial, int n
 // focal plane: the per-point images summed in point order from zero, as the
 // reference accumulates d_pyrfocalplane (sutra_wfs_pyr_pyrhr.cpp:398-401,501-506)
 __global__ void pyr_focal_sum_kernel(float *focal, const float *work, int npts, int64_t n2) {
+  dep_sync();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n2; i += (int64_t)gridDim.x * blockDim.x) {
     float acc = 0.f;
     for (int p = 0; p < npts; ++p) acc += work[(size_t)p * n2 + i];
@@ -355,7 +366,7 @@ static void pyr_launch(const PyrArgs &A, int device, cudaStream_t s) {
   const int nsm = num_sms(device);
   {
     constexpr int SEQ = PYR_ROW_THREADS / T;
-    pyr_rows_kernel<N><<<(A.npts * A.ntot + SEQ - 1) / SEQ, PYR_ROW_THREADS, 0, s>>>(A);
+    launch_after(pyr_rows_kernel<N>, (A.npts * A.ntot + SEQ - 1) / SEQ, PYR_ROW_THREADS, 0, s, A);
     AOB_LAUNCH_CHECK("pyr_rows_kernel");
   }
   {
@@ -376,7 +387,7 @@ static void pyr_launch(const PyrArgs &A, int device, cudaStream_t s) {
         split = ps;
       }
     }
-    kern<<<dim3(groups, split), threads, sm, s>>>(A);
+    launch_after(kern, dim3(groups, split), threads, sm, s, A);
     AOB_LAUNCH_CHECK("pyr_cols_kernel");
   }
   {
@@ -385,14 +396,14 @@ static void pyr_launch(const PyrArgs &A, int device, cudaStream_t s) {
     const int G = std::min(PYR_THREADS / T, (A.npts + unit - 1) / unit * unit);
     const size_t sm = std::max(sizeof(float2) * 2 * BS * G, sizeof(float) * N * G);
     pyr_smem(pyr_accum_kernel<N>, sm);
-    pyr_accum_kernel<N><<<N, G * T, sm, s>>>(A);
+    launch_after(pyr_accum_kernel<N>, N, G * T, sm, s, A);
     AOB_LAUNCH_CHECK("pyr_accum_kernel");
   }
   {
     constexpr int CB = pyr_conv_cols(N);
     const size_t sm = sizeof(float2) * 2 * BS * CB;
     pyr_smem(pyr_conv_cols_kernel<N>, sm);
-    pyr_conv_cols_kernel<N><<<N / CB, T * CB, sm, s>>>(A);
+    launch_after(pyr_conv_cols_kernel<N>, N / CB, T * CB, sm, s, A);
     AOB_LAUNCH_CHECK("pyr_conv_cols_kernel");
   }
   {
@@ -401,7 +412,7 @@ static void pyr_launch(const PyrArgs &A, int device, cudaStream_t s) {
     const int G = std::min(rows, PYR_THREADS / T);
     const size_t sm = sizeof(float2) * 2 * BS * G + sizeof(float) * N * rows;
     pyr_smem(pyr_bin_kernel<N>, sm);
-    pyr_bin_kernel<N><<<N / rows, G * T, sm, s>>>(A, rows);
+    launch_after(pyr_bin_kernel<N>, N / rows, G * T, sm, s, A, rows);
     AOB_LAUNCH_CHECK("pyr_bin_kernel");
   }
 }
@@ -511,14 +522,14 @@ void aob_pyr::comp_image(bool with_noise, cudaStream_t s) {
     default: pyr_launch<2048>(A, device, s); break;
   }
   if (compute_focalplane) {
-    pyr_focal_sum_kernel<<<(int)std::min<int64_t>((n2 + 255) / 256, 8 * num_sms(device)), 256, 0, s>>>(
+    launch_after(pyr_focal_sum_kernel, (int)std::min<int64_t>((n2 + 255) / 256, 8 * num_sms(device)), 256, 0, s, 
         focalplane.p, focal_work.p, npts, n2);
     AOB_LAUNCH_CHECK("pyr_focal_sum_kernel");
   }
   const float nz = with_noise ? noise : -1.f;
   const int noise_mode = nz > 0 ? 2 : (nz > -1 ? 1 : 0);
   const int nb2 = nbin() * nbin();
-  pyr_norm_noise_kernel<<<std::min((nb2 + 255) / 256, 4 * num_sms(device)), 256, 0, s>>>(
+  launch_after(pyr_norm_noise_kernel, std::min((nb2 + 255) / 256, 4 * num_sms(device)), 256, 0, s, 
       binimg.p, partial.p, nbin(), nphot, noise_mode, nz, (uint32_t)frame, (uint32_t)((uint64_t)seed & 0xffffffffu),
       (uint32_t)((uint64_t)seed >> 32));
   AOB_LAUNCH_CHECK("pyr_norm_noise_kernel");

@@ -49,7 +49,9 @@ __global__ void __launch_bounds__(SH_THREADS) sh_image_kernel(ShKernelArgs P, in
   extern __shared__ __align__(16) unsigned char smem[];
   const int pd = PD > 0 ? PD : P.pdiam;
   const ShSmem L(NFFT, P.nu, P.nv, pd, P.nrebin2 * P.npix * P.npix, P.npix * P.npix, S);
+  dep_launch();
   sh_load_tables<NFFT>(P, smem, threadIdx.x, blockDim.x);
+  dep_wait();
   // (the barrier closing sh_batch's stage 1 publishes the tables: stages 0-1
   // read none of them, so their loads overlap the field's)
   for (int base = blockIdx.x; base < P.nvalid; base += S * gridDim.x) {
@@ -90,6 +92,7 @@ __global__ void fs_mask_kernel(float2 *d, const float *mask, int64_t n2) {
 // (the float-to-integer conversion saturates at 0 and 65535).
 __global__ void digitalize_kernel(uint16_t *cam, const float *img, const float *dark, const float *flat,
                                   int max_flux, int max_pix, int64_t n) {
+  dep_sync();
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
     float v = (img[t] * flat[t] + dark[t]) / (float)max_flux;
     v = v < 1.f ? v : 1.f;
@@ -99,6 +102,7 @@ __global__ void digitalize_kernel(uint16_t *cam, const float *img, const float *
 
 __global__ void sh_fill_image_kernel(float *img, const float *cube, const int32_t *vx,
                                      const int32_t *vy, int npix, int nvalid, int size) {
+  dep_sync();
   const int npix2 = npix * npix;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < npix2 * nvalid; t += gridDim.x * blockDim.x) {
     const int k = t / npix2, p = t - k * npix2;
@@ -275,7 +279,7 @@ static void launch_sh_fs(const ShKernelArgs &P, int nvalid, int S, size_t sm, cu
   const int grid = std::max(1, (nvalid + S - 1) / S);
   // opt-in per (kernel, device), only ever raised (a driver call per launch costs microseconds)
   smem_opt_in(reinterpret_cast<const void *>(sh_image_kernel<NFFT, PD, FS>), (int)std::max<size_t>(sm, 48 * 1024));
-  sh_image_kernel<NFFT, PD, FS><<<grid, SH_THREADS, sm, s>>>(P, S);
+  launch_after(sh_image_kernel<NFFT, PD, FS>, grid, SH_THREADS, sm, s, P, S);
 }
 template <int NFFT, int PD>
 static void launch_sh(const ShKernelArgs &P, int nvalid, int S, size_t sm, cudaStream_t s) {
@@ -443,7 +447,7 @@ void aob_sh::set_fakecam(int enable, int max_flux, int max_pix) {
 
 void aob_sh::digitalize(cudaStream_t s) {
   const int64_t n = binimg.n;
-  digitalize_kernel<<<(int)std::min<int64_t>((n + 255) / 256, 4096), 256, 0, s>>>(
+  launch_after(digitalize_kernel, (int)std::min<int64_t>((n + 255) / 256, 4096), 256, 0, s, 
       camimg.p, binimg.p, cam_dark.p, cam_flat.p, max_flux_per_pix, max_pix_value, n);
   AOB_LAUNCH_CHECK("digitalize_kernel");
 }
@@ -451,7 +455,7 @@ void aob_sh::digitalize(cudaStream_t s) {
 void aob_sh::fill_binimage(cudaStream_t s) {
   AOB_CUDA(cudaSetDevice(device));
   const int n = npix * npix * nvalid;
-  sh_fill_image_kernel<<<std::min((n + 255) / 256, 4096), 256, 0, s>>>(
+  launch_after(sh_fill_image_kernel, std::min((n + 255) / 256, 4096), 256, 0, s, 
       binimg.p, bincube.p, validsubsx.p, validsubsy.p, npix, nvalid, npix * nxsub);
   AOB_LAUNCH_CHECK("sh_fill_image_kernel");
   ++image_gen;

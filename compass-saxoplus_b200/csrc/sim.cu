@@ -96,7 +96,7 @@ constexpr int EXTRUDE_PRE_Z = 2;  // stencil points a thread gathers ahead (nst 
 constexpr int EXTRUDE_ILP = 4;    // shift loads in flight per thread
 
 __global__ void __launch_bounds__(256) extrude_fused_kernel(const __grid_constant__ ExtrudeBatch B) {
-  if ((int)blockIdx.y >= B.njobs) return;
+  dep_launch();
   const ExtrudeJob &J = B.job[blockIdx.y];
   const int n = J.n, nst = J.nst, dir = J.dir;
   const float *__restrict__ src = J.src;
@@ -108,7 +108,6 @@ __global__ void __launch_bounds__(256) extrude_fused_kernel(const __grid_constan
   const bool pre = r0 < n && nst <= 32 * EXTRUDE_PRE && n <= 32 * EXTRUDE_PRE;
   float ref = 0.f;
   uint32_t iz[EXTRUDE_PRE_Z];
-  if (rows) ref = src[J.x0ref];
   if (prez) {
 #pragma unroll
     for (int q = 0; q < EXTRUDE_PRE_Z; ++q) {
@@ -127,6 +126,8 @@ __global__ void __launch_bounds__(256) extrude_fused_kernel(const __grid_constan
       pb[q] = t < n ? __ldg(b + t) : 0.f;
     }
   }
+  dep_wait();  // (the operators and the stencil, which no kernel writes, are on their way)
+  if (rows) ref = src[J.x0ref];
   // the shift; the new column / row is left to the rows below.  n*n < 2^31
   // (the stencil and column fit 48 KB of shared memory, so n < 12288).
   const int nn = n * n;
@@ -219,12 +220,13 @@ void launch_extrude(const ExtrudeBatch &B, int device, cudaStream_t s) {
   const int64_t want = std::max<int64_t>((nmax + rows_per_cta - 1) / rows_per_cta,
                                          (nn + threads * EXTRUDE_ILP - 1) / (threads * EXTRUDE_ILP));
   const int gx = (int)std::max<int64_t>(1, std::min<int64_t>(want, 4 * num_sms(device)));
-  extrude_fused_kernel<<<dim3(gx, B.njobs), threads, sm, s>>>(B);
+  launch_after(extrude_fused_kernel, dim3(gx, B.njobs), threads, sm, s, B);
   AOB_LAUNCH_CHECK("extrude_fused_kernel");
 }
 
 // ------------------------------------------------------------------ raytrace
 __global__ void raytrace_kernel(float *out, int nx, int ny, RaySources S, int reset) {
+  dep_sync();
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
   if (x >= nx || y >= ny) return;
@@ -254,6 +256,7 @@ constexpr int DM_GROUP = 16;
 
 __global__ void dm_shape_kernel(float *shape, int npix, const int32_t *rowptr, const int32_t *act, const float *w,
                                 const float *com) {
+  dep_sync();
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < npix; p += gridDim.x * blockDim.x) {
     const int k0 = __ldg(rowptr + p), k1 = __ldg(rowptr + p + 1);
     float v = 0.f;
@@ -292,9 +295,13 @@ __global__ void __launch_bounds__(TGT_THREADS)
                        unsigned int *maxes) {
   constexpr int T = N / 8, SEQ = TGT_THREADS / T, BS = fft_smem_elems(N);
   __shared__ float2 s[BS > 0 ? SEQ * 2 * BS : 1];
-  if (blockIdx.x == 0 && threadIdx.x < 2) maxes[threadIdx.x] = 0u;
   const int g = threadIdx.x / T, j = threadIdx.x % T;
   const int y = blockIdx.x * SEQ + g;
+  FftTw<N> W;
+  dep_launch();
+  W.load(tw, j);
+  dep_wait();
+  if (blockIdx.x == 0 && threadIdx.x < 2) maxes[threadIdx.x] = 0u;
   float mk[8], ph[8];
 #pragma unroll
   for (int m = 0; m < 8; ++m) {
@@ -303,8 +310,6 @@ __global__ void __launch_bounds__(TGT_THREADS)
     mk[m] = in ? mask[x + y * npup] : 0.f;
     ph[m] = in ? phase[x + y * npup] : 0.f;
   }
-  FftTw<N> W;
-  W.load(tw, j);
   float2 v[8];
 #pragma unroll
   for (int m = 0; m < 8; ++m) {
@@ -336,6 +341,10 @@ __global__ void __launch_bounds__(N / 8 * target_cols(N))
   __shared__ unsigned int red[2][32];
   const int c = threadIdx.x % CB, j = threadIdx.x / CB;
   const int x = blockIdx.x * CB + c;
+  FftTw<N> W;
+  dep_launch();
+  W.load(tw, j);
+  dep_wait();
   float2 v[8];
   float l[8];
 #pragma unroll
@@ -344,8 +353,6 @@ __global__ void __launch_bounds__(N / 8 * target_cols(N))
     v[m] = y < npup ? __ldcg(amp + (size_t)y * N + x) : make_float2(0.f, 0.f);
     l[m] = le[(size_t)y * N + x];
   }
-  FftTw<N> W;
-  W.load(tw, j);
   fft_regs<N, CB, BS, false>(v, W, j, sm + c, CtaSync{});
   unsigned int mse = 0, mle = 0;
 #pragma unroll
@@ -384,11 +391,11 @@ template <int N>
 static void target_image(float *se, float *le, float2 *amp, const float *phase, const float *mask, float scale,
                          int npup, float norm, int comp_le, unsigned int *maxes, const float2 *tw, cudaStream_t s) {
   constexpr int T = N / 8, SEQ = TGT_THREADS / T, CB = target_cols(N);
-  target_rows_kernel<N><<<(npup + SEQ - 1) / SEQ, TGT_THREADS, 0, s>>>(amp, phase, mask, scale, npup, tw, maxes);
+  launch_after(target_rows_kernel<N>, (npup + SEQ - 1) / SEQ, TGT_THREADS, 0, s, amp, phase, mask, scale, npup, tw, maxes);
   AOB_LAUNCH_CHECK("target_rows_kernel");
   constexpr int sm = (int)sizeof(float2) * 2 * fft_smem_elems(N) * CB;
   smem_opt_in(reinterpret_cast<const void *>(target_cols_kernel<N>), std::max(sm, 48 * 1024));
-  target_cols_kernel<N><<<N / CB, T * CB, sm, s>>>(se, le, amp, npup, norm, comp_le, tw, maxes);
+  launch_after(target_cols_kernel<N>, N / CB, T * CB, sm, s, se, le, amp, npup, norm, comp_le, tw, maxes);
   AOB_LAUNCH_CHECK("target_cols_kernel");
 }
 
@@ -669,7 +676,7 @@ void aob_dm::comp_shape(const float *dev_com, cudaStream_t s) {
   if (dev_com && dev_com != com.p)
     AOB_CUDA(cudaMemcpyAsync(com.p, dev_com, sizeof(float) * nact, cudaMemcpyDeviceToDevice, s));
   const int64_t npix = (int64_t)dim * dim;
-  dm_shape_kernel<<<(int)std::min<int64_t>((npix + 255) / 256, 8192), 256, 0, s>>>(shape.p, (int)npix, rowptr.p,
+  launch_after(dm_shape_kernel, (int)std::min<int64_t>((npix + 255) / 256, 8192), 256, 0, s, shape.p, (int)npix, rowptr.p,
                                                                                    actidx.p, weight.p, c);
   AOB_LAUNCH_CHECK("dm_shape_kernel");
 }
@@ -786,6 +793,6 @@ void aob_target::reset_le(cudaStream_t s) {
 // =================================================================== raytrace
 void aob::raytrace(float *out, int nx, int ny, const RaySources &S, bool reset, cudaStream_t s) {
   dim3 th(32, 8), gr((nx + 31) / 32, (ny + 7) / 8);
-  raytrace_kernel<<<gr, th, 0, s>>>(out, nx, ny, S, reset ? 1 : 0);
+  launch_after(raytrace_kernel, gr, th, 0, s, out, nx, ny, S, reset ? 1 : 0);
   AOB_LAUNCH_CHECK("raytrace_kernel");
 }
