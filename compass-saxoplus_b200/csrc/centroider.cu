@@ -277,6 +277,22 @@ __global__ void calib_kernel(const Tin *raw, float *cal, const float *dark, cons
     cal[t] = ((float)raw[lut[t]] - dark[t]) * flat[t];
 }
 
+__global__ void zero_img_kernel(float *img, int64_t n) {
+  dep_sync();
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x)
+    img[t] = 0.f;
+}
+
+// A camera frame from device memory (load_img): n pixels, eight per thread where both
+// buffers start on 16 bytes.
+__global__ void copy_frame_kernel(uint16_t *dst, const uint16_t *src, int64_t n, int vec) {
+  dep_sync();
+  const int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, st = (int64_t)gridDim.x * blockDim.x;
+  const int64_t nv = vec ? n / 8 : 0;
+  for (int64_t i = i0; i < nv; i += st) reinterpret_cast<uint4 *>(dst)[i] = reinterpret_cast<const uint4 *>(src)[i];
+  for (int64_t i = 8 * nv + i0; i < n; i += st) dst[i] = src[i];
+}
+
 // The same calibration on the valid pixels only, the rest of the image at zero
 // (calibrate_img_validPix, sutra_centroider.cpp:194-223): the npix x npix window of
 // every valid sub-aperture (calibration_validPix_sh_krnl, sutra_centroider.cu:68-90)
@@ -357,7 +373,9 @@ void aob_centro::calibrate(cudaStream_t s, bool valid_only) {
   const bool pixels = type == AOB_CENTRO_PYR || type == AOB_CENTRO_MASKEDPIX;
   const int nv = (int)validx.n, np = pixels ? 1 : npix;
   AOB_REQUIRE(np > 0, "calibrate_img_validPix: npix not set");
-  AOB_CUDA(cudaMemsetAsync(img.p, 0, sizeof(float) * n, s));
+  // (a kernel of the chain and not a memset, which would end it)
+  launch_after(zero_img_kernel, (int)std::min<int64_t>((n + 1023) / 1024, 4096), 256, 0, s, img.p, n);
+  AOB_LAUNCH_CHECK("zero_img_kernel");
   const int64_t work = (int64_t)nv * np * np;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((work + 255) / 256, 4096));
   if (raw_u16)
@@ -367,6 +385,16 @@ void aob_centro::calibrate(cudaStream_t s, bool valid_only) {
     launch_after(calib_valid_kernel<float>, grid, 256, 0, s, img_raw.p, img.p, dark.p, flat.p, lut.p, validx.p, validy.p, nv,
                                                    np, img_m);
   AOB_LAUNCH_CHECK("calib_valid_kernel");
+}
+
+// load_img of a frame in device memory: a kernel of the chain (a frame in place needs none)
+void aob_centro::copy_frame(const uint16_t *src, cudaStream_t s) {
+  const int64_t n = img_raw_u16.n;
+  if (src == img_raw_u16.p) return;
+  const int vec = ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(img_raw_u16.p)) & 15) == 0;
+  launch_after(copy_frame_kernel, (int)std::max<int64_t>(1, std::min<int64_t>((n / 8 + 255) / 256, 2048)), 256, 0, s,
+               img_raw_u16.p, src, n, vec);
+  AOB_LAUNCH_CHECK("copy_frame_kernel");
 }
 
 void aob_centro::get_cog(float *dev_slopes, cudaStream_t s) {
