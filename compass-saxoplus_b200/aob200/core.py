@@ -9,6 +9,7 @@ numpy arrays indexed [x, y] with x the fastest device index (Fortran order).
 from __future__ import annotations
 
 import ctypes
+import functools
 
 import numpy as np
 
@@ -234,6 +235,11 @@ class ShWfs:
     @property
     def d_phase(self):
         return self.buffer("phase", shape=(self.npup, self.npup))
+
+    @functools.cached_property
+    def phase_ptr(self) -> int:
+        """Device address of the phase (allocated once with the sensor)."""
+        return self.d_phase.ptr
 
     @property
     def d_bincube(self):
@@ -658,6 +664,11 @@ class LsController:
 
     def buffer(self, which, dtype=np.float32, shape=None):
         return _buffer("aob_ls_buffer", self.h, which, dtype, shape, self)
+
+    @functools.cached_property
+    def voltage_ptr(self) -> int:
+        """Device address of the voltages (allocated once with the controller)."""
+        return self.buffer("voltage").ptr
 
     def params(self):
         ns, na, ol, pr = ctypes.c_int(), ctypes.c_int(), ctypes.c_int(), ctypes.c_int()

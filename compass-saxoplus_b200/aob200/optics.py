@@ -8,6 +8,7 @@ SutraDm (libsutra/src.cpp/sutra_dm.cpp, sutra_dm.cu), SutraSource::raytrace
 from __future__ import annotations
 
 import ctypes
+import functools
 
 import numpy as np
 
@@ -44,6 +45,11 @@ class Dm:
     def d_shape(self):
         return self.buffer("shape", (self.dim, self.dim))
 
+    @functools.cached_property
+    def shape_ptr(self) -> int:
+        """Device address of the shape (allocated once with the DM)."""
+        return self.d_shape.ptr
+
     def set_com(self, com):
         self.buffer("com").set(com)
 
@@ -54,12 +60,18 @@ class Dm:
 def raytrace(dev_out, nx, ny, sources, reset=True, stream=None):
     """sources: list of (dev_ptr, dim, xoff, yoff); out = (0 or out) + bilinear sum."""
     n = len(sources)
-    ptrs = (ctypes.c_void_p * max(n, 1))(*[s[0] for s in sources])
-    dims = (ctypes.c_int * max(n, 1))(*[int(s[1]) for s in sources])
-    xo = (ctypes.c_float * max(n, 1))(*[float(s[2]) for s in sources])
-    yo = (ctypes.c_float * max(n, 1))(*[float(s[3]) for s in sources])
+    Ptr, Int, Flt = _ray_arrays(max(n, 1))
+    ptrs, dims, xo, yo = Ptr(), Int(), Flt(), Flt()
+    for k, (p, d, x, y) in enumerate(sources):
+        ptrs[k], dims[k], xo[k], yo[k] = p, d, x, y
     call("aob_raytrace", dev_out, int(nx), int(ny), n, ctypes.addressof(ptrs), ctypes.addressof(dims),
          ctypes.addressof(xo), ctypes.addressof(yo), 1 if reset else 0, stream)
+
+
+@functools.lru_cache(maxsize=None)
+def _ray_arrays(n):
+    """Array types of n sources (making a ctypes array type costs more than the call)."""
+    return ctypes.c_void_p * n, ctypes.c_int * n, ctypes.c_float * n
 
 
 class Target:
@@ -88,6 +100,11 @@ class Target:
     @property
     def d_phase(self):
         return self.buffer("phase", (self.npup, self.npup))
+
+    @functools.cached_property
+    def phase_ptr(self) -> int:
+        """Device address of the phase (allocated once with the target)."""
+        return self.d_phase.ptr
 
     @property
     def d_image_se(self):

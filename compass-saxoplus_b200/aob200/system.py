@@ -106,25 +106,29 @@ class ShAoSystem:
         self.iter = 0
 
     # ------------------------------------------------------------- raytracing
-    def _layer_sources(self, extra=0.0):
+    def _layers(self):
+        """The layers' current screens (they change place when the atmosphere moves)."""
+        return [self.atmos.screen(i) for i in range(len(self.layer_params))]
+
+    def _layer_sources(self, extra=0.0, layers=None):
         out = []
-        for i, lp in enumerate(self.layer_params):
-            p, dim, ax, ay = self.atmos.screen(i)
+        for p, dim, ax, ay in (self._layers() if layers is None else layers):
             off = (dim - self.n) / 2.0 + extra
             out.append((p, dim, off + ax, off + ay))
         return out
 
-    def trace_wfs(self, stream=None, with_atmos=True, with_dm=True):
-        srcs = (self._layer_sources() if with_atmos else [])
+    def trace_wfs(self, stream=None, with_atmos=True, with_dm=True, layers=None):
+        srcs = (self._layer_sources(layers=layers) if with_atmos else [])
         if with_dm:
-            srcs.append((self.dm.d_shape.ptr, self.dm.dim, self.dm_off, self.dm_off))
-        optics.raytrace(self.wfs.d_phase.ptr, self.n, self.n, srcs, reset=True, stream=stream)
+            srcs.append((self.dm.shape_ptr, self.dm.dim, self.dm_off, self.dm_off))
+        optics.raytrace(self.wfs.phase_ptr, self.n, self.n, srcs, reset=True, stream=stream)
 
-    def trace_target(self, stream=None):
-        srcs = self._layer_sources(extra=self.pupdiff)
-        srcs.append((self.dm.d_shape.ptr, self.dm.dim, self.dm_off + self.pupdiff, self.dm_off + self.pupdiff))
+    def trace_target(self, stream=None, layers=None):
+        srcs = self._layer_sources(extra=self.pupdiff, layers=layers)
+        off = self.dm_off + self.pupdiff
+        srcs.append((self.dm.shape_ptr, self.dm.dim, off, off))
         npup = self.target.npup
-        optics.raytrace(self.target.d_phase.ptr, npup, npup, srcs, reset=True, stream=stream)
+        optics.raytrace(self.target.phase_ptr, npup, npup, srcs, reset=True, stream=stream)
 
     # ------------------------------------------------------------ calibration
     def measure_slopes(self, stream=None):
@@ -204,9 +208,10 @@ class ShAoSystem:
         commands come from the learned reconstructor (aob_mlp_comp_com), with the
         LS MVM as fallback when the predicted command norm exceeds ``threshold``."""
         self.atmos.move(stream)
+        layers = self._layers()
         if compute_psf:
-            self.trace_target(stream)
-        self.trace_wfs(stream)
+            self.trace_target(stream, layers)
+        self.trace_wfs(stream, layers=layers)
         if mlp is None:
             self.loop.step(None, None, noise, stream)
         else:
@@ -214,7 +219,7 @@ class ShAoSystem:
             self.centro.get_cog(self.ls.buffer("centroids").ptr, stream)
             mlp.comp_com(self.ls, float(min(threshold, 3.0e38)), stream)
             self.ls.comp_voltage(stream)
-        self.dm.comp_shape(self.ls.buffer("voltage").ptr, stream)
+        self.dm.comp_shape(self.ls.voltage_ptr, stream)
         if compute_psf:
             self.target.comp_image(None, True, stream)
         self.iter += 1

@@ -14,6 +14,7 @@ function K_{5/6} (scipy.special.kv).
 from __future__ import annotations
 
 import ctypes
+import threading
 from dataclasses import dataclass
 
 import numpy as np
@@ -151,6 +152,7 @@ class Atmosphere:
 
     def __init__(self, layers, device=0):
         self.h = ctypes.c_void_p()
+        self._tls = threading.local()
         call("aob_atmos_create", ctypes.addressof(self.h), int(device))
         self.layers = layers
         self.device = device
@@ -186,12 +188,19 @@ class Atmosphere:
         call("aob_atmos_move", self.h, stream)
 
     def screen(self, idx):
-        p = ctypes.c_void_p()
-        dim = ctypes.c_int()
-        ax, ay = ctypes.c_float(), ctypes.c_float()
-        call("aob_atmos_screen", self.h, int(idx), ctypes.addressof(p), ctypes.addressof(dim), ctypes.addressof(ax),
-             ctypes.addressof(ay))
+        """(device pointer, size, x and y shift) of layer idx's current screen."""
+        (p, dim, ax, ay), at = self._screen_out()
+        call("aob_atmos_screen", self.h, int(idx), *at)
         return p.value, dim.value, ax.value, ay.value
+
+    def _screen_out(self):
+        # result slots of one screen() call, made once per thread (the call is on
+        # the iteration's path)
+        t = self._tls
+        if not hasattr(t, "slots"):
+            out = (ctypes.c_void_p(), ctypes.c_int(), ctypes.c_float(), ctypes.c_float())
+            t.slots = out, tuple(ctypes.addressof(o) for o in out)
+        return t.slots
 
     def screen_host(self, idx):
         p, dim, _, _ = self.screen(idx)
