@@ -216,7 +216,10 @@ struct aob_ls {
   void ensure_packed(int p);
   // use: device flag; when given and 0 the MVM is skipped (learned reconstructor path)
   void comp_com(cudaStream_t s, uint32_t *bump = nullptr, const uint32_t *use = nullptr);
-  void launch_mvm(struct aob::MvmArgs &A, cudaStream_t s);
+  bool launch_mvm(struct aob::MvmArgs &A, cudaStream_t s, bool dry = false);
+  void integrator_args(struct aob::MvmArgs &A);
+  bool comp_com_voltage(cudaStream_t s, bool dry);
+  void rotate_ring();
   void comp_voltage(cudaStream_t s);
   void clip(cudaStream_t s);
   void apply_perturb(cudaStream_t s);
@@ -246,6 +249,7 @@ struct aob_loop {
   int fused_batch = 0;                   // max sub-apertures per CTA and round in the fused kernel (0 = all)
   int last_kernels = 3;                  // kernels launched by the last device step
   uint32_t frame_host = 0;
+  bool host_step = false;                // the step under way reads or writes host buffers
   int host_io = 1;                       // 1: the fused kernel writes pinned host voltages itself
   float *io_volt = nullptr;              // device view of the caller's pinned voltages during a step
   uint32_t test_grid_polls = 0;          // wait-expiry test: grid-barrier poll limit (0 = the default)

@@ -46,6 +46,15 @@ struct MvmArgs {
   int rows_per_cta;       // bulk kernel: rows staged per CTA (host-checked to fit)
   const uint32_t *use;    // when set and *use == 0 the launch does nothing (the learned
                           // reconstructor's commands were used instead)
+  // bulk kernel, when volt is set: the voltage stage of comp_voltage in the same
+  // epilogue (delay interpolation from ring[0] and ring[1], ring[0] takes the new
+  // command, clip)
+  float *volt;
+  float *oldest;
+  const float *second;
+  float va, vb;
+  int delayed, do_clip;
+  float vmin, vmax;
 };
 
 // Dot product of one 16-byte packed chunk with its slopes sv[STRIDE * q],
@@ -222,9 +231,13 @@ __global__ void __launch_bounds__(MVM_THREADS) ls_mvm_bulk_kernel(MvmArgs A) {
   dep_wait();  // (the rows, which no kernel writes, are on their way while the slopes' producer ends)
   if (A.bump && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(A.bump, 1u);
   // epilogue inputs of this thread's row (R <= blockDim), fetched now
-  float e_sc = 1.f, e_mg = 1.f, e_cm = 0.f;
+  float e_sc = 1.f, e_mg = 1.f, e_cm = 0.f, e_o0 = 0.f, e_o1 = 0.f;
   if ((int)threadIdx.x < R) {
     const int gr = r0 + threadIdx.x;
+    if (A.volt && A.delayed) {
+      e_o0 = __ldcg(A.oldest + gr);
+      e_o1 = __ldcg(A.second + gr);
+    }
     if (A.rscale) e_sc = __ldg(A.rscale + gr);
     if (A.integrate) {
       if (A.mgain) e_mg = __ldg(A.mgain + gr);
@@ -284,7 +297,19 @@ __global__ void __launch_bounds__(MVM_THREADS) ls_mvm_bulk_kernel(MvmArgs A) {
     if (A.rscale) tot *= e_sc;
     const float e = -tot;
     A.err[gr] = e;
-    if (A.integrate) A.com[gr] = fmaf(A.gain, e * e_mg, A.berta * e_cm);
+    if (A.integrate) {
+      const float c = fmaf(A.gain, e * e_mg, A.berta * e_cm);
+      A.com[gr] = c;
+      if (A.volt) {
+        float v = c;
+        if (A.delayed) {
+          v = A.va * e_o0 + A.vb * e_o1;
+          A.oldest[gr] = c;
+        }
+        if (A.do_clip) v = fminf(fmaxf(v, A.vmin), A.vmax);
+        A.volt[gr] = v;
+      }
+    }
   }
   // no CTA may exit with a copy still landing in its shared memory
   if (!rows_ok && threadIdx.x == 0)
@@ -482,8 +507,16 @@ void aob_ls::comp_com(cudaStream_t s, uint32_t *bump, const uint32_t *use) {
     generic_comp_com(s, bump);
     return;
   }
-  ensure_packed(prec);
   MvmArgs A{};
+  integrator_args(A);
+  A.bump = bump;
+  A.use = use;
+  launch_mvm(A, s);
+}
+
+// The LS integrator's MVM: err = -cmat s, com += gain err modal gains.
+void aob_ls::integrator_args(MvmArgs &A) {
+  ensure_packed(prec);
   A.nrow = nactu;
   A.ncol = nslope;
   A.s = centroids.p;
@@ -493,9 +526,7 @@ void aob_ls::comp_com(cudaStream_t s, uint32_t *bump, const uint32_t *use) {
   A.gain = gain;
   A.berta = 1.f;
   A.integrate = 1;
-  A.bump = bump;
   A.status = status.p;
-  A.use = use;
   if (prec == AOB_PREC_F32) {
     A.mat = cm_f32.p;
     A.ld = (nslope + 3) / 4 * 4;
@@ -507,7 +538,34 @@ void aob_ls::comp_com(cudaStream_t s, uint32_t *bump, const uint32_t *use) {
     A.rscale = row_scale.p;
     A.ld = (nslope + 15) / 16 * 16;
   }
-  launch_mvm(A, s);
+}
+
+// comp_com and comp_voltage in one launch of the bulk-copy MVM.  False, and nothing
+// done, where that does not apply: other controllers, open loop, perturbations, rows
+// that do not fit in shared memory, and delays between 0 and 1 frame, whose voltage
+// interpolates with the command that the same launch is forming.
+// ``dry``: only say whether it applies.
+bool aob_ls::comp_com_voltage(cudaStream_t s, bool dry) {
+  if (kind != AOB_CTRL_LS || open_loop || (delay > 0.f && delay < 1.f)) return false;
+  for (auto &kv : perturb)
+    if (kv.second.on) return false;
+  AOB_CUDA(cudaSetDevice(device));
+  MvmArgs A{};
+  integrator_args(A);
+  A.volt = com_clipped.p;
+  A.delayed = delay > 0 ? 1 : 0;
+  if (A.delayed) {
+    A.oldest = ring[0].p;
+    A.second = ring[1].p;
+  }
+  A.va = a;
+  A.vb = b;
+  A.vmin = volt_min;
+  A.vmax = volt_max;
+  A.do_clip = volt_min < volt_max ? 1 : 0;
+  if (!launch_mvm(A, s, dry)) return false;
+  if (A.delayed && !dry) rotate_ring();
+  return true;
 }
 
 namespace {
@@ -537,7 +595,9 @@ constexpr size_t MVM_SMEM_MAX = 227 * 1024;
 // Kernel and grid for this matrix: the bulk-copy kernel when a CTA's rows fit in
 // shared memory with one CTA per SM, the register-streaming kernel otherwise
 // (or when the caller forces it).  ``nblocks`` > 0 overrides the grid size.
-void aob_ls::launch_mvm(MvmArgs &A, cudaStream_t s) {
+// A voltage stage (A.volt) needs the bulk-copy kernel: false, without a launch, where
+// it does not fit.
+bool aob_ls::launch_mvm(MvmArgs &A, cudaStream_t s, bool dry) {
   const int nsm = num_sms(device);
   int esize = prec == AOB_PREC_F32 ? 4 : (prec == AOB_PREC_BF16 ? 2 : 1);
   int V = 16 / esize;
@@ -548,12 +608,15 @@ void aob_ls::launch_mvm(MvmArgs &A, cudaStream_t s) {
   const size_t need = mvm_bars_bytes(rpc) + slope_bytes + (size_t)rpc * A.ld * esize +
                       sizeof(float) * (MVM_THREADS / 32) * rpc;
   const bool bulk = (mvm_kind == 0 || mvm_kind == 1) && need <= MVM_SMEM_MAX && mvm_kind != 2 && rpc <= MVM_THREADS;
+  if (A.volt && !bulk) return false;
+  if (dry) return true;
   if (prec == AOB_PREC_F32)
     launch_mvm_t<float>(A, grid, bulk, s);
   else if (prec == AOB_PREC_BF16)
     launch_mvm_t<__nv_bfloat16>(A, grid, bulk, s);
   else
     launch_mvm_t<__nv_fp8_e4m3>(A, grid, bulk, s);
+  return true;
 }
 
 // The command laws of SutraControllerGeneric::comp_com
@@ -685,12 +748,14 @@ void aob_ls::comp_voltage(cudaStream_t s) {
   A.n = nactu;
   launch_after(voltage_kernel, std::max(1, std::min((nactu + 255) / 256, 1024)), 256, 0, s, A);
   AOB_LAUNCH_CHECK("voltage_kernel");
-  if (A.delayed) {
-    // the oldest buffer now holds a copy of the current command and becomes it
-    aob::DevBuf<float> t = std::move(ring.front());
-    ring.pop_front();
-    ring.push_back(std::move(t));
-  }
+  if (A.delayed) rotate_ring();
+}
+
+// The oldest buffer now holds a copy of the current command and becomes it.
+void aob_ls::rotate_ring() {
+  aob::DevBuf<float> t = std::move(ring.front());
+  ring.pop_front();
+  ring.push_back(std::move(t));
 }
 
 // SutraController::add_perturb (sutra_controller.cpp:266-285): every enabled

@@ -133,6 +133,18 @@ void aob_loop::device_step(bool noise, cudaStream_t s, bool frame_on_device) {
     // the fused kernel's grid barrier is a 64-bit arrival counter that every
     // launch raises by exactly its grid size, so it needs no re-arming
     if (launch_fused(noise, s, frame_on_device, true)) {
+      // The sensor kernel, then commands and voltages, each started while the one
+      // before it ends, where nothing but kernels follows one another: a cooperative
+      // launch cannot overlap its predecessor's end (3.1 us from one kernel's end to
+      // the next one's start, 0.9 us this way) and pays a grid barrier besides.
+      // A step whose host reads or writes it has copies in between, and its
+      // voltages come out sooner from one kernel.
+      if (mode == 0 && fused_batch == 0 && !host_step && !frame_on_device && ls->comp_com_voltage(s, true)) {
+        wfs->comp_image_to(noise, s, ls->centroids.p, nullptr);
+        ls->comp_com_voltage(s, false);
+        last_kernels = 2;
+        return;
+      }
       if (launch_fused(noise, s, frame_on_device, false)) {
         last_kernels = 1;
         return;
@@ -311,6 +323,7 @@ void aob_loop::step(const float *host_phase, float *host_voltage, bool noise, cu
   io_volt = (host_io == 1 && host_voltage && mode != 1)
                 ? static_cast<float *>(const_cast<void *>(mapped_view(host_voltage)))
                 : nullptr;
+  host_step = host_phase || host_voltage;
   struct Reset {
     float *&p;
     ~Reset() { p = nullptr; }
