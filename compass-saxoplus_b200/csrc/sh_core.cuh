@@ -23,6 +23,8 @@
 // bit-identical images and slopes.
 #pragma once
 
+#include <type_traits>
+
 #include "aob_common.cuh"
 
 namespace aob {
@@ -231,11 +233,14 @@ __device__ __forceinline__ void sh_store_images(const ShKernelArgs &P, int base,
 // thread of the team once the field stage is complete (its global loads have
 // returned), before the DFTs.  With DEFER_IMG the cube and image writes are
 // left to sh_store_images (the noisy pixels stay in the work area).
+// ``before_phase`` runs on every thread once it has requested what no kernel writes
+// (windows, pupil, offsets, metadata) and before it reads the phase.
 template <int NFFT, int PD, int TK = TEAM_CTA, class Hook = NoHook, bool DEFER_IMG = false, bool FS = false,
-          class Src = ShStrided>
+          class Src = ShStrided, class Pre = NoHook>
 __device__ __forceinline__ void sh_batch(const ShKernelArgs &P, int base, int stride, int S,
                                          const unsigned char *tables, unsigned char *work, const ShSmem &L,
-                                         const Team &T, const Hook &after_field = Hook{}, const Src &src = Src{}) {
+                                         const Team &T, const Hook &after_field = Hook{}, const Src &src = Src{},
+                                         const Pre &before_phase = Pre{}) {
   auto sub = [&](int s) {
     if constexpr (Src::LISTED)
       return src.sub(s);
@@ -269,7 +274,9 @@ __device__ __forceinline__ void sh_batch(const ShKernelArgs &P, int base, int st
 
   // ---- 0. metadata of the batch (one global round trip for all of it:
   //      global-space loads, free to overtake the shared stores) ----
-  const uint32_t frame = P.frame_ptr ? __ldcg(P.frame_ptr) : P.frame;
+  constexpr bool WAITS = !std::is_same<Pre, NoHook>::value;
+  uint32_t frame = 0;
+  if constexpr (!WAITS) frame = P.frame_ptr ? __ldcg(P.frame_ptr) : P.frame;
   // (threads with no field element take the metadata when there are such:
   // the shared stores wait for their loads, which would otherwise hold back a
   // field thread's own loads by a round trip)
@@ -297,6 +304,7 @@ __device__ __forceinline__ void sh_batch(const ShKernelArgs &P, int base, int st
 
   // ---- 1. complex field: loads of up to 4 elements issued before any use ----
   if constexpr (FS) {
+    before_phase();
     // field stop: the sub-aperture's window of the filtered full-pupil field times
     // exp(-i offset), normalised (camplipup_krnl, libsutra/src.cu/sutra_wfs.cu:87-117)
     for (int i0 = tid; i0 < nE; i0 += 4 * nt) {
@@ -328,6 +336,7 @@ __device__ __forceinline__ void sh_batch(const ShKernelArgs &P, int base, int st
   } else
   for (int i0 = tid; i0 < nE; i0 += 4 * nt) {
     float ph[4], am[4], of[4];
+    int id[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int i = i0 + j * nt;
@@ -338,14 +347,20 @@ __device__ __forceinline__ void sh_batch(const ShKernelArgs &P, int base, int st
         const int x = l - y * pd;
         const int k = sub(s);
         const int X = x + __ldg(P.puppixx + k), Y = y + __ldg(P.puppixy + k);
-        const int id = X + Y * P.npup;
+        id[j] = X + Y * P.npup;
         if constexpr (Src::LISTED)
           ph[j] = src.phase(s, X, Y);
-        else
-          ph[j] = __ldcg(P.phase + id);  // (L2: a resident kernel reads a new phase every step)
-        am[j] = __ldg(P.pupil + id);
+        else if constexpr (!WAITS)
+          ph[j] = __ldcg(P.phase + id[j]);  // (L2: a resident kernel reads a new phase every step)
+        am[j] = __ldg(P.pupil + id[j]);
         of[j] = __ldg(P.offsets + l);
       }
+    }
+    if constexpr (WAITS) {
+      before_phase();
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (i0 + j * nt < nE) ph[j] = __ldcg(P.phase + id[j]);
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -356,6 +371,10 @@ __device__ __forceinline__ void sh_batch(const ShKernelArgs &P, int base, int st
         E[i] = make_float2(cs * am[j], sn * am[j]);
       }
     }
+  }
+  if constexpr (WAITS) {
+    if (tid >= nE) before_phase();  // (threads without a sample)
+    frame = P.frame_ptr ? __ldcg(P.frame_ptr) : P.frame;
   }
   team_sync<TK>(T);
   after_field();

@@ -51,13 +51,18 @@ __global__ void __launch_bounds__(SH_THREADS) sh_image_kernel(ShKernelArgs P, in
   const ShSmem L(NFFT, P.nu, P.nv, pd, P.nrebin2 * P.npix * P.npix, P.npix * P.npix, S);
   dep_launch();
   sh_load_tables<NFFT>(P, smem, threadIdx.x, blockDim.x);
-  dep_wait();
   // (the barrier closing sh_batch's stage 1 publishes the tables: stages 0-1
-  // read none of them, so their loads overlap the field's)
+  // read none of them, so their loads overlap the field's.  The wait for the kernel
+  // before this one stands right before the phase is read: all that is behind it is
+  // one round trip to L2)
+  struct Wait {
+    __device__ void operator()() const { dep_wait(); }
+  };
   for (int base = blockIdx.x; base < P.nvalid; base += S * gridDim.x) {
     const int Sb = min(S, (P.nvalid - base + (int)gridDim.x - 1) / (int)gridDim.x);
-    sh_batch<NFFT, PD, TEAM_CTA, NoHook, false, FS>(P, base, gridDim.x, Sb, smem, smem + L.hdr, L,
-                                                    Team{(int)threadIdx.x, (int)blockDim.x, 0});
+    sh_batch<NFFT, PD, TEAM_CTA, NoHook, false, FS, ShStrided, Wait>(P, base, gridDim.x, Sb, smem, smem + L.hdr, L,
+                                                                     Team{(int)threadIdx.x, (int)blockDim.x, 0},
+                                                                     NoHook{}, ShStrided{}, Wait{});
   }
 }
 
