@@ -41,7 +41,12 @@
 namespace aob {
 
 constexpr int PYR_MAX_REBIN = 8;
-constexpr int PYR_THREADS = 512;      // accum: threads per CTA, at most
+constexpr int PYR_THREADS = 512;      // binning: threads per CTA, at most
+// accum: threads per CTA, at most -- two CTAs of 256 on an SM overlap one's last steps
+// (the sum over its groups and one group's transform) with the other's planes: 83.1 us
+// for the 512 x 512 image, its slopes and commands, 89.2 with CTAs of 512, 82.7 with
+// 128, which nfft 2048 (256 threads a sequence) does not allow
+constexpr int PYR_ACC_THREADS = 256;
 constexpr int PYR_ROW_THREADS = 256;
 
 struct PyrArgs {
@@ -108,14 +113,16 @@ __global__ void __launch_bounds__(PYR_ROW_THREADS) pyr_rows_kernel(PyrArgs A) {
 // columns per CTA: 8 (64-byte segments), fewer where 8 would pass 512 threads
 constexpr int pyr_cols(int n) { return n <= 512 ? 8 : 4096 / n; }
 
-// 2. per group of columns of the modulation planes blockIdx.y, blockIdx.y +
-//    gridDim.y, ...: inverse transform along y (rows outside the pupil are
-//    zero), x field stop, x pyramid phase mask (submask_krnl,
-//    submaskpyr_krnl), forward transform along y.  In place in work[p].
+// 2. per unit -- a group of columns of one modulation plane: inverse transform
+//    along y (rows outside the pupil are zero), x field stop, x pyramid phase mask
+//    (submask_krnl, submaskpyr_krnl), forward transform along y.  In place in
+//    work[p].  A CTA takes an equal run of units, a column group's planes one after
+//    the other, so that it loads the mask once per group and no SM waits for a
+//    last wave (1536 units at nfft 512 and 24 points: 11 on the fullest of 148 SMs).
 //    Bound: instruction issue (about 300 per thread and transform) with one
-//    512-thread CTA per SM at these registers; the next plane's loads go out
+//    512-thread CTA per SM at these registers; the next unit's loads go out
 //    before the current one's transforms.  The whole image and its slopes at nfft
-//    512, 24 points, with a 1600-actuator command matrix: 112 us per pass, 181 us
+//    512, 24 points, with a 1600-actuator command matrix: 83 us per pass, 181 us
 //    when every radix-8 pass went through shared memory and every point was
 //    read and written with bank conflicts.
 template <int N, bool FOCAL>
@@ -123,37 +130,50 @@ __global__ void __launch_bounds__(N / 8 * pyr_cols(N)) pyr_cols_kernel(PyrArgs A
   extern __shared__ float2 sm[];
   constexpr int T = N / 8, CB = pyr_cols(N), BS = fft_smem_elems(N) * CB;
   const int c = threadIdx.x % CB, j = threadIdx.x / CB;
-  const int x = blockIdx.x * CB + c;
   float2 *s = sm + c;
   FftTw<N> W;
   dep_launch();
   W.load(A.tw, j);
+  const int64_t units = (int64_t)(N / CB) * A.npts;  // unit = group * npts + point
+  int u = (int)(blockIdx.x * units / gridDim.x);
+  const int u1 = (int)((blockIdx.x + 1) * units / gridDim.x);
   float2 mask[8];
+  auto load_mask = [&](int x) {
 #pragma unroll
-  for (int m = 0; m < 8; ++m) {
-    const size_t g = x + (size_t)(j + T * m) * N;
-    const float msk = A.submask[g];
-    mask[m] = A.phalfxy[g];
-    if (!FOCAL) mask[m] = make_float2(mask[m].x * msk, mask[m].y * msk);
-  }
-  auto load = [&](float2(&v)[8], int p) {
-    const float2 *base = A.work + (size_t)p * N * N + x;
+    for (int m = 0; m < 8; ++m) {
+      const size_t g = x + (size_t)(j + T * m) * N;
+      const float msk = A.submask[g];
+      mask[m] = A.phalfxy[g];
+      if (!FOCAL) mask[m] = make_float2(mask[m].x * msk, mask[m].y * msk);
+    }
+  };
+  auto load = [&](float2(&v)[8], int unit) {
+    const int g = unit / A.npts;
+    const float2 *base = A.work + (size_t)(unit - g * A.npts) * N * N + g * CB + c;
 #pragma unroll
     for (int m = 0; m < 8; ++m) {
       const int yb = j + T * m - A.off;
       v[m] = (yb >= 0 && yb < A.ntot) ? __ldcg(base + (size_t)yb * N) : make_float2(0.f, 0.f);
     }
   };
+  int group = u / A.npts;
+  load_mask(group * CB + c);
+  dep_wait();
   // rows [0, ntot) hold the input and are overwritten by the output: every
   // thread of the column has its input in registers by the first barrier
   float2 nxt[8];
-  dep_wait();
-  load(nxt, blockIdx.y);
-  for (int p = blockIdx.y; p < A.npts; p += gridDim.y) {
+  load(nxt, u);
+  for (; u < u1; ++u) {
+    const int g0 = u / A.npts, p = u - g0 * A.npts;
+    if (g0 != group) {
+      group = g0;
+      load_mask(group * CB + c);
+    }
+    const int x = group * CB + c;
     float2 v[8];
 #pragma unroll
     for (int m = 0; m < 8; ++m) v[m] = nxt[m];
-    if (p + (int)gridDim.y < A.npts) load(nxt, p + gridDim.y);
+    if (u + 1 < u1) load(nxt, u + 1);
     fft_regs<N, CB, BS, true>(v, W, j, s, CtaSync{});
     if (fft_odd_exchanges(N)) __syncthreads();
 #pragma unroll
@@ -180,7 +200,7 @@ __global__ void __launch_bounds__(N / 8 * pyr_cols(N)) pyr_cols_kernel(PyrArgs A
 //    CTA sums points g, g + G, ..., the groups are added in order -- then the
 //    pixel transfer function's inverse transform along x of that row.
 template <int N>
-__global__ void __launch_bounds__(PYR_THREADS) pyr_accum_kernel(PyrArgs A) {
+__global__ void __launch_bounds__(PYR_ACC_THREADS) pyr_accum_kernel(PyrArgs A) {
   extern __shared__ float2 sm[];
   constexpr int T = N / 8, BS = fft_smem_elems(N);
   const int g = threadIdx.x / T, j = threadIdx.x % T, G = blockDim.x / T;
@@ -374,26 +394,15 @@ static void pyr_launch(const PyrArgs &A, int device, cudaStream_t s) {
     const size_t sm = sizeof(float2) * 2 * BS * CB;
     auto kern = A.focal_work ? pyr_cols_kernel<N, true> : pyr_cols_kernel<N, false>;
     pyr_smem(kern, sm);
-    // the points are split over as many CTAs per column group as give the
-    // shortest longest queue: points per CTA x waves (+ half a point of set-up)
     const int slots = nsm * std::max(1, 512 / threads);
-    int split = 1;
-    double best = 1e30;
-    for (int ps = 1; ps <= A.npts; ++ps) {
-      const int per = (A.npts + ps - 1) / ps;
-      const double cost = (double)((groups * ps + slots - 1) / slots) * (per + 0.5);
-      if (cost < best) {
-        best = cost;
-        split = ps;
-      }
-    }
-    launch_after(kern, dim3(groups, split), threads, sm, s, A);
+    const int grid = (int)std::min<int64_t>(slots, (int64_t)groups * A.npts);
+    launch_after(kern, grid, threads, sm, s, A);
     AOB_LAUNCH_CHECK("pyr_cols_kernel");
   }
   {
-    // groups of threads per row: one per point, in whole warps, up to PYR_THREADS
+    // groups of threads per row: one per point, in whole warps, up to PYR_ACC_THREADS
     const int unit = T < 32 ? 32 / T : 1;
-    const int G = std::min(PYR_THREADS / T, (A.npts + unit - 1) / unit * unit);
+    const int G = std::min(PYR_ACC_THREADS / T, (A.npts + unit - 1) / unit * unit);
     const size_t sm = std::max(sizeof(float2) * 2 * BS * G, sizeof(float) * N * G);
     pyr_smem(pyr_accum_kernel<N>, sm);
     launch_after(pyr_accum_kernel<N>, N, G * T, sm, s, A);
