@@ -305,20 +305,23 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
   if (warp == 0) {
     if (lane == 0) {
       // ---- TMA producer ----
-      int it = 0;
+      // (stage and phase run along: one thread's instructions are on the path of
+      // every stage -- with a division by a run-time stage count they cost 0.2 us)
+      int it = 0, s = 0;
+      uint32_t phase = 1;  // parity of the hand-back before this use of the ring
+      const uint32_t lead = cluster_addr(smem_addr(full), 0);
       for (int t = pair; ok && t < T.ntiles; t += npairs) {
         const TcTile X(T, t);
         const bool a_mn = T.prob[X.i].a_mn, b_mn = T.prob[X.i].b_mn;
         const int m0 = X.mt * TC_BM + (int)rank * TC_ROWS, n0 = X.nt * bn + (int)rank * bh;
         for (int kt = 0; kt < X.nk; ++kt, ++it) {
-          const int s = it % TC_STAGES;
-          if (it >= TC_STAGES && !mbar_wait(&empty[s], (uint32_t)(it / TC_STAGES - 1) & 1u, TC_MAX_POLLS)) {
+          if (it >= TC_STAGES && !mbar_wait(&empty[s], phase, TC_MAX_POLLS)) {
             ok = false;
             break;
           }
           unsigned char *sa = sm + s * TC_STAGE_BYTES, *sb = sa + TC_TILE_BYTES;
           if (rank == 0) mbar_expect_tx(&full[s], 2u * (uint32_t)(TC_TILE_BYTES + bh * TC_BK * 2));
-          const uint32_t bar = cluster_addr(smem_addr(&full[s]), 0);
+          const uint32_t bar = lead + 8u * (uint32_t)s;
           const bool second = kt >= X.nk1;
           const CUtensorMap *ma = &maps.m[second ? 2 : 2 * X.i], *mb = ma + 1;
           const int k0 = (second ? kt - X.nk1 : kt) * TC_BK;
@@ -333,6 +336,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
           } else {
             tma_load_2d(sb, mb, k0, n0, bar);
           }
+          if (++s == TC_STAGES) {
+            s = 0;
+            phase ^= 1u;
+          }
         }
       }
       // the last stages' hand-backs have arrived before the CTA may end
@@ -343,7 +350,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
   } else if (warp == 1) {
     if (lane == 0 && rank == 0) {
       // ---- MMA issuer ----
-      int it = 0, n = 0;
+      int n = 0, s = 0;
+      uint32_t phase = 0;
       for (int t = pair; ok && t < T.ntiles; t += npairs, ++n) {
         const TcTile X(T, t);
         const int a_mn = T.prob[X.i].a_mn, b_mn = T.prob[X.i].b_mn;
@@ -359,9 +367,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
           break;
         }
         tc_fence_after();
-        for (int kt = 0; kt < X.nk; ++kt, ++it) {
-          const int s = it % TC_STAGES;
-          if (!mbar_wait(&full[s], (uint32_t)(it / TC_STAGES) & 1u, TC_MAX_POLLS)) {
+        for (int kt = 0; kt < X.nk; ++kt) {
+          if (!mbar_wait(&full[s], phase, TC_MAX_POLLS)) {
             ok = false;
             break;
           }
@@ -371,6 +378,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
           for (int k = 0; k < TC_BK / 16; ++k)
             umma_bf16(acc, da0 + off + k * ka, db0 + off + k * kb, idesc, (kt > 0 || k > 0) ? 1u : 0u);
           umma_commit_pair(&empty[s]);
+          if (++s == TC_STAGES) {
+            s = 0;
+            phase ^= 1u;
+          }
         }
         if (ok) umma_commit_pair(&accfull[n & 1]);
       }
