@@ -714,6 +714,7 @@ def main():
     loop.use_graph(False)
     t_step = graph_time(torch, flush, lambda sp: loop.step(None, None, True, sp))
     fused = loop.kernels_per_step() == 1
+    pair = loop.kernels_per_step() == 2
     t_wfs = graph_time(torch, flush, lambda sp: wfs.comp_image(True, sp))
     t_mvm = graph_time(torch, flush, lambda sp: ls.comp_com(sp))
     loop.use_graph(not args.no_graph)
@@ -729,6 +730,9 @@ def main():
     peak, peak_kind = _peaks()
     if fused:
         dom, dbytes, dt, prof = "rtc_fused_kernel", mvm_bytes + wfs_bytes, t_step, f"rtc_fused_saxo40_{args.precision}"
+    elif pair:
+        dom, dbytes, dt = "sh_image_kernel + ls_mvm_bulk_kernel", mvm_bytes + wfs_bytes, t_step
+        prof = f"rtc_pair_saxo40_{args.precision}"
     elif t_mvm >= t_wfs:
         dom, dbytes, dt, prof = "ls_mvm_bulk_kernel", mvm_bytes, t_mvm, f"ls_mvm_saxo40_{args.precision}"
     else:

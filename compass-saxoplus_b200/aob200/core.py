@@ -704,7 +704,8 @@ class Loop:
         call("aob_loop_use_graph", self.h, 1 if on else 0)
 
     def set_mode(self, mode=0, fused_batch=0):
-        """0: fused cooperative kernel when it fits, 1: three kernels, 2: fused only.
+        """0: when the configuration fits the fused cooperative kernel, that kernel for steps with
+        host buffers and two overlapping kernels for steps without; 1: three kernels, 2: fused only.
 
         fused_batch: at most this many sub-apertures per CTA and round in the fused
         kernel (0 = a CTA's whole share at once); results are unchanged."""

@@ -140,7 +140,7 @@ class ShAoSystem:
 
     def interaction_matrix(self, push=None, chunk=0):
         """Push-pull interaction matrix of the DM seen by the sensor, every actuator
-        poked in one batch (aob_imat_build: four launches per chunk of actuators)."""
+        poked in one batch (aob_imat_build)."""
         push = self.cfg.push4imat if push is None else push
         self.centro.attach(self.wfs)
         imat = np.zeros((self.ls.nslope, self.nactu), dtype=np.float32)

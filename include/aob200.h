@@ -540,8 +540,8 @@ int aob_target_buffer(aob_target *t, const char *which, void **dev_ptr, int64_t 
  * The per-iteration RTC sequence that CompassSupervisor.next() drives
  * through separate calls (shesha/shesha/supervisor/compassSupervisor.py:
  * 175-289: compute_wfs_image -> do_centroids -> do_control -> apply_control
- * with comp_voltage), bound into one object so that it runs as three kernels
- * (SH image + fused centroids, MVM + integrator, voltage) with the slopes
+ * with comp_voltage), bound into one object so that it runs as one to three
+ * kernels (SH image + fused centroids, MVM + integrator, voltage) with the slopes
  * written straight into the controller's input. */
 typedef struct aob_loop aob_loop;
 int aob_loop_create(aob_loop **out, aob_sh *wfs, aob_centro *centro, aob_ls *ls);
@@ -630,9 +630,10 @@ int aob_loop_time(aob_loop *l, int noise, int warmup, int iters, float *ms_per_s
 int aob_loop_use_graph(aob_loop *l, int enable);
 /* Kernels launched by the device part of the last step. */
 int aob_loop_kernels_per_step(aob_loop *l, int *n);
-/* mode 0 = fused single cooperative kernel when the configuration fits
- * (otherwise three kernels), 1 = always three kernels, 2 = fused only (error
- * if it does not fit); fused_batch = at most this many sub-apertures per CTA
+/* mode 0 = when the configuration fits the fused cooperative kernel, that kernel
+ * for steps with host buffers and two overlapping kernels (image, then commands
+ * and voltages) for steps without (otherwise three kernels), 1 = always three
+ * kernels, 2 = fused only (error if it does not fit); fused_batch = at most this many sub-apertures per CTA
  * and round in the fused kernel (0 = a CTA's whole share in one round). */
 int aob_loop_set_mode(aob_loop *l, int mode, int fused_batch);
 /* Voltage output of aob_loop_step: mode 1 (default) = when host_voltage is
