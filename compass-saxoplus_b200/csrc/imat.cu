@@ -130,10 +130,16 @@ __global__ void __launch_bounds__(IMAT_THREADS) imat_kernel(ShKernelArgs P, Imat
   float *col = A.imat + (int64_t)a * 2 * nvalid;
   if (threadIdx.x == 0) s_n = 0;
   __syncthreads();
+  // s_n only hands out places in the list; how many there are, each thread counts for
+  // itself from the barrier's sum, so that every thread comes to the same decision
+  // whatever the other warps have gone on to append.
+  int n = 0;
   for (int base = 0; base < nvalid; base += IMAT_THREADS) {
     const int k = base + (int)threadIdx.x;
+    bool reached = false;
     if (k < nvalid) {
-      if (src.reaches(__ldg(P.puppixx + k), __ldg(P.puppixy + k), pd)) {
+      reached = src.reaches(__ldg(P.puppixx + k), __ldg(P.puppixy + k), pd);
+      if (reached) {
         list[atomicAdd(&s_n, 1)] = k;  // (the order within the list does not matter to any value)
       } else {
         const int ix = P.c_order ? 2 * k : k, iy = P.c_order ? 2 * k + 1 : k + nvalid;
@@ -142,8 +148,7 @@ __global__ void __launch_bounds__(IMAT_THREADS) imat_kernel(ShKernelArgs P, Imat
         col[iy] = (fy - fy) / (2.f * A.push);
       }
     }
-    __syncthreads();
-    const int n = s_n;
+    n += __syncthreads_count(reached);
     if (n + IMAT_THREADS > IMAT_LIST || base + IMAT_THREADS >= nvalid) {
       imat_images<NFFT, PD>(P, src, 2 * n, S, smem, L);
       for (int j = threadIdx.x; j < n; j += IMAT_THREADS) {
@@ -152,6 +157,7 @@ __global__ void __launch_bounds__(IMAT_THREADS) imat_kernel(ShKernelArgs P, Imat
         col[P.c_order ? 2 * m : m] = (sp.x - sm.x) / (2.f * A.push);
         col[P.c_order ? 2 * m + 1 : m + nvalid] = (sp.y - sm.y) / (2.f * A.push);
       }
+      n = 0;
       if (threadIdx.x == 0) s_n = 0;
       __syncthreads();
     }

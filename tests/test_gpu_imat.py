@@ -65,3 +65,40 @@ def test_imat_equals_pokes(nxsub, pd, isz, off, order, ref):
         got = np.array(imat).reshape(nslope, nact, order="F")
         np.testing.assert_array_equal(got, _poked(core, optics, w, c, dm, off, push, nact, nslope, out))
     assert np.isfinite(got).all() == np.isfinite(ref)
+
+
+@pytest.mark.parametrize("nxsub,isz", [
+    (19, 200),   # nvalid just above one round of 256 candidates, all reached
+    (24, 78),    # more than 256 reached, fewer than the list's 512
+    (40, 300),   # every one of about 1250
+])
+def test_pokes_that_reach_many(nxsub, isz):
+    """A CTA lists its actuator's sub-apertures 256 candidates at a time and forms the
+    listed ones when 512 places could run out.  With a whole round reached (tip-tilt and
+    modal influence functions) the count stands at the limit, where every thread has to
+    take the same branch: each of several calls equals the pokes bit for bit."""
+    from aob200 import _lib, core, optics
+    from aob200 import geometry as G
+
+    pd = 4
+    g = G.sh_geometry(G.ShParams(nxsub=nxsub, npix=6, pixsize=0.36, wavelength_um=0.7), nxsub * pd)
+    w = core.ShWfs.from_geometry(g)
+    c = core.Centroider(g.nvalid, g.npix / 2 - 0.5, g.pixsize, "cog")
+    c.set_npix(g.npix)
+    c.load_validpos(g.validsubsx, g.validsubsy)
+    c.attach(w)
+    assert g.nvalid > 256
+    dim, nact, off = g.tel.n + 13, 5, 6.0
+    x, y = (np.arange(isz) - isz / 2)[:, None], (np.arange(isz) - isz / 2)[None, :]
+    modes = np.stack([x + 0 * y, y + 0 * x, x * y / isz, (x * x + y * y) / isz, (x * x - y * y) / isz], -1)
+    at = np.full(nact, dim // 2 - isz // 2, np.int32)
+    dm = optics.Dm(dim, (modes / isz).astype(np.float32), at, at)
+    nslope, push = 2 * g.nvalid, 0.05
+    out = core.OwnedDeviceArray(nslope)
+    want = _poked(core, optics, w, c, dm, off, push, nact, nslope, out)
+    assert (want != 0).any(axis=1).sum() > 2 * 256 - 16
+    imat = core.OwnedDeviceArray(nslope * nact)
+    for _ in range(8):
+        imat.set(np.full(nslope * nact, 7.0, np.float32))
+        _lib.call("aob_imat_build", w.h, c.h, dm.h, off, off, push, 0, imat.ptr, None)
+        np.testing.assert_array_equal(np.array(imat).reshape(nslope, nact, order="F"), want)
