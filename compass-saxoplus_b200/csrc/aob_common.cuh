@@ -52,16 +52,18 @@ inline void smem_opt_in(const void *fn, int bytes) {
 // Programmatic dependent launch.  The step of a controller is a chain of kernels of
 // a few microseconds each; started one after the other's end, every link costs
 // 1.5 - 2 us of launch latency (image, slopes, commands and voltages of a 40 x 40
-// sensor as four calls: 26.2 us a pass, 17.3 us started this way; a 512 x 512 pyramid
-// with its command matrix, nine kernels: 111.6 and 88.4 us).  A kernel started by launch_after may become
-// resident while the kernel before it on the stream still runs, once all of that
-// one's CTAs have said so (dep_launch, at their start) or ended, and waits in
-// dep_wait until it has completed and its writes are visible.  Every such
-// kernel calls dep_wait in every CTA before it reads anything another kernel
-// may write and before it writes anything; ahead of it are only index arithmetic,
-// barrier set-up and reads of tables and matrices that no kernel writes.  So a
-// kernel that completes has seen all its predecessors complete, and launches of
-// any other kind (copies, events, other libraries' kernels) order as always.
+// sensor as four calls: 24.7 us a pass, 17.3 us started this way; a 512 x 512 pyramid
+// with its command matrix, nine kernels: 111.6 and 88.4 us).  A kernel started by
+// launch_after may become resident while the kernel before it on the stream still runs,
+// once all of that one's CTAs have said so (dep_launch, at their start) or ended, and
+// waits in dep_wait until it has completed and its writes are visible.  Every such
+// kernel calls dep_wait in every CTA before it reads anything that another kernel --
+// the library's, or one of the caller's that was given the buffer's address -- may
+// write, and before it writes anything.  Ahead of it are only index arithmetic, barrier
+// set-up and reads of matrices and tables that are uploaded from the host and whose
+// addresses have stayed inside the library.  So a kernel that completes has seen all its
+// predecessors complete, and launches of any other kind (copies, events, other
+// libraries' kernels) order as always.
 __device__ __forceinline__ void dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void dep_sync() {

@@ -62,6 +62,7 @@ struct aob_sh {
   aob::DevBuf<float> twiddle;       // exp(-2 pi i m / nfft) as (re, im) pairs
   aob::DevBuf<float> wxy;           // the same values gathered per (frequency, sample)
   aob::DevBuf<int4> tblob;          // shared-memory table image (see ShSmem)
+  bool tables_out = false;          // the address of an input table has been handed out (sh_image_kernel)
   // centroider whose slopes are fused into comp_image (may be null)
   aob_centro *fused = nullptr;
   uint64_t image_gen = 0;  // bumped whenever binimg changes
@@ -105,6 +106,7 @@ struct aob_pyr {
   aob::DevBuf<float> cx, cy, weights;              // modulation points
   aob::DevBuf<float> submask, sincar;              // nfft x nfft (x fastest)
   aob::DevBuf<float2> phalfxy;                     // exp(i pyramid phase), nfft x nfft
+  bool tables_out = false;                         // the address of one of these three has been handed out
   aob::DevBuf<float2> work;                        // npts x nfft x nfft focal / pupil planes
   aob::DevBuf<float2> conv;                        // nfft x nfft, pixel-transfer convolution
   aob::DevBuf<float> hrimg;                        // nfft x nfft high-resolution image
@@ -145,6 +147,7 @@ struct aob_centro {
   aob::DevBuf<int32_t> validx, validy;
   aob::DevBuf<float> ref, weights, intensities;
   aob::DevBuf<float> pyr_partial;  // pyramid slopes: per-CTA flux sums
+  bool tables_out = false;  // the address of ref or weights has been handed out
   int weights_per_sub = 0;  // 0: one npix^2 map, 1: npix^2*nvalid
   // image path when not attached to a sensor (load_img + calibrate_img)
   int img_m = 0, img_n = 0;

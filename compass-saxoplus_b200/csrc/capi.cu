@@ -253,6 +253,8 @@ int aob_sh_buffer(aob_sh *h, const char *which, void **p, int64_t *n) {
   AOB_API_BEGIN
   NEED(h); NEED(which); NEED(p); NEED(n);
   std::string w(which);
+  for (const char *t : {"pupil", "offsets", "fluxPerSub", "validsubsx", "validsubsy", "istart", "jstart"})
+    if (w == t) h->tables_out = true;  // (the caller's kernels may write it: sh_image_kernel waits for them)
 #define B(name, buf)        \
   if (w == name) {          \
     *p = (void *)h->buf.p;  \
@@ -529,6 +531,7 @@ int aob_centro_buffer(aob_centro *c, const char *which, void **p, int64_t *n) {
   AOB_API_BEGIN
   NEED(c); NEED(which); NEED(p); NEED(n);
   std::string w(which);
+  if (w == "centroids_ref" || w == "weights") c->tables_out = true;  // (as in aob_sh_buffer)
 #define B(name, buf)        \
   if (w == name) {          \
     *p = (void *)c->buf.p;  \
@@ -953,6 +956,7 @@ int aob_pyr_buffer(aob_pyr *h, const char *which, void **dev_ptr, int64_t *nelem
   const std::string w(which);
   void *p = nullptr;
   int64_t n = 0;
+  if (w == "submask" || w == "phalfxy" || w == "sincar") h->tables_out = true;  // (as in aob_sh_buffer)
   if (w == "phase") { p = h->phase.p; n = h->phase.n; }
   else if (w == "pupil") { p = h->pupil.p; n = h->pupil.n; }
   else if (w == "binimg") { p = h->binimg.p; n = h->binimg.n; }

@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(MVM_THREADS) ls_mvm_kernel(MvmArgs A) {
     if (lane == 0) {
       // all loads before the first store (global-space loads, one round trip)
       const float sc = A.rscale ? __ldg(A.rscale + r) : 1.f;
-      const float mg = (A.integrate && A.mgain) ? __ldg(A.mgain + r) : 1.f;
+      const float mg = (A.integrate && A.mgain) ? __ldcg(A.mgain + r) : 1.f;
       const float cm = A.integrate ? __ldcg(A.com + r) : 0.f;
       if (A.rscale) tot *= sc;
       const float e = -tot;
@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(MVM_THREADS) ls_mvm_bulk_kernel(MvmArgs A) {
     }
     if (A.rscale) e_sc = __ldg(A.rscale + gr);
     if (A.integrate) {
-      if (A.mgain) e_mg = __ldg(A.mgain + gr);
+      if (A.mgain) e_mg = __ldcg(A.mgain + gr);  // (its address is handed out)
       e_cm = __ldcg(A.com + gr);
     }
   }

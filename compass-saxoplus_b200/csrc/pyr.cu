@@ -57,6 +57,7 @@ struct PyrArgs {
   const float *submask;
   const float2 *phalfxy;
   const float *sincar;
+  int early;         // the tables' addresses have stayed inside the library
   const float2 *tw;  // N/2 forward twiddles (global)
   float2 *work;      // npts x N x N
   float2 *conv;      // N x N
@@ -157,6 +158,9 @@ __global__ void __launch_bounds__(N / 8 * pyr_cols(N)) pyr_cols_kernel(PyrArgs A
     }
   };
   int group = u / A.npts;
+  // the mask is uploaded by the host and asked for ahead of the wait, until its address has
+  // been handed out (aob_pyr_buffer): a kernel of the caller may then write it
+  if (!A.early) dep_wait();
   load_mask(group * CB + c);
   dep_wait();
   // rows [0, ntot) hold the input and are overwritten by the output: every
@@ -277,6 +281,7 @@ __global__ void __launch_bounds__(N / 8 * pyr_conv_cols(N)) pyr_conv_cols_kernel
   FftTw<N> W;
   dep_launch();
   W.load(A.tw, j);
+  if (!A.early) dep_wait();  // (see pyr_cols_kernel)
 #pragma unroll
   for (int m = 0; m < 8; ++m) msk[m] = A.sincar[x + (size_t)(j + T * m) * N];
   dep_wait();
@@ -507,6 +512,7 @@ void aob_pyr::comp_image(bool with_noise, cudaStream_t s) {
   A.submask = submask.p;
   A.phalfxy = phalfxy.p;
   A.sincar = sincar.p;
+  A.early = !tables_out;
   A.tw = fft_twiddles(device, nfft);
   A.work = work.p;
   A.conv = conv.p;

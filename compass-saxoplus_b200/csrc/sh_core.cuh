@@ -56,6 +56,7 @@ struct ShKernelArgs {
   int noise_mode;  // 0 none, 1 photon, 2 photon + readout
   float noise;
   uint32_t frame, k0, k1;
+  int early;  // the tables' addresses have stayed inside the library (sh_image_kernel)
   const uint32_t *frame_ptr;  // when set, the frame number is read from device memory
   // field stop: the filtered full-pupil field (fs_n x fs_n complex) read in place
   // of the phase and pupil, scaled by fs_inv = 1 / fs_n^2 (sh_batch<..., FS = true>)
@@ -133,6 +134,18 @@ __device__ __forceinline__ void team_sync(const Team &t) {
     asm volatile("bar.sync %0, %1;" ::"r"(t.bar), "r"(t.nt) : "memory");
 }
 
+// One value of a table whose address the library hands out (the pupil, offsets, windows,
+// fluxes, valid positions, reference slopes and weights).  A kernel that starts before its
+// predecessor has ended (WAITS) reads them through coherent loads: the read-only path is
+// for data that no one writes while the kernel runs.
+template <bool WAITS, class T>
+__device__ __forceinline__ T sh_table(const T *p) {
+  if constexpr (WAITS)
+    return __ldcg(p);
+  else
+    return __ldg(p);
+}
+
 // The bulk-copyable part of the tables: the table image (ShSmem::rk bytes at
 // offset 0) and, when its size and address allow a bulk copy (16-byte
 // multiple and alignment), the shared wCoG weights (wt_bytes at ShSmem::wt).
@@ -151,7 +164,7 @@ struct ShTableCopy {
 // sensor's table image with 16-byte loads (one page, one request per
 // thread), the wCoG weights and the 1/k table of the Poisson sampler.
 // image_done / wt_done: those parts already arrive by bulk copy.
-template <int NFFT>
+template <int NFFT, bool WAITS = false>
 __device__ __forceinline__ void sh_load_tables(const ShKernelArgs &P, unsigned char *smem, int tid, int nthreads,
                                                bool image_done = false, bool wt_done = false) {
   const int npix2 = P.npix * P.npix;
@@ -161,7 +174,7 @@ __device__ __forceinline__ void sh_load_tables(const ShKernelArgs &P, unsigned c
     for (int i = tid; i < (int)(L.rk / 16); i += nthreads) dst[i] = __ldg(P.tblob + i);
   if (P.ckind == 2 && !P.c_wper && !wt_done) {
     float *wt = reinterpret_cast<float *>(smem + L.wt);
-    for (int i = tid; i < npix2; i += nthreads) wt[i] = __ldg(P.c_weights + i);
+    for (int i = tid; i < npix2; i += nthreads) wt[i] = sh_table<WAITS>(P.c_weights + i);
   }
   if (P.noise_mode >= 1) {
     float *rk = reinterpret_cast<float *>(smem + L.rk);
@@ -234,7 +247,7 @@ __device__ __forceinline__ void sh_store_images(const ShKernelArgs &P, int base,
 // returned), before the DFTs.  With DEFER_IMG the cube and image writes are
 // left to sh_store_images (the noisy pixels stay in the work area).
 // ``before_phase`` runs on every thread once it has requested what no kernel writes
-// (windows, pupil, offsets, metadata) and before it reads the phase.
+// (windows, pupil, offsets, metadata; see sh_image_kernel) and before it reads the phase.
 template <int NFFT, int PD, int TK = TEAM_CTA, class Hook = NoHook, bool DEFER_IMG = false, bool FS = false,
           class Src = ShStrided, class Pre = NoHook>
 __device__ __forceinline__ void sh_batch(const ShKernelArgs &P, int base, int stride, int S,
@@ -285,12 +298,12 @@ __device__ __forceinline__ void sh_batch(const ShKernelArgs &P, int base, int st
   for (int mt = tid - t0; mt < S; mt += nt) {
     if (mt < 0) break;
     const int k = sub(mt);
-    const int vx = __ldg(P.validsubsx + k), vy = __ldg(P.validsubsy + k);
-    const float fl = __ldg(P.flux + k);
+    const int vx = sh_table<WAITS>(P.validsubsx + k), vy = sh_table<WAITS>(P.validsubsy + k);
+    const float fl = sh_table<WAITS>(P.flux + k);
     float rx = 0.f, ry = 0.f;
     if (P.ckind >= 0) {
-      rx = __ldg(P.c_ref + (P.c_order ? 2 * k : k));
-      ry = __ldg(P.c_ref + (P.c_order ? 2 * k + 1 : k + P.nvalid));
+      rx = sh_table<WAITS>(P.c_ref + (P.c_order ? 2 * k : k));
+      ry = sh_table<WAITS>(P.c_ref + (P.c_order ? 2 * k + 1 : k + P.nvalid));
     }
     m_vx[mt] = vx;
     m_vy[mt] = vy;
@@ -319,8 +332,8 @@ __device__ __forceinline__ void sh_batch(const ShKernelArgs &P, int base, int st
           const int y = PD > 0 ? l / PD : udiv(l, P.mg_pd);
           const int x = l - y * pd;
           const int k = sub(s);
-          fv[j] = P.fs_field[(x + __ldg(P.puppixx + k)) + (y + __ldg(P.puppixy + k)) * P.fs_n];
-          of[j] = __ldg(P.offsets + l);
+          fv[j] = P.fs_field[(x + sh_table<WAITS>(P.puppixx + k)) + (y + sh_table<WAITS>(P.puppixy + k)) * P.fs_n];
+          of[j] = sh_table<WAITS>(P.offsets + l);
         }
       }
 #pragma unroll
@@ -346,14 +359,14 @@ __device__ __forceinline__ void sh_batch(const ShKernelArgs &P, int base, int st
         const int y = PD > 0 ? l / PD : udiv(l, P.mg_pd);
         const int x = l - y * pd;
         const int k = sub(s);
-        const int X = x + __ldg(P.puppixx + k), Y = y + __ldg(P.puppixy + k);
+        const int X = x + sh_table<WAITS>(P.puppixx + k), Y = y + sh_table<WAITS>(P.puppixy + k);
         id[j] = X + Y * P.npup;
         if constexpr (Src::LISTED)
           ph[j] = src.phase(s, X, Y);
         else if constexpr (!WAITS)
           ph[j] = __ldcg(P.phase + id[j]);  // (L2: a resident kernel reads a new phase every step)
-        am[j] = __ldg(P.pupil + id[j]);
-        of[j] = __ldg(P.offsets + l);
+        am[j] = sh_table<WAITS>(P.pupil + id[j]);
+        of[j] = sh_table<WAITS>(P.offsets + l);
       }
     }
     if constexpr (WAITS) {

@@ -1,6 +1,7 @@
 """Chains of kernels started while their predecessor runs give what a chain with a
 host wait after every call gives, bit for bit: calls on one stream, on two streams
-that take turns, and captured in a CUDA graph."""
+that take turns, and captured in a CUDA graph.  What a kernel
+writes into a table whose address the library hands out is what the next image uses."""
 
 import numpy as np
 import pytest
@@ -87,3 +88,101 @@ def test_chain_in_a_graph():
     # the noise frame is part of the captured launch, so the second replay repeats the first's images
     np.testing.assert_array_equal(got[0], first[0])
     np.testing.assert_array_equal(got[1], first[1])
+
+
+def _writers(shape, values):
+    """Ways of writing ``values`` (x fastest) to a device buffer by a kernel on a stream: the
+    library's raytracing of a screen, whose grid lets its successor start early, and an
+    operation of another library."""
+    import torch
+
+    from aob200 import core, optics
+
+    nx, ny = shape
+    d = max(nx, ny) + 1
+    screen = core.OwnedDeviceArray(d * d)
+    host = np.zeros((d, d), np.float32)
+    host[:nx, :ny] = values.reshape(nx, ny, order="F")
+    screen.set(host)
+    src = torch.from_numpy(values.ravel(order="F").copy()).cuda()
+
+    def traced(buf, sp):
+        optics.raytrace(buf.ptr, nx, ny, [(screen.ptr, d, 0.0, 0.0)], True, sp)
+
+    def copied(buf, sp):
+        with torch.cuda.stream(torch.cuda.ExternalStream(sp)):
+            torch.add(src, 0.0, out=torch.as_tensor(core.DeviceArray(buf.ptr, nx * ny, np.float32), device="cuda"))
+
+    return traced, copied
+
+
+def _check_table(buf, shape, image, result, rng):
+    """image(stream) behind a kernel that writes the table, without a host wait in
+    between, gives what it gives with one."""
+    import torch
+
+    stream = torch.cuda.Stream()
+    sp = stream.cuda_stream
+    old = np.array(buf).ravel(order="F")[: shape[0] * shape[1]]
+    sets = [old, (old * rng.uniform(0.5, 1.5, old.size) + 0.01 * rng.standard_normal(old.size)).astype(np.float32)]
+    want = []
+    for v in sets:
+        _writers(shape, v)[0](buf, sp)
+        torch.cuda.synchronize()
+        image(sp)
+        torch.cuda.synchronize()
+        want.append(result())
+    assert not all(np.array_equal(a, b) for a, b in zip(*want))
+    ways = [_writers(shape, v) for v in sets]
+    torch.cuda.synchronize()
+    for k in range(24):
+        ways[k % 2][k // 2 % 2](buf, sp)
+        image(sp)
+        torch.cuda.synchronize()
+        for a, b in zip(result(), want[k % 2]):
+            np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("table", ["pupil", "offsets", "fluxPerSub", "centroids_ref", "weights", "gain"])
+def test_sensor_tables_written_on_the_stream(table):
+    from aob200 import workloads as W
+
+    s = W.sh_loop_setup("plain16")
+    s.centroider = "wcog" if table == "weights" else "cog"
+    wfs, c, ls, loop = W.build_sh_loop(s, graph=False)
+    rng = np.random.default_rng(3)
+    wfs.set_phase((0.1 * rng.standard_normal((wfs.npup, wfs.npup))).astype(np.float32))
+    buf = {"centroids_ref": c, "weights": c, "gain": ls}.get(table, wfs).buffer(table)
+    n = {"pupil": wfs.npup, "offsets": s.geom.pdiam, "weights": wfs.npix}.get(table)
+    shape = (n, n) if n else (buf.n, 1)
+    com = np.zeros(ls.buffer("com").n, np.float32)
+
+    def image(sp):
+        ls.set_com(com)
+        loop.step(None, None, False, sp)
+
+    def result():
+        return [np.array(x) for x in (wfs.d_bincube, ls.buffer("centroids"), ls.buffer("voltage"))]
+
+    _check_table(buf, shape, image, result, rng)
+
+
+@pytest.mark.parametrize("table", ["submask", "phalfxy", "sincar"])
+def test_pyramid_tables_written_on_the_stream(table):
+    from aob200 import core
+
+    rng = np.random.default_rng(4)
+    nfft, ntot, npts = 256, 72, 5
+    x = np.arange(nfft) - nfft / 2
+    ang = 2 * np.pi * np.arange(npts) / npts
+    r = np.hypot(x[:, None], x[None, :])
+    w = core.PyrWfs(4, 1, 2, 2, 4, nfft, ntot, npts, 1.0, 1000.0, lambda_um=0.7)
+    w.load_arrays(np.fft.fftshift(0.05 * np.minimum(np.abs(x[:, None] + 0.3 * x[None, :]), 9.0)).astype(np.float32),
+                  (0.05 * np.sin(ang)).astype(np.float32), (0.05 * np.cos(ang)).astype(np.float32),
+                  np.ones(npts, np.float32),
+                  np.fft.fftshift(np.sinc(x[:, None] / nfft) * np.sinc(x[None, :] / nfft)).astype(np.float32),
+                  np.fft.fftshift(np.clip(1.2 - r / nfft, 0, 1)).astype(np.float32), np.zeros(4), np.zeros(4))
+    w.set_pupil(np.ones((ntot, ntot), np.float32))
+    w.set_phase((0.05 * rng.standard_normal((ntot, ntot))).astype(np.float32))
+    buf = w.buffer(table)
+    _check_table(buf, (nfft, nfft), lambda sp: w.comp_image(False, sp), lambda: [np.array(w.d_binimg)], rng)
