@@ -183,8 +183,10 @@ template <int EPI>
 __device__ __forceinline__ void tc_epilogue(const TcProb &Q, int m0, int n0, int bn, int part, uint32_t taddr,
                                             float *stage, int lane) {
   const int M = Q.P.M, N = Q.P.N, ldc = Q.P.ldc, ldp = Q.P.ldp, out_n = Q.out_n;
-  const float *__restrict__ bias = Q.P.bias;
-  const float *__restrict__ pre_in = Q.P.pre_in;
+  // (written by kernels that this one may overlap: coherent loads, __ldca, and not the
+  // read-only path)
+  const float *bias = Q.P.bias;
+  const float *pre_in = Q.P.pre_in;
   float *__restrict__ pre_out = Q.P.pre_out;
   float *__restrict__ Cf = Q.P.Cf;
   __nv_bfloat16 *__restrict__ Cb = Q.P.Cb;
@@ -195,37 +197,36 @@ __device__ __forceinline__ void tc_epilogue(const TcProb &Q, int m0, int n0, int
   const bool full = m0 + 32 <= M;
 #pragma unroll 1
   for (int c = part; c < bn / 16 && n0 + c * 16 < N; c += TC_EPI_WARPS / 4) {
-    uint32_t r[16];
-    tmem_ld16(taddr + (uint32_t)(c * 16), r);
     const int cn = n0 + c * 16 + cp;
     const bool in = cn < N;  // (N is even: both columns or neither)
-    // the chunk's global inputs go out before the transpose
-    float2 x[8];
-    if (EPI == MG_EPI_DGELU) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int m = m0 + 4 * i + rq;
-        x[i] = (in && (full || m < M)) ? __ldg(reinterpret_cast<const float2 *>(pre_in + (size_t)m * ldp + cn))
-                                       : make_float2(0.f, 0.f);
-      }
-    }
+    // (GELU': z comes in four rows at a time, or the registers do not hold it beside the tile)
     float2 bv = make_float2(0.f, 0.f);
-    if (EPI != MG_EPI_DGELU && bias && in) bv = __ldg(reinterpret_cast<const float2 *>(bias + cn));
+    if (EPI != MG_EPI_DGELU && bias && in) bv = __ldca(reinterpret_cast<const float2 *>(bias + cn));
+    uint32_t r[16];
+    tmem_ld16(taddr + (uint32_t)(c * 16), r);
 #pragma unroll
     for (int j = 0; j < 16; j += 2)
       *reinterpret_cast<float2 *>(stage + lane * TC_STAGING_PITCH + j) =
           make_float2(__uint_as_float(r[j]), __uint_as_float(r[j + 1]));
     __syncwarp();
     float2 csum = make_float2(0.f, 0.f);
+    float2 x[4];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int row = 4 * i + rq, m = m0 + row;
+      if (EPI == MG_EPI_DGELU && i % 4 == 0) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          x[k] = (in && (full || m + 4 * k < M))
+                     ? __ldca(reinterpret_cast<const float2 *>(pre_in + (size_t)(m + 4 * k) * ldp + cn))
+                     : make_float2(0.f, 0.f);
+      }
       float2 v = *reinterpret_cast<const float2 *>(stage + row * TC_STAGING_PITCH + cp);
       if (!in || !(full || m < M)) continue;
       const size_t o = (size_t)m * ldc + cn;
       if (EPI == MG_EPI_DGELU) {
-        v.x *= gelu_grad_f(x[i].x);
-        v.y *= gelu_grad_f(x[i].y);
+        v.x *= gelu_grad_f(x[i % 4].x);
+        v.y *= gelu_grad_f(x[i % 4].y);
       } else {
         v.x += bv.x;
         v.y += bv.y;

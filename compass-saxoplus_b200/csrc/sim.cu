@@ -99,8 +99,10 @@ __global__ void __launch_bounds__(256) extrude_fused_kernel(const __grid_constan
   dep_launch();
   const ExtrudeJob &J = B.job[blockIdx.y];
   const int n = J.n, nst = J.nst, dir = J.dir;
-  const float *__restrict__ src = J.src;
-  float *__restrict__ dst = J.dst;
+  // (the previous move's screen, whose kernel this one may overlap: no __restrict__, which
+  // would let its loads take the read-only path)
+  const float *src = J.src;
+  float *dst = J.dst;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   const int r0 = blockIdx.x * nw + warp;
   const bool rows = (int)blockIdx.x * nw < n;  // this block computes rows (block-uniform)

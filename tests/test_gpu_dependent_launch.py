@@ -186,3 +186,50 @@ def test_pyramid_tables_written_on_the_stream(table):
     w.set_phase((0.05 * rng.standard_normal((ntot, ntot))).astype(np.float32))
     buf = w.buffer(table)
     _check_table(buf, (nfft, nfft), lambda sp: w.comp_image(False, sp), lambda: [np.array(w.d_binimg)], rng)
+
+
+def test_training_chain():
+    """Forward, backward and Adam of several steps, with and without a host wait after each call:
+    a step's epilogues read the biases that the step before has just written."""
+    import torch
+
+    from aob200 import mlp
+
+    rng = np.random.default_rng(6)
+    nin, h1, h2, nout, batch = 200, 96, 72, 50, 700
+    x = torch.from_numpy(rng.standard_normal((batch, nin)).astype(np.float32)).cuda()
+    t = torch.from_numpy(rng.standard_normal((batch, nout)).astype(np.float32)).cuda()
+    got = []
+    for wait in (True, False):
+        m = mlp.MlpReconstructor(nin, nout, h1, h2, seed=7)
+        y = torch.empty((batch, nout), device="cuda")
+        for _ in range(20):
+            for f in (lambda: m.train_step(x.data_ptr(), t.data_ptr(), batch, 1e-2),
+                      lambda: m.forward(x.data_ptr(), batch, y.data_ptr())):
+                f()
+                if wait:
+                    torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        got.append([y.cpu().numpy()] + [p for layer in m.get_params() for p in layer if p is not None])
+    for a, b in zip(*got):
+        np.testing.assert_array_equal(a, b)
+
+
+def test_atmosphere_chain():
+    """Moves that extrude several columns in a row: each reads the screen that the one before
+    wrote."""
+    import torch
+
+    from aob200 import system as S
+
+    got = []
+    for wait in (True, False):
+        sy = S.ShAoSystem(S.plain16(), 0)
+        for _ in range(30):
+            sy.atmos.move()
+            if wait:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        got.append([sy.atmos.screen_host(i) for i in range(len(sy.layer_params))])
+    for a, b in zip(*got):
+        np.testing.assert_array_equal(a, b)
