@@ -385,6 +385,7 @@ struct TcOp {
   GemmArgs P;
   bool a_km, b_kn;
   const GemmArgs *P2 = nullptr;
+  bool slices = false;  // K accumulated in slices (a weight gradient's K is the batch)
   float *colpart = nullptr;
   float *out = nullptr;
   int out_n = 0;
@@ -421,6 +422,10 @@ static void tc_gemm(const TcOp *ops, int n, int device, uint32_t *status, cudaSt
                      : P.epi == MG_EPI_GELU ? P.bias && P.pre_out && P.Cb && !P.Cf
                                             : P.pre_in && P.Cb && !P.Cf && !P.bias && ops[i].colpart),
                 "mlp gemm: outputs that the epilogue does not have");
+    AOB_REQUIRE(!ops[i].slices || (P.epi == MG_EPI_NONE && !P.bias && !ops[i].out && !ops[i].P2),
+                "mlp gemm: K slices go with a plain product");
+    AOB_REQUIRE(P.epi == ops[0].P.epi && ops[i].slices == ops[0].slices,
+                "mlp gemm: the products of a launch have the same epilogue");
     nk = std::max(nk, k);
     boxes |= ops[i].b_kn;
   }
@@ -480,8 +485,13 @@ static void tc_gemm(const TcOp *ops, int n, int device, uint32_t *status, cudaSt
     M.m[2 * i] = M.m[0];
     M.m[2 * i + 1] = M.m[1];
   }
-  smem_opt_in(reinterpret_cast<const void *>(tc_gemm_kernel), (int)TC_SMEM_BYTES);
-  launch_after(tc_gemm_kernel, 2 * (int)std::min<int64_t>(tiles, pairs), TC_THREADS, TC_SMEM_BYTES, s, M, T);
+  const int epi = ops[0].P.epi;
+  auto kern = ops[0].slices          ? tc_gemm_kernel<TC_EPI_SLICES>
+              : epi == MG_EPI_GELU   ? tc_gemm_kernel<MG_EPI_GELU>
+              : epi == MG_EPI_DGELU  ? tc_gemm_kernel<MG_EPI_DGELU>
+                                     : tc_gemm_kernel<MG_EPI_NONE>;
+  smem_opt_in(reinterpret_cast<const void *>(kern), (int)TC_SMEM_BYTES);
+  launch_after(kern, 2 * (int)std::min<int64_t>(tiles, pairs), TC_THREADS, TC_SMEM_BYTES, s, M, T);
   AOB_LAUNCH_CHECK("tc_gemm_kernel");
 }
 
@@ -681,7 +691,10 @@ void aob_mlp::backward(const float *target, int batch, float *loss, cudaStream_t
     O.P = D1;
     O.colpart = colpart[0].p;
     tc_gemm(&O, 1, device, tc_status.p, s);
-    const TcOp W[4] = {{GS, true, true}, {G1, true, true}, {G3, true, true}, {G2, true, true}};
+    const TcOp W[4] = {{GS, true, true, nullptr, true},
+                       {G1, true, true, nullptr, true},
+                       {G3, true, true, nullptr, true},
+                       {G2, true, true, nullptr, true}};
     tc_gemm(W, 4, device, tc_status.p, s);
   } else {
     rparts = COLSUM_CHUNKS;

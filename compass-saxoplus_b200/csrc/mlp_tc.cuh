@@ -11,10 +11,15 @@
 // four 128 x 128 tiles do.  Bound: that traffic -- with either tile the SMs draw
 // 9 - 10 TB/s from L2 (0.42 us per stage at 256 x 256, 1.28 PFLOP/s in the main
 // loop; 128 x 128 tiles reached 0.68).  A training step at batch 4096 (2496 -> 1024
-// -> 1024 -> 1377) takes 315 us, 500 us with 128 x 128 tiles, split K and a
-// launch per bias and parameter array.  Pairs are persistent: pair p takes tiles p, p + pairs, ... of a list of up to
+// -> 1024 -> 1377) takes 319 us, 503 us with 128 x 128 tiles, split K and a launch
+// per bias and parameter array.
+// Pairs are persistent: pair p takes tiles p, p + pairs, ... of a list of up to
 // TC_MAX_PROBS products, so the four weight gradients of a training step
-// (independent, K = the batch) fill the GPU in one launch without split K.
+// (independent, K = the batch) fill the GPU in one launch.  Their K is accumulated in
+// slices of TC_SLICE stages that the epilogue adds in registers: in one run the
+// accumulator's rounding grows with the batch (against float64 sums of the same bfloat16
+// values 9e-6 at batch 4096 and 1e-4 at 20,000; 3e-7 at either in slices, 3 % of the step's
+// time).
 // Per CTA, 18 warps:
 //  * warp 0, one lane: TMA producer -- 2-D tensor loads with 128-byte swizzle
 //    (K-major tile: one box of 64 (K) x rows; MN-major: boxes of 64 (M or N) x
@@ -24,7 +29,7 @@
 //    the leader issues tcgen05.mma.cta_group::2.kind::f16 (M 256, N bn, K 16) and
 //    commits each stage to both CTAs' "empty" mbarriers, and each finished
 //    tile to both CTAs' accumulator barriers;
-//  * 16 warps: the epilogue of a tile while the next one is multiplied -- a warp
+//  * 16 warps: the epilogue of a tile (or slice) while the next one is multiplied -- a warp
 //    reads the TMEM lanes of its quadrant (warp & 3) in chunks of 16 columns,
 //    transposes each through shared memory and applies bias / GELU / GELU' with
 //    row accesses of whole sectors.
@@ -49,6 +54,10 @@ constexpr int TC_EPI_WARPS = 16, TC_THREADS = 64 + 32 * TC_EPI_WARPS;
 constexpr int TC_TILE_BYTES = TC_ROWS * TC_BK * 2;  // one operand tile of a CTA and stage (16 KB)
 constexpr int TC_STAGE_BYTES = 2 * TC_TILE_BYTES;
 constexpr int TC_MAX_PROBS = 4;
+// K stages of one slice of a weight gradient (512 samples): the tensor cores' FP32
+// accumulator loses a little at every addition, in proportion to its sum, so a long K is
+// accumulated in slices, added in order in registers.
+constexpr int TC_SLICE = 8;
 constexpr uint32_t TC_MAX_POLLS = 1u << 22;
 enum : uint32_t { ERR_TC_TIMEOUT = 8u };
 
@@ -264,6 +273,56 @@ __device__ __forceinline__ void tc_epilogue(const TcProb &Q, int m0, int n0, int
   }
 }
 
+// One warp's chunks of a tile whose K was accumulated in slices: tc_epilogue's chunks,
+// held in registers while the slices are added, then stored.
+struct TcSums {
+  static constexpr int CHUNKS = TC_MAX_BN / 16 / (TC_EPI_WARPS / 4);
+  float v[CHUNKS][16];
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int k = 0; k < CHUNKS; ++k)
+#pragma unroll
+      for (int j = 0; j < 16; ++j) v[k][j] = 0.f;
+  }
+  __device__ __forceinline__ void add(uint32_t taddr, int part, int bn) {
+#pragma unroll
+    for (int k = 0; k < CHUNKS; ++k) {
+      const int c = part + k * (TC_EPI_WARPS / 4);
+      if (c >= bn / 16) break;
+      uint32_t r[16];
+      tmem_ld16(taddr + (uint32_t)(c * 16), r);
+#pragma unroll
+      for (int j = 0; j < 16; ++j) v[k][j] += __uint_as_float(r[j]);
+    }
+  }
+  __device__ __forceinline__ void store(const TcProb &Q, int m0, int n0, int bn, int part, float *stage, int lane) const {
+    const int M = Q.P.M, N = Q.P.N, ldc = Q.P.ldc;
+    const int cp = 2 * (lane & 7), rq = lane >> 3;
+    float *C = Q.P.Cf + (size_t)(m0 + rq) * ldc + n0 + cp;
+#pragma unroll
+    for (int k = 0; k < CHUNKS; ++k) {
+      const int c = part + k * (TC_EPI_WARPS / 4);
+      if (c >= bn / 16 || n0 + c * 16 >= N) break;
+#pragma unroll
+      for (int j = 0; j < 16; j += 2)
+        *reinterpret_cast<float2 *>(stage + lane * TC_STAGING_PITCH + j) = make_float2(v[k][j], v[k][j + 1]);
+      __syncwarp();
+      const bool in = n0 + c * 16 + cp < N;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float2 x = *reinterpret_cast<const float2 *>(stage + (4 * i + rq) * TC_STAGING_PITCH + cp);
+        if (in && m0 + 4 * i + rq < M) *reinterpret_cast<float2 *>(C + (size_t)(4 * i) * ldc + c * 16) = x;
+      }
+      __syncwarp();
+    }
+  }
+};
+
+// EPI: the products' epilogue (all of a launch have the same), or TC_EPI_SLICES: plain
+// products accumulated TC_SLICE stages at a time.  A kernel each: with all in one body the
+// sums in registers made the other epilogues spill (61.9 -> 65.0 us the forward pass).
+constexpr int TC_EPI_SLICES = 3;
+template <int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
     tc_gemm_kernel(const __grid_constant__ TcMaps maps, const __grid_constant__ TcArgs T) {
   extern __shared__ __align__(1024) unsigned char tc_raw[];
@@ -353,7 +412,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
       // ---- MMA issuer ----
       int n = 0, s = 0;
       uint32_t phase = 0;
-      for (int t = pair; ok && t < T.ntiles; t += npairs, ++n) {
+      for (int t = pair; ok && t < T.ntiles; t += npairs) {
         const TcTile X(T, t);
         const int a_mn = T.prob[X.i].a_mn, b_mn = T.prob[X.i].b_mn;
         const uint32_t idesc = umma_idesc_bf16(a_mn, b_mn, bn);
@@ -362,29 +421,34 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
         const uint64_t da0 = umma_desc_sw128(smem_addr(sm), a_mn ? TC_TILE_BYTES / 2 : 16, 1024);
         const uint64_t db0 = umma_desc_sw128(smem_addr(sm) + TC_TILE_BYTES, b_mn ? TC_TILE_BYTES / 2 : 16, 1024);
         const uint32_t ka = a_mn ? 128 : 2, kb = b_mn ? 128 : 2;
-        const uint32_t acc = tmem + (uint32_t)(n & 1) * TC_MAX_BN;
-        if (n >= 2 && !mbar_wait(&accempty[n & 1], (uint32_t)(n / 2 - 1) & 1u, TC_MAX_POLLS)) {
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        for (int kt = 0; kt < X.nk; ++kt) {
-          if (!mbar_wait(&full[s], phase, TC_MAX_POLLS)) {
+        // (n counts slices: each takes the other accumulator)
+        const int ks = EPI == TC_EPI_SLICES ? TC_SLICE : X.nk;
+        for (int k0 = 0; ok && k0 < X.nk; k0 += ks, ++n) {
+          const uint32_t acc = tmem + (uint32_t)(n & 1) * TC_MAX_BN;
+          if (n >= 2 && !mbar_wait(&accempty[n & 1], (uint32_t)(n / 2 - 1) & 1u, TC_MAX_POLLS)) {
             ok = false;
             break;
           }
           tc_fence_after();
-          const uint64_t off = (uint64_t)(s * (TC_STAGE_BYTES / 16));
+          const int k1 = min(X.nk, k0 + ks);
+          for (int kt = k0; kt < k1; ++kt) {
+            if (!mbar_wait(&full[s], phase, TC_MAX_POLLS)) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            const uint64_t off = (uint64_t)(s * (TC_STAGE_BYTES / 16));
 #pragma unroll
-          for (int k = 0; k < TC_BK / 16; ++k)
-            umma_bf16(acc, da0 + off + k * ka, db0 + off + k * kb, idesc, (kt > 0 || k > 0) ? 1u : 0u);
-          umma_commit_pair(&empty[s]);
-          if (++s == TC_STAGES) {
-            s = 0;
-            phase ^= 1u;
+            for (int k = 0; k < TC_BK / 16; ++k)
+              umma_bf16(acc, da0 + off + k * ka, db0 + off + k * kb, idesc, (kt > k0 || k > 0) ? 1u : 0u);
+            umma_commit_pair(&empty[s]);
+            if (++s == TC_STAGES) {
+              s = 0;
+              phase ^= 1u;
+            }
           }
+          if (ok) umma_commit_pair(&accfull[n & 1]);
         }
-        if (ok) umma_commit_pair(&accfull[n & 1]);
       }
     }
     __syncwarp();
@@ -393,25 +457,39 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
     const int quad = warp & 3, part = (warp - 2) >> 2;
     float *stage = staging + (warp - 2) * TC_STAGING_FLOATS;
     int n = 0;
-    for (int t = pair; t < T.ntiles; t += npairs, ++n) {
-      const TcTile X(T, t);
-      const TcProb &Q = T.prob[X.i];
-      const int m0 = X.mt * TC_BM + (int)rank * TC_ROWS + quad * 32, n0 = X.nt * bn;
+    // the accumulator of slice n is finished; its columns of this warp's lanes
+    auto finished = [&]() {
       ok = mbar_wait(&accfull[n & 1], (uint32_t)(n / 2) & 1u, TC_MAX_POLLS);
       ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
       tc_fence_after();
-      const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(n & 1) * TC_MAX_BN;
-      const int epi = Q.P.epi;
-      if (epi == MG_EPI_GELU)
-        tc_epilogue<MG_EPI_GELU>(Q, m0, n0, bn, part, taddr, stage, lane);
-      else if (epi == MG_EPI_DGELU)
-        tc_epilogue<MG_EPI_DGELU>(Q, m0, n0, bn, part, taddr, stage, lane);
-      else
-        tc_epilogue<MG_EPI_NONE>(Q, m0, n0, bn, part, taddr, stage, lane);
+      return tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(n & 1) * TC_MAX_BN;
+    };
+    auto hand_back = [&]() {
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(cluster_addr(smem_addr(&accempty[n & 1]), 0));
+      ++n;
+    };
+    for (int t = pair; ok && t < T.ntiles; t += npairs) {
+      const TcTile X(T, t);
+      const TcProb &Q = T.prob[X.i];
+      const int m0 = X.mt * TC_BM + (int)rank * TC_ROWS + quad * 32, n0 = X.nt * bn;
+      if constexpr (EPI == TC_EPI_SLICES) {
+        TcSums sums;
+        sums.clear();
+        for (int k0 = 0; k0 < X.nk; k0 += TC_SLICE) {
+          const uint32_t taddr = finished();
+          if (!ok) break;
+          sums.add(taddr, part, bn);
+          hand_back();
+        }
+        if (ok) sums.store(Q, m0, n0, bn, part, stage, lane);
+      } else {
+        const uint32_t taddr = finished();
+        if (!ok) break;
+        tc_epilogue<EPI>(Q, m0, n0, bn, part, taddr, stage, lane);
+        hand_back();
+      }
     }
   }
   tc_fence_before();

@@ -14,6 +14,47 @@ from oracle import mlp as omlp
 pytestmark = pytest.mark.gpu
 
 
+def _skip_gradient(nin, nout, batch, seed):
+    """The skip path's weight and the output bias's gradients of a network of zeros, with the
+    same from float64 sums: its output is zero, so the bfloat16 operands of the
+    product over the batch are known exactly."""
+    import torch
+
+    from aob200 import _lib, mlp
+
+    def bf16(a):
+        return torch.from_numpy(a).to(torch.bfloat16).double().numpy()
+
+    net = mlp.MlpReconstructor(nin, nout, 16, 8)
+    net.set_params([(np.zeros((16, nin)), np.zeros(16)), (np.zeros((8, 16)), np.zeros(8)),
+                    (np.zeros((nout, 8)), np.zeros(nout)), (np.zeros((nout, nin)), None)])
+    rng = np.random.default_rng(seed)
+    x = rng.uniform(0.5, 1.5, (batch, nin)).astype(np.float32)
+    t = rng.uniform(0.5, 1.5, (batch, nout)).astype(np.float32)
+    dx, dt = torch.from_numpy(x).cuda(), torch.from_numpy(t).cuda()
+    net.forward(dx.data_ptr(), batch)
+    net.backward(dt.data_ptr(), batch)
+    torch.cuda.synchronize()
+    assert net.gemm_status() == 0
+    dy = bf16(np.float32(2) / (np.float32(batch) * np.float32(nout)) * -t)
+    pin, _, _, pout = net.padded_dims()
+    got = [_lib.d2h(*net.buffer(k), np.float32).astype(np.float64) for k in ("dWs", "db3")]
+    return (got[0].reshape(pout, pin)[:nout, :nin], dy.T @ bf16(x)), (got[1][:nout], dy.sum(0))
+
+
+@pytest.mark.parametrize("nin,nout,batch", [(40, 24, 511), (264, 300, 513), (520, 130, 1024), (264, 300, 4096),
+                                            (40, 24, 20001)])
+def test_gradients_over_a_long_batch(nin, nout, batch):
+    """A weight gradient sums the batch in slices of 512 samples.  A slice is 32 additions to
+    an FP32 accumulator, each off by 2^-23 of the partial sum at most (half the slice's sum
+    on average): 1.9e-6; the slices' own additions, rounded to nearest, add 2^-24 of half the sum
+    each, with either sign.  In one run over the batch 4096 samples would be 256 additions."""
+    (dw, want), (db, wantb) = _skip_gradient(nin, nout, batch, batch)
+    slices = -(-batch // 512)
+    assert np.abs(dw / want - 1).max() < 32 * 2.0**-24 + np.sqrt(slices) * 2.0**-23 + 2.0**-23
+    assert np.abs(db / wantb - 1).max() < 2e-6
+
+
 @pytest.mark.parametrize("dims,batch", [
     ((24, 16, 8, 9), 1), ((72, 65, 257, 64), 129), ((400, 264, 56, 520), 257), ((65, 1032, 513, 255), 640),
     ((328, 300, 200, 1000), 5000),
