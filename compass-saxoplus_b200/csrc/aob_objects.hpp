@@ -361,7 +361,7 @@ struct aob_mlp {
   // batch workspace
   int cap = 0;
   aob::DevBuf<uint16_t> xb, h1b, h2b, dy, dz2, dz1;
-  aob::DevBuf<float> z1, z2, y, loss_part;
+  aob::DevBuf<float> z1, z2, y;
   // batch-1 inference
   aob::DevBuf<float> ix, ih1, ih2, iy;
   aob::DevBuf<uint32_t> use_ls, fallbacks;
@@ -369,7 +369,9 @@ struct aob_mlp {
   int fused_mode = 0;  // 0: fused kernel when it fits, 1: multi-kernel path
   int gemm_kind = 1;   // training GEMMs: 0 mma.sync kernel, 1 tcgen05 kernel
   aob::DevBuf<uint32_t> tc_status;  // bounded waits of the tcgen05 GEMM that expired
-  aob::DevBuf<float> colpart[3];    // partial column sums of the bias gradients
+  // a backward pass's partial sums: the bias gradients' columns, the loss
+  aob::DevBuf<float> parts;
+  float *colpart[3] = {}, *loss_part = nullptr;
   aob::DevBuf<float> partial;
   aob::DevBuf<unsigned long long> gbar;
 

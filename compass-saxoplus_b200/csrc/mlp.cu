@@ -609,10 +609,12 @@ void aob_mlp::ensure_batch(int batch) {
   // partial sums: the loss kernel's blocks, and the bias gradients' (a row per 32
   // samples, the output layer's per LOSS_ROWS; COLSUM_CHUNKS rows on the mma.sync path)
   const int nchunk = (cap + LOSS_ROWS - 1) / LOSS_ROWS, rparts = std::max((cap + 31) / 32, COLSUM_CHUNKS);
-  loss_part.alloc((int64_t)nchunk * ((pout + 31) / 32));
-  colpart[0].alloc((int64_t)rparts * ph1);
-  colpart[1].alloc((int64_t)rparts * ph2);
-  colpart[2].alloc((int64_t)nchunk * pout);
+  const int64_t np[4] = {(int64_t)rparts * ph1, (int64_t)rparts * ph2, (int64_t)nchunk * pout,
+                         (int64_t)nchunk * ((pout + 31) / 32)};
+  parts.alloc(np[0] + np[1] + np[2] + np[3]);  // (one allocation: they are on the path of a first forward)
+  colpart[0] = parts.p;
+  for (int l = 1; l < 3; ++l) colpart[l] = colpart[l - 1] + np[l - 1];
+  loss_part = colpart[2] + np[2];
 }
 
 static __nv_bfloat16 *bf(aob::DevBuf<uint16_t> &b) { return reinterpret_cast<__nv_bfloat16 *>(b.p); }
@@ -665,8 +667,8 @@ void aob_mlp::backward(const float *target, int batch, float *loss, cudaStream_t
   AOB_REQUIRE(batch <= cap, "mlp.backward: run forward on this batch first");
   AOB_CUDA(cudaSetDevice(device));
   const dim3 lgrid((pout + 31) / 32, (batch + LOSS_ROWS - 1) / LOSS_ROWS);
-  launch_after(mlp_loss_kernel, lgrid, dim3(32, 8), 0, s, y.p, target, nout, pout, batch, 1.f / out_scale, bf(dy), colpart[2].p,
-                                                loss_part.p);
+  launch_after(mlp_loss_kernel, lgrid, dim3(32, 8), 0, s, y.p, target, nout, pout, batch, 1.f / out_scale, bf(dy), colpart[2],
+               loss_part);
   AOB_LAUNCH_CHECK("mlp_loss_kernel");
   // data gradients: dz2 = (dy W3) * GELU'(z2), dz1 = (dz2 W2) * GELU'(z1)
   const GemmArgs D2{batch, ph2, pout, bf(dy), pout, bf(wb[2]), ph2, nullptr, MG_EPI_DGELU, z2.p, nullptr, ph2,
@@ -686,10 +688,10 @@ void aob_mlp::backward(const float *target, int batch, float *loss, cudaStream_t
   if (gemm_kind == 1) {
     rparts = (batch + 31) / 32;
     TcOp O{D2, false, true};
-    O.colpart = colpart[1].p;
+    O.colpart = colpart[1];
     tc_gemm(&O, 1, device, tc_status.p, s);
     O.P = D1;
-    O.colpart = colpart[0].p;
+    O.colpart = colpart[0];
     tc_gemm(&O, 1, device, tc_status.p, s);
     const TcOp W[4] = {{GS, true, true, nullptr, true},
                        {G1, true, true, nullptr, true},
@@ -704,23 +706,23 @@ void aob_mlp::backward(const float *target, int batch, float *loss, cudaStream_t
     };
     gemm<true, true>(G3, s);
     gemm<false, true>(D2, s);
-    colsum(bf(dz2), ph2, colpart[1].p);
+    colsum(bf(dz2), ph2, colpart[1]);
     gemm<true, true>(G2, s);
     gemm<false, true>(D1, s);
-    colsum(bf(dz1), ph1, colpart[0].p);
+    colsum(bf(dz1), ph1, colpart[0]);
     gemm<true, true>(G1, s);
     gemm<true, true>(GS, s);
   }
   FinishArgs F{};
   const int cols[3] = {ph1, ph2, pout}, parts[3] = {rparts, rparts, (int)lgrid.y};
   for (int l = 0; l < 3; ++l) {
-    F.part[l] = colpart[l].p;
+    F.part[l] = colpart[l];
     F.out[l] = gb[l].p;
     F.nparts[l] = parts[l];
     F.cols[l] = cols[l];
     F.block0[l + 1] = F.block0[l] + (cols[l] + 31) / 32;
   }
-  F.loss_part = loss_part.p;
+  F.loss_part = loss_part;
   F.nloss = (int)(lgrid.x * lgrid.y);
   F.denom = (float)batch * (float)nout;
   F.loss = loss;
