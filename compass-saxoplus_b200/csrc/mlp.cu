@@ -92,8 +92,10 @@ __global__ void __launch_bounds__(256)
   dep_sync();
   __shared__ float red[8][33], red2[8];
   const float g = 2.f / ((float)batch * (float)nout);
-  const int c = blockIdx.x * 32 + threadIdx.x;
-  const int r0 = blockIdx.y * LOSS_ROWS + threadIdx.y, r1 = min(batch, (int)(blockIdx.y + 1) * LOSS_ROWS);
+  // (one grid dimension: the chunks of a large batch pass the 65535 of the others)
+  const int ncb = (pout + 31) / 32, chunk = blockIdx.x / ncb;
+  const int c = ((int)blockIdx.x - chunk * ncb) * 32 + threadIdx.x;
+  const int r0 = chunk * LOSS_ROWS + threadIdx.y, r1 = min(batch, (chunk + 1) * LOSS_ROWS);
   float csum = 0.f, acc = 0.f;
   if (c < pout)
     for (int b0 = r0; b0 < r1; b0 += 32) {
@@ -124,12 +126,12 @@ __global__ void __launch_bounds__(256)
     float v = 0.f;
 #pragma unroll
     for (int k = 0; k < 8; ++k) v += red[k][threadIdx.x];
-    if (c < pout) colpart[(int64_t)blockIdx.y * pout + c] = v;
+    if (c < pout) colpart[(int64_t)chunk * pout + c] = v;
     if (threadIdx.x == 0) {
       v = 0.f;
 #pragma unroll
       for (int k = 0; k < 8; ++k) v += red2[k];
-      part[blockIdx.y * gridDim.x + blockIdx.x] = v;
+      part[blockIdx.x] = v;
     }
   }
 }
@@ -666,8 +668,10 @@ void aob_mlp::forward(const float *x, int batch, float *y_out, cudaStream_t s) {
 void aob_mlp::backward(const float *target, int batch, float *loss, cudaStream_t s) {
   AOB_REQUIRE(batch <= cap, "mlp.backward: run forward on this batch first");
   AOB_CUDA(cudaSetDevice(device));
-  const dim3 lgrid((pout + 31) / 32, (batch + LOSS_ROWS - 1) / LOSS_ROWS);
-  launch_after(mlp_loss_kernel, lgrid, dim3(32, 8), 0, s, y.p, target, nout, pout, batch, 1.f / out_scale, bf(dy), colpart[2],
+  const int nchunk = (batch + LOSS_ROWS - 1) / LOSS_ROWS;
+  const int64_t lgrid = (int64_t)nchunk * ((pout + 31) / 32);
+  AOB_REQUIRE(lgrid <= INT32_MAX, "mlp.backward: batch too large");
+  launch_after(mlp_loss_kernel, (unsigned)lgrid, dim3(32, 8), 0, s, y.p, target, nout, pout, batch, 1.f / out_scale, bf(dy), colpart[2],
                loss_part);
   AOB_LAUNCH_CHECK("mlp_loss_kernel");
   // data gradients: dz2 = (dy W3) * GELU'(z2), dz1 = (dz2 W2) * GELU'(z1)
@@ -714,7 +718,7 @@ void aob_mlp::backward(const float *target, int batch, float *loss, cudaStream_t
     gemm<true, true>(GS, s);
   }
   FinishArgs F{};
-  const int cols[3] = {ph1, ph2, pout}, parts[3] = {rparts, rparts, (int)lgrid.y};
+  const int cols[3] = {ph1, ph2, pout}, parts[3] = {rparts, rparts, nchunk};
   for (int l = 0; l < 3; ++l) {
     F.part[l] = colpart[l];
     F.out[l] = gb[l].p;
@@ -723,7 +727,7 @@ void aob_mlp::backward(const float *target, int batch, float *loss, cudaStream_t
     F.block0[l + 1] = F.block0[l] + (cols[l] + 31) / 32;
   }
   F.loss_part = loss_part;
-  F.nloss = (int)(lgrid.x * lgrid.y);
+  F.nloss = (int)lgrid;
   F.denom = (float)batch * (float)nout;
   F.loss = loss;
   launch_after(mlp_finish_kernel, F.block0[3] + (loss ? 1 : 0), dim3(32, 8), 0, s, F);
