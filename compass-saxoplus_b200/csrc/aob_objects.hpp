@@ -166,7 +166,7 @@ struct aob_centro {
   int nslopes() const { return type == AOB_CENTRO_MASKEDPIX ? nvalid : 2 * nvalid; }
   void touch() { ++params_gen; }
   bool fused_ready() const;
-  void copy_frame(const uint16_t *src, cudaStream_t s);
+  bool copy_frame(const uint16_t *src, cudaStream_t s);
   void get_cog(float *dev_slopes, cudaStream_t s);
   void init_calib();
   void calibrate(cudaStream_t s, bool valid_only = false);

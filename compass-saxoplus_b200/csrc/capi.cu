@@ -467,14 +467,11 @@ int aob_centro_load_img_u16(aob_centro *c, const uint16_t *img, int m, int n, in
   if (c->img_raw_u16.n != mn) c->img_raw_u16.alloc(mn);
   c->img_m = m;
   c->img_n = n;
-  cudaPointerAttributes at{};
-  if (on_device && (cudaPointerGetAttributes(&at, img) != cudaSuccess || at.type != cudaMemoryTypeDevice ||
-                    at.device != c->device)) {
-    cudaGetLastError();
-    // (managed memory, another GPU's, or none: the copy decides)
-    AOB_CUDA(cudaMemcpyAsync(c->img_raw_u16.p, img, sizeof(uint16_t) * mn, cudaMemcpyDeviceToDevice, S(stream)));
-  } else if (on_device) {
-    c->copy_frame(img, S(stream));
+  if (on_device) {
+    // (where the kernel does not apply -- managed memory, another GPU's, a frame on an odd
+    // byte, or one that its allocation does not hold -- the copy decides)
+    if (!c->copy_frame(img, S(stream)))
+      AOB_CUDA(cudaMemcpyAsync(c->img_raw_u16.p, img, sizeof(uint16_t) * mn, cudaMemcpyDeviceToDevice, S(stream)));
   } else {
     AOB_CUDA(cudaMemcpyAsync(c->img_raw_u16.p, img, sizeof(uint16_t) * mn, cudaMemcpyHostToDevice, S(stream)));
     AOB_CUDA(cudaStreamSynchronize(S(stream)));

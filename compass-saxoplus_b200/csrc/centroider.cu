@@ -11,6 +11,8 @@
 // sensor kernel (sh_wfs.cu) and this kernel only runs if the image changed
 // after that or a parameter was modified.
 
+#include <cuda.h>
+
 #include <algorithm>
 #include <vector>
 
@@ -387,14 +389,45 @@ void aob_centro::calibrate(cudaStream_t s, bool valid_only) {
   AOB_LAUNCH_CHECK("calib_valid_kernel");
 }
 
-// load_img of a frame in device memory: a kernel of the chain (a frame in place needs none)
-void aob_centro::copy_frame(const uint16_t *src, cudaStream_t s) {
+// Whether a kernel on this device may read [p, p + bytes): device memory of this device, on
+// an address that uint16 loads take, inside one allocation.
+static bool readable_u16(const void *p, size_t bytes, int device) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+  if (a & 1) return false;
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  if (at.type != cudaMemoryTypeDevice || at.device != device) return false;
+  using RangeFn = CUresult (*)(CUdeviceptr *, size_t *, CUdeviceptr);
+  static const RangeFn range = [] {
+    void *f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &f, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      f = nullptr;
+    }
+    return reinterpret_cast<RangeFn>(f);
+  }();
+  CUdeviceptr base = 0;
+  size_t size = 0;
+  if (!range || range(&base, &size, (CUdeviceptr)a) != CUDA_SUCCESS) return false;
+  return a - base <= size && bytes <= size - (a - base);
+}
+
+// load_img of a frame in device memory: a kernel of the chain (a frame in place needs
+// none).  False, and nothing done, where the kernel may not read it.
+bool aob_centro::copy_frame(const uint16_t *src, cudaStream_t s) {
   const int64_t n = img_raw_u16.n;
-  if (src == img_raw_u16.p) return;
+  if (src == img_raw_u16.p) return true;
+  if (!readable_u16(src, sizeof(uint16_t) * (size_t)n, device)) return false;
   const int vec = ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(img_raw_u16.p)) & 15) == 0;
   launch_after(copy_frame_kernel, (int)std::max<int64_t>(1, std::min<int64_t>((n / 8 + 255) / 256, 2048)), 256, 0, s,
                img_raw_u16.p, src, n, vec);
   AOB_LAUNCH_CHECK("copy_frame_kernel");
+  return true;
 }
 
 void aob_centro::get_cog(float *dev_slopes, cudaStream_t s) {

@@ -117,3 +117,27 @@ def test_uint16_frame_from_host(cam):
     s, _, _ = ortc.centroids(frame.astype(np.float64), g.validsubsx, g.validsubsy, g.npix, g.pixsize,
                              g.npix / 2 - 0.5)
     assert rel_rms(np.array(ls.buffer("centroids")), s) < 1e-4
+
+
+@pytest.mark.parametrize("m,n", [(1, 3), (16, 16), (37, 41)])
+def test_uint16_frame_at_any_device_address(m, n):
+    """A frame in device memory that starts on 16 bytes, on another even byte, and on an odd one
+    (a camera packet behind a header of odd length), up to the end of its allocation, and
+    in place."""
+    import torch
+
+    from aob200 import _lib, core
+
+    rng = np.random.default_rng(m * n)
+    frame = rng.integers(0, 65536, m * n).astype(np.uint16)
+    for off in (0, 16, 2, 6, 1, 3, 17):
+        c = core.Centroider(4, 1.5, 1.0, "cog")
+        buf = core.OwnedDeviceArray(off + 2 * m * n, np.uint8)
+        buf.set(np.concatenate([np.full(off, 255, np.uint8), frame.view(np.uint8)]))
+        for _ in range(2):
+            _lib.call("aob_centro_load_img_u16", c.h, buf.ptr + off, m, n, 1, None)
+            torch.cuda.synchronize()
+            np.testing.assert_array_equal(np.array(c.buffer("img_raw", np.uint16)), frame)
+        own = c.buffer("img_raw", np.uint16)  # the frame in place
+        _lib.call("aob_centro_load_img_u16", c.h, own.ptr, m, n, 1, None)
+        np.testing.assert_array_equal(np.array(own), frame)
