@@ -62,13 +62,13 @@ def raytrace(dev_out, nx, ny, sources, reset=True, stream=None):
     n = len(sources)
     Ptr, Int, Flt = _ray_arrays(max(n, 1))
     ptrs, dims, xo, yo = Ptr(), Int(), Flt(), Flt()
-    for k, (p, d, x, y) in enumerate(sources):
-        ptrs[k], dims[k], xo[k], yo[k] = p, d, x, y
+    for k, s in enumerate(sources):
+        ptrs[k], dims[k], xo[k], yo[k] = s[0], int(s[1]), float(s[2]), float(s[3])
     call("aob_raytrace", dev_out, int(nx), int(ny), n, ctypes.addressof(ptrs), ctypes.addressof(dims),
          ctypes.addressof(xo), ctypes.addressof(yo), 1 if reset else 0, stream)
 
 
-@functools.lru_cache(maxsize=None)
+@functools.lru_cache(maxsize=16)
 def _ray_arrays(n):
     """Array types of n sources (making a ctypes array type costs more than the call)."""
     return ctypes.c_void_p * n, ctypes.c_int * n, ctypes.c_float * n
