@@ -32,7 +32,7 @@ import time
 
 from ._lib import AobError, call
 
-DEFAULT_BATCH_SPACE = dict(subaps=(8, 16, 32), team=(64, 256), mvm_kb=(24, 48, 96), lag=(64,),
+DEFAULT_BATCH_SPACE = dict(subaps=(8, 16, 32), team=(64, 256), mvm_kb=(24, 48, 96), lag=(-1, 64),
                            ctas_per_sm=(2, 3, 4), order=(0,))
 _BATCH_KEYS = ("subaps", "team", "mvm_kb", "lag", "ctas_per_sm", "order")
 DEFAULT_LOOP_SPACE = dict(fused_batch=(0, 1, 2, 4, 8))

@@ -302,7 +302,7 @@ struct aob_batch {
   std::vector<aob_loop *> loops;
   // tuning: sub-apertures per sensor item, threads per sensor team, command-matrix
   // KB per MVM item, CTAs per SM (0: chosen by pick_tuning), MVM items queued
-  // `lag` instances after their sensor items (-1: see build), instance order
+  // `lag` instances after their sensor items (-1: by the queue's length, see build), instance order
   // (0 = largest first, 1 = as added)
   int subaps = 0, team = 0, mvm_kb = 0, lag = -1, ctas_per_sm = 0, order = 0;
   struct Tuning {

@@ -359,7 +359,7 @@ void aob_batch::set_tuning(int subaps_, int team_, int mvm_kb_, int lag_, int ct
   AOB_REQUIRE(team_ == 0 || team_ == 32 || team_ == 64 || team_ == 128 || team_ == 256,
               "batch.set_tuning: team_threads must be 0, 32, 64, 128 or 256");
   AOB_REQUIRE(mvm_kb_ >= 0 && mvm_kb_ <= 200, "batch.set_tuning: mvm_kb must be in [0, 200]");
-  AOB_REQUIRE(lag_ >= 0 && lag_ <= 1024, "batch.set_tuning: lag must be in [0, 1024]");
+  AOB_REQUIRE(lag_ >= -1 && lag_ <= 1024, "batch.set_tuning: lag must be in [-1, 1024]");
   AOB_REQUIRE(ctas_per_sm_ >= 0 && ctas_per_sm_ <= 4, "batch.set_tuning: ctas_per_sm must be in [0, 4]");
   AOB_REQUIRE(order_ == 0 || order_ == 1, "batch.set_tuning: order must be 0 or 1");
   subaps = subaps_;

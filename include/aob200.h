@@ -680,9 +680,9 @@ int aob_batch_add(aob_batch *b, aob_loop *loop);
  * 1024), threads per sensor team (32, 64, 128 or 256: an item's sub-apertures
  * are shared by the CTA's teams, each runs its share as one batch),
  * command-matrix KB per MVM item (at most 200), lag in instances between an
- * instance's sensor and MVM items, CTAs per SM (at most 4); 0 for any but the lag
- * leaves it to the batch, which chooses by its size (as all are, the lag too,
- * until this is called).  Instance order: 0 = largest first, 1 = as added. */
+ * instance's sensor and MVM items, CTAs per SM (at most 4); 0, or -1 for the lag,
+ * leaves a value to the batch, which chooses by its size (as all are until
+ * this is called).  Instance order: 0 = largest first, 1 = as added. */
 int aob_batch_set_tuning(aob_batch *b, int subaps_per_item, int team_threads, int mvm_kb, int lag, int ctas_per_sm,
                          int order);
 int aob_batch_use_graph(aob_batch *b, int enable);

@@ -22,7 +22,7 @@ def _batch(sizes, prec):
 def test_picked_shapes_equal_the_fixed_one(sizes, prec):
     outs = []
     for tuning in (None, dict(subaps_per_item=32, team_threads=32, mvm_kb=48, lag=2, ctas_per_sm=2),
-                   dict(ctas_per_sm=3), dict(mvm_kb=24, lag=0), dict(team_threads=64, ctas_per_sm=4)):
+                   dict(ctas_per_sm=3), dict(mvm_kb=24, lag=0), dict(lag=-1), dict(team_threads=64, ctas_per_sm=4)):
         loops, b = _batch(sizes, prec)
         if tuning is not None:
             b.set_tuning(**tuning)
@@ -34,3 +34,17 @@ def test_picked_shapes_equal_the_fixed_one(sizes, prec):
         for x, y in zip(outs[0], other):
             np.testing.assert_array_equal(x[0], y[0])
             np.testing.assert_array_equal(x[1], y[1])
+
+
+def test_lag_left_to_the_batch():
+    """set_tuning leaves the lag to the batch unless it is given, and takes -1 for that; below -1 it
+    is refused."""
+    from aob200._lib import AobError
+
+    loops, b = _batch([(24, 6)] * 6, "bf16")
+    for kw in ({}, dict(ctas_per_sm=3), dict(lag=-1, mvm_kb=24)):
+        b.set_tuning(**kw)
+        b.step(True)
+    assert b.status() == 0
+    with pytest.raises(AobError, match="lag"):
+        b.set_tuning(lag=-2)
