@@ -36,7 +36,10 @@ inline void cuda_check(cudaError_t e, const char *what) {
 // device.  Recorded per (kernel, device) and only ever raised, under a lock,
 // so that every device gets its own opt-in and no caller lowers the limit
 // another one relies on.
-inline void smem_opt_in(const void *fn, int bytes) {
+// ``beside``: the kernel is to become resident beside its predecessor (launch_after), or its
+// successor beside it.  An SM changes its split between L1 and shared memory only when it
+// is empty, so such a pair asks for the same split, all of it shared memory.
+inline void smem_opt_in(const void *fn, int bytes, bool beside = false) {
   static std::mutex mu;
   static std::map<std::pair<const void *, int>, int> done;
   int dev = 0;
@@ -44,6 +47,8 @@ inline void smem_opt_in(const void *fn, int bytes) {
   std::lock_guard<std::mutex> lock(mu);
   int &cur = done[{fn, dev}];
   if (bytes > cur) {
+    if (beside && cur == 0)
+      AOB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
     AOB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
     cur = bytes;
   }
@@ -55,7 +60,8 @@ inline void smem_opt_in(const void *fn, int bytes) {
 // sensor as four calls: 24.7 us a pass, 17.3 us started this way; a 512 x 512 pyramid
 // with its command matrix, nine kernels: 111.6 and 88.4 us).  A kernel started by
 // launch_after may become resident while the kernel before it on the stream still runs,
-// once all of that one's CTAs have said so (dep_launch, at their start) or ended, and
+// once all of that one's CTAs have said so (dep_launch, at their start, the sensor
+// kernel's once its loads are in) or ended, and
 // waits in dep_wait until it has completed and its writes are visible.  Every such
 // kernel calls dep_wait in every CTA before it reads anything that another kernel --
 // the library's, or one of the caller's that was given the buffer's address -- may

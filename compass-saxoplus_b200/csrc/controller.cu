@@ -228,7 +228,8 @@ __global__ void __launch_bounds__(MVM_THREADS) ls_mvm_bulk_kernel(MvmArgs A) {
     for (int r = 0; r < R; ++r)
       bulk_g2s(rows + (size_t)r * row_bytes, src + (size_t)r * row_bytes, row_bytes, &bars[0]);
   }
-  dep_wait();  // (the rows, which no kernel writes, are on their way while the slopes' producer ends)
+  dep_wait();  // (the rows, which no kernel writes, are on their way while the slopes' producer ends --
+               // where a CTA found room beside it: see sh_image_kernel's registers)
   if (A.bump && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(A.bump, 1u);
   // epilogue inputs of this thread's row (R <= blockDim), fetched now
   float e_sc = 1.f, e_mg = 1.f, e_cm = 0.f, e_o0 = 0.f, e_o1 = 0.f;
@@ -578,7 +579,7 @@ void launch_mvm_t(const MvmArgs &A0, int grid, bool bulk, cudaStream_t s) {
     A.rows_per_cta = (A.nrow + grid - 1) / grid;
     const size_t sm = mvm_bars_bytes(A.rows_per_cta) + slope_bytes + (size_t)A.rows_per_cta * A.ld * sizeof(T) +
                       sizeof(float) * (MVM_THREADS / 32) * A.rows_per_cta;
-    smem_opt_in(reinterpret_cast<const void *>(ls_mvm_bulk_kernel<T>), (int)sm);
+    smem_opt_in(reinterpret_cast<const void *>(ls_mvm_bulk_kernel<T>), (int)sm, true);
     launch_after(ls_mvm_bulk_kernel<T>, grid, MVM_THREADS, sm, s, A);
     AOB_LAUNCH_CHECK("ls_mvm_bulk_kernel");
   } else {

@@ -137,6 +137,10 @@ void aob_loop::device_step(bool noise, cudaStream_t s, bool frame_on_device) {
       // before it ends, where nothing but kernels follows one another: a cooperative
       // launch cannot overlap its predecessor's end (3.1 us from one kernel's end to
       // the next one's start, 0.9 us this way) and pays a grid barrier besides.
+      // saxo40: 13.9 us a step back to back, 16.7 as one kernel; among other kernels with the L2
+      // flushed 22.3 and 24.6; alone in a loop of flushes, where the one kernel's code
+      // stays cached, 21.9 and 20.8 (mode 2 keeps the one kernel).  plain16: 8.4 and 12.3 back to
+      // back, 15.4 and 20.5 among others.
       // A step whose host reads or writes it has copies in between, and its
       // voltages come out sooner from one kernel.
       if (mode == 0 && fused_batch == 0 && !host_step && !frame_on_device && ls->comp_com_voltage(s, true)) {

@@ -45,11 +45,13 @@ constexpr int SH_MAX_BATCH = 32;
 // their shared-memory loads issue back to back); PD == 0: runtime side.
 // Sub-apertures k = blockIdx.x + (r * S + s) * gridDim.x, s < S, rounds r.
 template <int NFFT, int PD, bool FS = false>
-__global__ void __launch_bounds__(SH_THREADS) sh_image_kernel(ShKernelArgs P, int S) {
+// (registers: with two of its CTAs on an SM, 96 a thread leave room for the MVM's 512
+// threads of 32, so that the rows come in beside the sensor's stages.  6 pixels need no more
+// than 92; 8 would be 0.7 us slower at 96)
+__global__ void __maxnreg__(PD == 6 ? 96 : 112) sh_image_kernel(ShKernelArgs P, int S) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int pd = PD > 0 ? PD : P.pdiam;
   const ShSmem L(NFFT, P.nu, P.nv, pd, P.nrebin2 * P.npix * P.npix, P.npix * P.npix, S);
-  dep_launch();
   // The tables are uploaded by the host, so they can be asked for ahead of the wait -- until
   // their address has been handed out (aob_sh_buffer, aob_centro_buffer): a kernel of the
   // caller may then write them on the stream.  (At 40 x 40: 14.1 us a step back to back, 14.8
@@ -63,11 +65,18 @@ __global__ void __launch_bounds__(SH_THREADS) sh_image_kernel(ShKernelArgs P, in
   struct Wait {
     __device__ void operator()() const { dep_wait(); }
   };
+  // The next kernel may start once the field's loads have come in: a command matrix's rows,
+  // which it asks for at once, would hold them up (with the L2 flushed a saxo40 step of kernels
+  // replayed from a graph takes 15.8 us, 17.1 when it started with this one; plain16 back
+  // to back 8.4 and 8.9).
+  struct Next {
+    __device__ void operator()() const { dep_launch(); }
+  };
   for (int base = blockIdx.x; base < P.nvalid; base += S * gridDim.x) {
     const int Sb = min(S, (P.nvalid - base + (int)gridDim.x - 1) / (int)gridDim.x);
-    sh_batch<NFFT, PD, TEAM_CTA, NoHook, false, FS, ShStrided, Wait>(P, base, gridDim.x, Sb, smem, smem + L.hdr, L,
-                                                                     Team{(int)threadIdx.x, (int)blockDim.x, 0},
-                                                                     NoHook{}, ShStrided{}, Wait{});
+    sh_batch<NFFT, PD, TEAM_CTA, Next, false, FS, ShStrided, Wait>(P, base, gridDim.x, Sb, smem, smem + L.hdr, L,
+                                                                   Team{(int)threadIdx.x, (int)blockDim.x, 0}, Next{},
+                                                                   ShStrided{}, Wait{});
   }
 }
 
@@ -288,7 +297,7 @@ template <int NFFT, int PD, bool FS>
 static void launch_sh_fs(const ShKernelArgs &P, int nvalid, int S, size_t sm, cudaStream_t s) {
   const int grid = std::max(1, (nvalid + S - 1) / S);
   // opt-in per (kernel, device), only ever raised (a driver call per launch costs microseconds)
-  smem_opt_in(reinterpret_cast<const void *>(sh_image_kernel<NFFT, PD, FS>), (int)std::max<size_t>(sm, 48 * 1024));
+  smem_opt_in(reinterpret_cast<const void *>(sh_image_kernel<NFFT, PD, FS>), (int)std::max<size_t>(sm, 48 * 1024), true);
   launch_after(sh_image_kernel<NFFT, PD, FS>, grid, SH_THREADS, sm, s, P, S);
 }
 template <int NFFT, int PD>
