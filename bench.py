@@ -349,8 +349,7 @@ def run_mc64(args, torch):
     loops, batch = W.build_mc_batch(insts, precision="bf16")
     setup_s = time.perf_counter() - t0
     if args.no_tune:
-        batch.set_tuning(16, 256, 96, 16, 2, 0)
-        tune = {"tuning": {"subaps": 16, "team": 256, "mvm_kb": 96, "lag": 16, "ctas_per_sm": 2, "order": 0}}
+        tune = {"tuning": "chosen by the batch from its size"}
     else:
         tune = AT.tune_batch(batch, noise=True)
     info = batch.info()
@@ -640,7 +639,7 @@ def main():
     ap.add_argument("--epochs", type=int, default=16, help="c4: training epochs")
     ap.add_argument("--settle", type=int, default=100, help="c4: closed-loop iterations before the long exposure")
     ap.add_argument("--instances", type=int, default=64, help="mc64: number of instances (the first N of the list)")
-    ap.add_argument("--no-tune", action="store_true", help="mc64: fixed tile shapes instead of the autotuner")
+    ap.add_argument("--no-tune", action="store_true", help="mc64: the tile shapes that the batch chooses by its size instead of the autotuner")
     args = ap.parse_args()
     args.warmup = max(args.warmup, 3)
     if args.impl == "reference":
@@ -683,29 +682,46 @@ def main():
         _lib.call("aob_memcpy_d2d", phase_ptr, d_screens[i % nscreen].data_ptr(), nbytes_phase, sptr)
 
     # ---- value: device-resident inputs, L2 flushed before each step --------
-    for i in range(args.warmup):
-        load_phase(i)
-        flush.zero_()
-        loop.step(None, None, noise=True, stream=sptr)
-    torch.cuda.synchronize()
-    if dist:
-        dist.barrier()
-    torch.cuda.synchronize()
-    starts = [torch.cuda.Event(enable_timing=True) for _ in range(args.steps)]
-    ends = [torch.cuda.Event(enable_timing=True) for _ in range(args.steps)]
-    with ClockSampler(device) as clk:
-        for i in range(args.steps):
+    def timed_steps():
+        for i in range(args.warmup):
             load_phase(i)
             flush.zero_()
-            starts[i].record(stream)
             loop.step(None, None, noise=True, stream=sptr)
-            ends[i].record(stream)
         torch.cuda.synchronize()
-    if dist:
-        dist.barrier()
-    torch.cuda.synchronize()
-    total_ms = max_over_ranks(dist, torch, [sum(s.elapsed_time(e) for s, e in zip(starts, ends))], "cuda")[0]
-    clocks = clk.summary()
+        if dist:
+            dist.barrier()
+        torch.cuda.synchronize()
+        starts = [torch.cuda.Event(enable_timing=True) for _ in range(args.steps)]
+        ends = [torch.cuda.Event(enable_timing=True) for _ in range(args.steps)]
+        with ClockSampler(device) as clk:
+            for i in range(args.steps):
+                load_phase(i)
+                flush.zero_()
+                starts[i].record(stream)
+                loop.step(None, None, noise=True, stream=sptr)
+                ends[i].record(stream)
+            torch.cuda.synchronize()
+        if dist:
+            dist.barrier()
+        torch.cuda.synchronize()
+        ms = max_over_ranks(dist, torch, [sum(s.elapsed_time(e) for s, e in zip(starts, ends))], "cuda")[0]
+        return ms, clk.summary(), loop.kernels_per_step()
+
+    # The steps stand alone between flushes, which the one cooperative kernel suits (mode 2);
+    # steps that follow other work run as two overlapping kernels by default (mode 0), timed
+    # the same way beside it.
+    default_ms, _, default_kernels = timed_steps()
+    mode = 2
+    loop.set_mode(mode)
+    try:
+        total_ms, clocks, _ = timed_steps()
+    except _lib.AobError:  # a configuration that the one kernel does not fit
+        mode = 0
+        loop.set_mode(mode)
+        total_ms, clocks, _ = timed_steps()
+    default_step = {"value": job_rate(ws, args.steps, default_ms), "unit": UNIT,
+                    "ms_per_step": default_ms / args.steps, "kernels_per_step": default_kernels,
+                    "what": "the same steps in mode 0, Loop's default"}
     ms_per_step = total_ms / args.steps
     value = job_rate(ws, args.steps, total_ms)
     launches = loop.kernels_per_step() * args.steps
@@ -732,14 +748,14 @@ def main():
         dom, dbytes, dt, prof = "rtc_fused_kernel", mvm_bytes + wfs_bytes, t_step, f"rtc_fused_saxo40_{args.precision}"
     elif pair:
         dom, dbytes, dt = "sh_image_kernel + ls_mvm_bulk_kernel", mvm_bytes + wfs_bytes, t_step
-        prof = f"rtc_pair_saxo40_{args.precision}"
+        prof = None
     elif t_mvm >= t_wfs:
         dom, dbytes, dt, prof = "ls_mvm_bulk_kernel", mvm_bytes, t_mvm, f"ls_mvm_saxo40_{args.precision}"
     else:
         dom, dbytes, dt, prof = "sh_image_kernel", wfs_bytes, t_wfs, "sh_image_saxo40"
     achieved = dbytes / dt / 1e9
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                "traffic": _profile_traffic(prof), "kernel": dom, "algorithmic_bytes_per_launch": dbytes,
+                "traffic": _profile_traffic(prof) if prof else None, "kernel": dom, "algorithmic_bytes_per_launch": dbytes,
                 "duration_us": dt * 1e6, "peak_source": peak_kind, "timing": "graph replay, L2 flushed per launch",
                 "kernels_us": {"rtc_step": t_step * 1e6, "sh_image": t_wfs * 1e6, "ls_mvm": t_mvm * 1e6}}
 
@@ -897,7 +913,7 @@ def main():
                   "dm_shape_bytes": dm_bytes, "dm_shape_gbs": dm_bytes / ex_us[2] / 1e3, "iteration_us": ex_us[3],
                   "what": f"saxo40 closed loop (3 von Karman layers, {dm_nact}-actuator DM): extrusion of every layer, "
                           "raytrace into the sensor's phase, DM shape, and the whole iteration (extrusion, "
-                          "raytrace, fused RTC step, DM shape)"}
+                          "raytrace, RTC step, DM shape)"}
 
     # ---- persistent mode: the fused kernel resident (matrix rows, sensor tables
     # and integrator state in shared memory), one doorbell per step; the L2 flush
@@ -972,9 +988,13 @@ def main():
                    "l2": "flushed before every timed step (256 MB write)",
                    "parallelism": f"replicas x{ws}",
                    "launch": ("one cooperative kernel per step, launched directly" if fused
-                              else ("three kernels per step, CUDA graph" if not args.no_graph else "three kernels per step")),
+                              else "two overlapping kernels per step, launched directly" if pair
+                              else "three kernels per step, CUDA graph" if not args.no_graph
+                              else "three kernels per step"),
+                   "loop_mode": mode,
                    "mvm_precision": args.precision},
         "roofline": roofline, "cpu_baseline": cpu, "e2e": e2e, "clocks": clocks, "gpu_launches": launches,
+        "default_step": default_step,
         "persistent": persistent,
         "learned": learned,
         "closed_loop_extras": extras,
