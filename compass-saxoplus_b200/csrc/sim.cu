@@ -371,9 +371,9 @@ __global__ void __launch_bounds__(N / 8 * target_cols(N))
     mle = max(mle, __float_as_uint(l[m]));
   }
   // one atomic per CTA (unsigned maxima of float bits, as the images are not negative)
-  const unsigned active = __activemask();
-  mse = __reduce_max_sync(active, mse);
-  mle = __reduce_max_sync(active, mle);
+  constexpr unsigned lanes = T * CB < 32 ? (1u << (T * CB)) - 1u : 0xffffffffu;  // (a whole warp from N = 64 on)
+  mse = __reduce_max_sync(lanes, mse);
+  mle = __reduce_max_sync(lanes, mle);
   if ((threadIdx.x & 31) == 0) {
     red[0][threadIdx.x >> 5] = mse;
     red[1][threadIdx.x >> 5] = mle;
