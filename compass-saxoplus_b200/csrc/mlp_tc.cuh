@@ -37,8 +37,8 @@
 // in the same K loop, so y = h2 W3^T + x Ws^T is one GEMM with no read-back of
 // the output.
 // Every mbarrier wait is bounded: on expiry a status bit is set, nothing of the
-// tile is stored, and the CTA goes to its end, where it frees its TMEM.  No load
-// uses multicast.
+// tile is stored, and the CTA goes to its end, where it waits (bounded) for its loads and
+// the pair's MMAs in flight and frees its TMEM.  No load uses multicast.
 #pragma once
 
 #include <cuda.h>
@@ -333,8 +333,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
   float *staging = reinterpret_cast<float *>(sm + TC_STAGES * TC_STAGE_BYTES);
   uint64_t *full = reinterpret_cast<uint64_t *>(staging + TC_STAGING_FLOATS * TC_EPI_WARPS);
   uint64_t *empty = full + TC_STAGES;
-  uint64_t *accfull = empty + TC_STAGES, *accempty = accfull + 2;
-  uint32_t *tslot = reinterpret_cast<uint32_t *>(accempty + 2);
+  uint64_t *accfull = empty + TC_STAGES, *accempty = accfull + 2, *drained = accempty + 2;
+  uint32_t *tslot = reinterpret_cast<uint32_t *>(drained + 1);
   dep_launch();
   if (threadIdx.x == 0) {
     for (int s = 0; s < TC_STAGES; ++s) {
@@ -345,6 +345,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
       mbar_init(&accfull[b], 1);
       mbar_init(&accempty[b], 2 * TC_EPI_WARPS);
     }
+    mbar_init(drained, 1);
     fence_mbar_init();
   }
   if (warp == 1) {
@@ -405,6 +406,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
       // the last stages' hand-backs have arrived before the CTA may end
       for (int k = max(0, it - TC_STAGES); ok && k < it; ++k)
         ok = mbar_wait(&empty[k % TC_STAGES], (uint32_t)(k / TC_STAGES) & 1u, TC_MAX_POLLS);
+      // a wait that expired: its loads may still be landing (a load takes microseconds)
+      if (!ok)
+        for (int k = 0; k < 1000; ++k) __nanosleep(1000);
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -450,6 +454,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
           if (ok) umma_commit_pair(&accfull[n & 1]);
         }
       }
+      umma_commit_pair(drained);
     }
     __syncwarp();
   } else {
@@ -494,6 +499,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
   }
   tc_fence_before();
   __syncthreads();
+  if (warp == 1) {  // every MMA that was issued has completed, also where a wait above has expired
+    if (lane == 0) ok = mbar_wait(drained, 0, TC_MAX_POLLS) && ok;
+    __syncwarp();
+  }
   cluster_sync();  // the pair's MMAs, loads and arrivals are done (or its bounded waits have expired)
   if (warp == 1)
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
