@@ -36,9 +36,9 @@ inline void cuda_check(cudaError_t e, const char *what) {
 // device.  Recorded per (kernel, device) and only ever raised, under a lock,
 // so that every device gets its own opt-in and no caller lowers the limit
 // another one relies on.
-// ``beside``: the kernel is to become resident beside its predecessor (launch_after), or its
-// successor beside it.  An SM changes its split between L1 and shared memory only when it
-// is empty, so such a pair asks for the same split, all of it shared memory.
+// ``beside``: a kernel whose successor is to become resident beside it (launch_after) and
+// needs more shared memory than it.  An SM changes its split between L1 and shared memory
+// only when it is empty, so the first of the two asks for all of it as shared memory.
 inline void smem_opt_in(const void *fn, int bytes, bool beside = false) {
   static std::mutex mu;
   static std::map<std::pair<const void *, int>, int> done;

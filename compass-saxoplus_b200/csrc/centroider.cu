@@ -506,7 +506,7 @@ void aob_centro::get_cog(float *dev_slopes, cudaStream_t s) {
                              cudaMemcpyDeviceToDevice, s));
     if (type == 1) {
       const int n = npix * npix * nvalid;
-      launch_after(tcog_writeback_kernel, std::min((n + 255) / 256, 4096), 256, 0, s, 
+      launch_after(tcog_writeback_kernel, std::min((n + 255) / 256, 4096), 256, 0, s,
           wfs->binimg.p, wfs->npix * wfs->nxsub, validx.p, validy.p, nvalid, npix, threshold);
       AOB_LAUNCH_CHECK("tcog_writeback_kernel");
       ++wfs->image_gen;  // a second get_cog thresholds again, as the reference does

@@ -579,7 +579,7 @@ void launch_mvm_t(const MvmArgs &A0, int grid, bool bulk, cudaStream_t s) {
     A.rows_per_cta = (A.nrow + grid - 1) / grid;
     const size_t sm = mvm_bars_bytes(A.rows_per_cta) + slope_bytes + (size_t)A.rows_per_cta * A.ld * sizeof(T) +
                       sizeof(float) * (MVM_THREADS / 32) * A.rows_per_cta;
-    smem_opt_in(reinterpret_cast<const void *>(ls_mvm_bulk_kernel<T>), (int)sm, true);
+    smem_opt_in(reinterpret_cast<const void *>(ls_mvm_bulk_kernel<T>), (int)sm);
     launch_after(ls_mvm_bulk_kernel<T>, grid, MVM_THREADS, sm, s, A);
     AOB_LAUNCH_CHECK("ls_mvm_bulk_kernel");
   } else {
@@ -637,7 +637,7 @@ void aob_ls::generic_comp_com(cudaStream_t s, uint32_t *bump) {
   float berta = leaky;
   if (polc) {
     AOB_REQUIRE(imat_rows.p != nullptr, "comp_com: polc needs the interaction matrix (set_imat)");
-    launch_after(gemv_rows_kernel, std::max(1, std::min((nslope + 7) / 8, 4096)), 256, 0, s, 
+    launch_after(gemv_rows_kernel, std::max(1, std::min((nslope + 7) / 8, 4096)), 256, 0, s,
         imat_rows.p, nactu, nslope, nactu, com_clipped.p, -1.f, 1.f, centroids.p, ol_meas.p);
     AOB_LAUNCH_CHECK("gemv_rows_kernel (polc)");
     sin = ol_meas.p;

@@ -32,7 +32,9 @@ namespace aob {
 
 constexpr int IMAT_THREADS = 256;
 constexpr int IMAT_LIST = 512;  // sub-apertures of one actuator listed at a time
-constexpr int IMAT_ITEMS = 16;  // images per batch, at most: 51 KB of shared memory at 40 x 40, four CTAs per SM
+// images per batch, at most: 51 KB of shared memory at 40 x 40 (the registers, 80 a thread, allow
+// three CTAs on an SM)
+constexpr int IMAT_ITEMS = 16;
 
 struct ImatArgs {
   const float *influ;
@@ -206,8 +208,9 @@ extern "C" int aob_imat_build(aob_sh *w, aob_centro *c, aob_dm *dm, float xoff, 
     // (SutraRtc::comp_images_imat, sutra_rtc.cpp:380-395); 0 keeps nphot
     if (w->nphot4imat > 0.f) P.nphot = w->nphot4imat;
     const int nact = dm->nact;
-    const int per = chunk > 0 ? std::min(chunk, nact) : nact;
-    AOB_REQUIRE(2 * (int64_t)per <= 65535, "aob_imat_build: at most 32767 actuators per chunk");
+    // (chunk is a limit on the scratch that earlier forms needed; only its check is left)
+    AOB_REQUIRE((chunk > 0 ? std::min(chunk, nact) : nact) <= 32767,
+                "aob_imat_build: at most 32767 actuators per chunk");
     DevBuf<float> flat(2 * (int64_t)w->nvalid);
     ImatArgs A{};
     A.influ = dm->influ.p;

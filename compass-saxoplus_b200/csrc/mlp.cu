@@ -627,7 +627,7 @@ void aob_mlp::forward(const float *x, int batch, float *y_out, cudaStream_t s) {
   {
     const int64_t ngrp = (int64_t)batch * (pin / 4);
     const int vec = nin % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
-    launch_after(mlp_input_kernel, (int)std::max<int64_t>(1, std::min<int64_t>((ngrp + 511) / 512, 8 * num_sms(device))), 256, 0, s, 
+    launch_after(mlp_input_kernel, (int)std::max<int64_t>(1, std::min<int64_t>((ngrp + 511) / 512, 8 * num_sms(device))), 256, 0, s,
         x, nin, pin, ngrp, vec, in_scale, bf(xb));
     AOB_LAUNCH_CHECK("mlp_input_kernel");
   }
@@ -697,10 +697,12 @@ void aob_mlp::backward(const float *target, int batch, float *loss, cudaStream_t
     O.P = D1;
     O.colpart = colpart[0];
     tc_gemm(&O, 1, device, tc_status.p, s);
-    const TcOp W[4] = {{GS, true, true, nullptr, true},
-                       {G1, true, true, nullptr, true},
-                       {G3, true, true, nullptr, true},
-                       {G2, true, true, nullptr, true}};
+    // (a batch of one slice needs no sums)
+    const bool slices = batch > TC_SLICE * TC_BK;
+    const TcOp W[4] = {{GS, true, true, nullptr, slices},
+                       {G1, true, true, nullptr, slices},
+                       {G3, true, true, nullptr, slices},
+                       {G2, true, true, nullptr, slices}};
     tc_gemm(W, 4, device, tc_status.p, s);
   } else {
     rparts = COLSUM_CHUNKS;

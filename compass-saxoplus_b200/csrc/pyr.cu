@@ -537,14 +537,14 @@ void aob_pyr::comp_image(bool with_noise, cudaStream_t s) {
     default: pyr_launch<2048>(A, device, s); break;
   }
   if (compute_focalplane) {
-    launch_after(pyr_focal_sum_kernel, (int)std::min<int64_t>((n2 + 255) / 256, 8 * num_sms(device)), 256, 0, s, 
+    launch_after(pyr_focal_sum_kernel, (int)std::min<int64_t>((n2 + 255) / 256, 8 * num_sms(device)), 256, 0, s,
         focalplane.p, focal_work.p, npts, n2);
     AOB_LAUNCH_CHECK("pyr_focal_sum_kernel");
   }
   const float nz = with_noise ? noise : -1.f;
   const int noise_mode = nz > 0 ? 2 : (nz > -1 ? 1 : 0);
   const int nb2 = nbin() * nbin();
-  launch_after(pyr_norm_noise_kernel, std::min((nb2 + 255) / 256, 4 * num_sms(device)), 256, 0, s, 
+  launch_after(pyr_norm_noise_kernel, std::min((nb2 + 255) / 256, 4 * num_sms(device)), 256, 0, s,
       binimg.p, partial.p, nbin(), nphot, noise_mode, nz, (uint32_t)frame, (uint32_t)((uint64_t)seed & 0xffffffffu),
       (uint32_t)((uint64_t)seed >> 32));
   AOB_LAUNCH_CHECK("pyr_norm_noise_kernel");

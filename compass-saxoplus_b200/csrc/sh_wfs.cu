@@ -468,7 +468,7 @@ void aob_sh::set_fakecam(int enable, int max_flux, int max_pix) {
 
 void aob_sh::digitalize(cudaStream_t s) {
   const int64_t n = binimg.n;
-  launch_after(digitalize_kernel, (int)std::min<int64_t>((n + 255) / 256, 4096), 256, 0, s, 
+  launch_after(digitalize_kernel, (int)std::min<int64_t>((n + 255) / 256, 4096), 256, 0, s,
       camimg.p, binimg.p, cam_dark.p, cam_flat.p, max_flux_per_pix, max_pix_value, n);
   AOB_LAUNCH_CHECK("digitalize_kernel");
 }
@@ -476,7 +476,7 @@ void aob_sh::digitalize(cudaStream_t s) {
 void aob_sh::fill_binimage(cudaStream_t s) {
   AOB_CUDA(cudaSetDevice(device));
   const int n = npix * npix * nvalid;
-  launch_after(sh_fill_image_kernel, std::min((n + 255) / 256, 4096), 256, 0, s, 
+  launch_after(sh_fill_image_kernel, std::min((n + 255) / 256, 4096), 256, 0, s,
       binimg.p, bincube.p, validsubsx.p, validsubsy.p, npix, nvalid, npix * nxsub);
   AOB_LAUNCH_CHECK("sh_fill_image_kernel");
   ++image_gen;

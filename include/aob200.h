@@ -505,9 +505,9 @@ int aob_dm_buffer(aob_dm *d, const char *which, void **dev_ptr, int64_t *nelem);
  * columns (s_push - s_pull) / (2 push) into dev_imat, nslope x nact column-major on
  * the device.  Equal bit for bit to poking one actuator after the other with
  * aob_dm_comp_shape, aob_raytrace, aob_sh_comp_image and aob_centro_get_cog
- * (at the same photon count).  chunk: actuators per pass (0 = all, at most 32767);
- * the matrix does not depend on it.  Needs 2 nvalid floats of scratch; waits for
- * the stream. */
+ * (at the same photon count).  chunk: without effect on the matrix or the work; 0, or a
+ * number of actuators; at most 32767 of them (0: the DM's) are accepted, as when it bounded
+ * the scratch.  Needs 2 nvalid floats of scratch; waits for the stream. */
 int aob_imat_build(aob_sh *w, aob_centro *c, aob_dm *dm, float xoff, float yoff, float push, int chunk,
                    float *dev_imat, void *stream);
 
