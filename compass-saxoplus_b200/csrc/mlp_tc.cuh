@@ -11,15 +11,15 @@
 // four 128 x 128 tiles do.  Bound: that traffic -- with either tile the SMs draw
 // 9 - 10 TB/s from L2 (0.42 us per stage at 256 x 256, 1.28 PFLOP/s in the main
 // loop; 128 x 128 tiles reached 0.68).  A training step at batch 4096 (2496 -> 1024
-// -> 1024 -> 1377) takes 319 us, 503 us with 128 x 128 tiles, split K and a launch
+// -> 1024 -> 1377) takes 309 us, 503 us with 128 x 128 tiles, split K and a launch
 // per bias and parameter array.
 // Pairs are persistent: pair p takes tiles p, p + pairs, ... of a list of up to
 // TC_MAX_PROBS products, so the four weight gradients of a training step
 // (independent, K = the batch) fill the GPU in one launch.  Their K is accumulated in
 // slices of TC_SLICE stages that the epilogue adds in registers: in one run the
 // accumulator's rounding grows with the batch (against float64 sums of the same bfloat16
-// values 9e-6 at batch 4096 and 1e-4 at 20,000; 3e-7 at either in slices, 3 % of the step's
-// time).
+// values 9e-6 at batch 4096 and 1e-4 at 20,000; 3e-7 at either in slices, 1 to 8 us of a
+// step).
 // Per CTA, 18 warps:
 //  * warp 0, one lane: TMA producer -- 2-D tensor loads with 128-byte swizzle
 //    (K-major tile: one box of 64 (K) x rows; MN-major: boxes of 64 (M or N) x
@@ -208,7 +208,16 @@ __device__ __forceinline__ void tc_epilogue(const TcProb &Q, int m0, int n0, int
   for (int c = part; c < bn / 16 && n0 + c * 16 < N; c += TC_EPI_WARPS / 4) {
     const int cn = n0 + c * 16 + cp;
     const bool in = cn < N;  // (N is even: both columns or neither)
-    // (GELU': z comes in four rows at a time, or the registers do not hold it beside the tile)
+    // the chunk's global inputs go out ahead of its TMEM read and the transpose
+    float2 x[8];
+    if (EPI == MG_EPI_DGELU) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int m = m0 + 4 * i + rq;
+        x[i] = (in && (full || m < M)) ? __ldca(reinterpret_cast<const float2 *>(pre_in + (size_t)m * ldp + cn))
+                                       : make_float2(0.f, 0.f);
+      }
+    }
     float2 bv = make_float2(0.f, 0.f);
     if (EPI != MG_EPI_DGELU && bias && in) bv = __ldca(reinterpret_cast<const float2 *>(bias + cn));
     uint32_t r[16];
@@ -219,23 +228,15 @@ __device__ __forceinline__ void tc_epilogue(const TcProb &Q, int m0, int n0, int
           make_float2(__uint_as_float(r[j]), __uint_as_float(r[j + 1]));
     __syncwarp();
     float2 csum = make_float2(0.f, 0.f);
-    float2 x[4];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int row = 4 * i + rq, m = m0 + row;
-      if (EPI == MG_EPI_DGELU && i % 4 == 0) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          x[k] = (in && (full || m + 4 * k < M))
-                     ? __ldca(reinterpret_cast<const float2 *>(pre_in + (size_t)(m + 4 * k) * ldp + cn))
-                     : make_float2(0.f, 0.f);
-      }
       float2 v = *reinterpret_cast<const float2 *>(stage + row * TC_STAGING_PITCH + cp);
       if (!in || !(full || m < M)) continue;
       const size_t o = (size_t)m * ldc + cn;
       if (EPI == MG_EPI_DGELU) {
-        v.x *= gelu_grad_f(x[i % 4].x);
-        v.y *= gelu_grad_f(x[i % 4].y);
+        v.x *= gelu_grad_f(x[i].x);
+        v.y *= gelu_grad_f(x[i].y);
       } else {
         v.x += bv.x;
         v.y += bv.y;
