@@ -414,8 +414,8 @@ static size_t mvm_item_bytes(const aob_ls *c, int r) {
 // SM.  Measured on B200 over 9 batches (2 to 64 loops, 8 to 40 sub-apertures across,
 // every precision; all shapes with 8 .. 64 sub-apertures, teams of 32 .. 256, 24 .. 96 KB
 // and 2 .. 4 CTAs per SM): the shapes below are within 8 % of the best of each, 17 %
-// at one.  Many sub-apertures: large items, three CTAs (170 us for 32 loops of 24 .. 40
-// sub-apertures across, 371 us with the former fixed shape and a lag of two
+// at one.  Many sub-apertures: large items, three CTAs (196 us for 32 loops of 24 .. 40
+// sub-apertures across, 378 us with the former fixed shape and a lag of two
 // instances, whose rows waited for sensor items still running).  Few: small items, so
 // that every CTA has one (67 -> 31 us for 5 loops of 10 .. 20).  Two CTAs and the
 // former shape where an item would not fit otherwise.

@@ -18,7 +18,7 @@
 // so the matrix equals the poke-by-poke one bit for bit.
 //
 // Bound: issue of the sensor stages (about 86,000 images at that size).  One call
-// takes 0.26 ms (B200, warm); forming all 3.4 M images from DM shapes and phases
+// takes 0.245 ms (B200, warm); forming all 3.4 M images from DM shapes and phases
 // in memory took 22 ms (14.7 ms images, 2.8 ms shapes, 0.65 ms tracing, the rest
 // 1.5 GB of scratch).
 
